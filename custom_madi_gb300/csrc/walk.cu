@@ -808,79 +808,210 @@ __global__ void __launch_bounds__(128) walk_f64_kernel(const madi_walk_desc d) {
 // ---------------------------------------------------------------------------
 // Column reduction from stored Y (replaces _reduce_kernel, madi/walker_gpu.py:
 // 658-695, which re-reads Y once per column).  A CTA takes a block of
-// REDUCE_THREADS * REDUCE_CPT columns and a range of walkers: walker rows are
-// staged in shared memory a few at a time and every thread adds, for its
-// columns, cos / sin(coef * dM) over the 3 axes with dM = Y[jd] + Y[jD] - Y[js]
-// (the reference's operation order) into fp64 partial sums in a fixed order.
-// Each (CTA, column) partial is then rounded once to 2^-32 fixed point and
-// added to an int64 accumulator: integer addition is order independent, so the
-// sums do not depend on how the grid was scheduled.  Y is read from HBM/L2
-// ceil(n_cols / (REDUCE_THREADS * REDUCE_CPT)) times instead of n_cols times.
+// REDUCE_COLS columns and a range of walkers.  Consecutive columns with the same
+// (jd, jD, js) form a run (the b values of one pair): per walker and axis
+// dM = Y[jd] + Y[jD] - Y[js] (the reference's operation order) is computed once
+// per run into shared memory and every thread adds cos / sin(coef * dM) of its
+// columns.
+//
+// Bound: the fp64 pipe retires about two lanes per SM and cycle, so a library
+// sincos (~35 fp64 operations) made this kernel 303 ms for 31,125 columns x
+// 50,000 walkers.  Here a term costs one fp64 operation,
+//   r = coef / 2 pi * dM + 1.5 * 2^8 + 2^-13  (fma),
+// which leaves the phase in turns modulo 1 in the low 44 mantissa bits: the
+// upper 12 choose a table entry (cos, sin of i / 4096 turn in 2^-48 fixed
+// point) and the lower 32 the offset x, |x| <= 2^-13 turn.  The addition
+// formulas with cos x = 1 - e, sin x = x - x^3 / 6 run in 32 x 32 -> 64 bit
+// integer products on the int pipe, terms rounded to 2^-40.  Emulated against
+// extended precision: at most 1.8e-12 a term, 4e-13 rms, sums over 1.5e5 terms
+// within 2e-10 rms for phases spread over 1e-4 to 50 rad and exact for phase 0.
+// A CTA's sums are integers in 2^-48; each is rounded once to 2^-q, the finest
+// unit in which 3 n_walkers fits 63 bits, and added to the column's total, so the
+// result does not depend on scheduling (bit-identical from run to run).
+// Measured at 31,125 columns x 50,000 walkers: 12.0 ms (fp64 pipe 72 % busy);
+// error against 64 bits 1.6e-14 of the sums' norm, 3.0e-14 before.
+// A chunk of walkers with any |phase| >= 127 turns (or a NaN) goes through
+// sincos() in fp64 instead.
 // ---------------------------------------------------------------------------
-constexpr int REDUCE_THREADS = 256;
-constexpr int REDUCE_CPT = 4;                                // columns per thread
-constexpr int REDUCE_COLS = REDUCE_THREADS * REDUCE_CPT;     // columns per CTA
+constexpr int REDUCE_CPT = 2;                                // columns per thread
+constexpr int REDUCE_COLS = 1024;                            // columns per CTA, at most
+constexpr int REDUCE_TAB = 4096;                             // table entries per turn
+constexpr int REDUCE_Q = 48;                                 // fraction bits of a CTA's sums
+constexpr int REDUCE_WALKERS = 8192;                         // walkers per CTA: 3 * 2^13 * 2^48 < 2^63
+constexpr int REDUCE_DM_BYTES = 39424;                       // dM of one walker for 1,024 runs, and more
+// table + run triples (uint16 x 3) + largest |coef| of each run + dM: two CTAs an SM
+constexpr int REDUCE_SMEM = REDUCE_TAB * 16 + REDUCE_COLS * 6 + REDUCE_COLS * 4 + REDUCE_DM_BYTES;
+static_assert(REDUCE_DM_BYTES >= REDUCE_COLS * 24, "one walker's dM must fit");
 
-__global__ void __launch_bounds__(REDUCE_THREADS) reduce_Y_kernel(const double* __restrict__ Y, int64_t n_walkers,
-                                                                  int n_grid, int wt, int64_t per_block,
-                                                                  const int32_t* __restrict__ jd,
-                                                                  const int32_t* __restrict__ jD,
-                                                                  const int32_t* __restrict__ js,
-                                                                  const double* __restrict__ coef, int n_cols,
-                                                                  unsigned long long* accum) {
-    extern __shared__ double sy[];                            // [wt][n_grid * 3]
-    const int row_len = n_grid * 3;
-    int a[REDUCE_CPT], b[REDUCE_CPT], c[REDUCE_CPT];
-    double pc[REDUCE_CPT], cs[REDUCE_CPT], sn[REDUCE_CPT];
+// cos and sin of one phase, given r = turns + 384 + 2^-13, added to (ac, as).
+// Every product is rounded to nearest: a phase of 0 adds exactly (1, 0).
+constexpr double REDUCE_MAGIC = 384.0 + 0x1p-13;             // half a table step: the floor of r is the nearest entry
+// A table value in 2^-31 (+1 saturates).
+MADI_DEV int q31(long long v) {
+    const int hi = (int)(v >> 32);
+    return hi == 1 << (REDUCE_Q - 32) ? 0x7fffffff : (int)__funnelshift_r((unsigned)v, (unsigned)hi, REDUCE_Q - 31);
+}
+
+MADI_DEV void add_cos_sin(double r, const longlong2* tab, long long& ac, long long& as) {
+    const int hi = __double2hiint(r), lo = __double2loint(r);
+    const longlong2 cs = tab[hi & (REDUCE_TAB - 1)];
+    const int x = lo ^ (int)0x80000000;                      // offset from the entry, 2^-44 turn
+    const int xx = __mulhi(x, x);
+    // 1 - cos(2 pi x) in 2^-51: 2^31 2 pi^2 / 16, less 2.9e-8 of it for the mean of the x^4 term
+    const int e = (int)__umulhi((unsigned)xx, 0x9DE9E600u);
+    const int e3 = __mulhi(xx, 1685);                        // a third of it in 2^-32
+    const int xs = x - (int)(((long long)x * e3 + 0x80000000ll) >> 32);
+    const int X = (int)(((long long)xs * 0x6487ED51 + 0x40000000ll) >> 31);   // sin(2 pi x) in 2^-41: 2 pi 2^28
+    const int c = q31(cs.x), s = q31(cs.y);
+    const int dc = -(int)(((long long)s * X + 0x80000000ll) >> 32) - ((__mulhi(c, e) + 512) >> 10);
+    const int ds = (int)(((long long)c * X + 0x80000000ll) >> 32) - ((__mulhi(s, e) + 512) >> 10);
+    ac += cs.x + (long long)dc * 256;
+    as += cs.y + (long long)ds * 256;
+}
+
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS, 2) reduce_Y_kernel(const double* __restrict__ Y, int64_t n_walkers,
+                                                              int n_grid, int64_t per_block,
+                                                              const int32_t* __restrict__ jd,
+                                                              const int32_t* __restrict__ jD,
+                                                              const int32_t* __restrict__ js,
+                                                              const double* __restrict__ coef, int n_cols,
+                                                              int shift, unsigned long long* accum) {
+    extern __shared__ __align__(16) unsigned char rsm[];
+    longlong2* tab = reinterpret_cast<longlong2*>(rsm);
+    uint16_t* run = reinterpret_cast<uint16_t*>(rsm + REDUCE_TAB * 16);                          // [runs][3]
+    int* run_max = reinterpret_cast<int*>(rsm + REDUCE_TAB * 16 + REDUCE_COLS * 6);              // |turns per dM|
+    double* dM = reinterpret_cast<double*>(rsm + REDUCE_TAB * 16 + REDUCE_COLS * 10);            // [walkers][runs][3]
+    __shared__ int seg[REDUCE_COLS / 32 + 1];
+    const int tid = threadIdx.x, lane = tid & 31;
+    constexpr int COLS = THREADS * REDUCE_CPT;
+    static_assert(COLS <= REDUCE_COLS && COLS / 32 <= 32, "run table and segment scan");
+    const int col0 = blockIdx.x * COLS;
+    const int cols = min(COLS, n_cols - col0);
+    // ---- table: cos / sin of i / 4096 turn from 32 coarse and 32 fine
+    // angles of the first quadrant (one complex product), mirrored ----
+    double2* cf = reinterpret_cast<double2*>(dM);
+    if (tid < 64) {
+        const double turn = tid < 32 ? tid / 128.0 : (tid - 32) / 4096.0;
+        double sn, cn;
+        sincospi(2.0 * turn, &sn, &cn);
+        cf[tid] = make_double2(cn, sn);
+    }
+    __syncthreads();
+    for (int i = tid; i < REDUCE_TAB / 4; i += THREADS) {
+        const double2 u = cf[i >> 5], v = cf[32 + (i & 31)];
+        const long long c = __double2ll_rn((u.x * v.x - u.y * v.y) * (double)(1ll << REDUCE_Q));
+        const long long s = __double2ll_rn((u.y * v.x + u.x * v.y) * (double)(1ll << REDUCE_Q));
+        tab[i] = make_longlong2(c, s);
+        tab[i + REDUCE_TAB / 4] = make_longlong2(-s, c);
+        tab[i + REDUCE_TAB / 2] = make_longlong2(-c, -s);
+        tab[i + 3 * REDUCE_TAB / 4] = make_longlong2(s, -c);
+    }
+    // ---- runs of equal (jd, jD, js) among this block's columns ----
+    for (int i = tid; i < COLS; i += THREADS) run_max[i] = 0;
+    double pc[REDUCE_CPT];                                   // turns per dM
+    int my_run[REDUCE_CPT];
+    long long ac[REDUCE_CPT], as[REDUCE_CPT];
 #pragma unroll
     for (int k = 0; k < REDUCE_CPT; ++k) {
-        const int col = blockIdx.x * REDUCE_COLS + k * REDUCE_THREADS + threadIdx.x;
-        const bool live = col < n_cols;
-        a[k] = live ? 3 * jd[col] : 0;
-        b[k] = live ? 3 * jD[col] : 0;
-        c[k] = live ? 3 * js[col] : 0;
-        pc[k] = live ? coef[col] : 0.0;
-        cs[k] = 0.0;
-        sn[k] = 0.0;
+        const int i = k * THREADS + tid;
+        const int col = col0 + i;
+        const bool live = i < cols;
+        const bool head = live && (i == 0 || jd[col] != jd[col - 1] || jD[col] != jD[col - 1] || js[col] != js[col - 1]);
+        const unsigned heads = __ballot_sync(MADI_FULL, head);
+        if (lane == 0) seg[i >> 5] = __popc(heads);
+        my_run[k] = __popc(heads & (0xffffffffu >> (31 - lane))) - 1;
+        pc[k] = live ? __dmul_rn(coef[col], 0.15915494309189535) : 0.0;
+        ac[k] = as[k] = 0;
     }
+    __syncthreads();
+    if (tid < 32) {
+        int v = lane < COLS / 32 ? seg[lane] : 0;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(MADI_FULL, v, o);
+            if (lane >= o) v += u;
+        }
+        __syncwarp();
+        seg[lane + 1] = v;
+        if (lane == 0) seg[0] = 0;
+    }
+    __syncthreads();
+    const int runs = seg[COLS / 32];
+    const int kmax = (cols + THREADS - 1) / THREADS;
+#pragma unroll
+    for (int k = 0; k < REDUCE_CPT; ++k) {
+        const int i = k * THREADS + tid;
+        my_run[k] += seg[i >> 5];
+        if (i < cols) {
+            const int col = col0 + i;
+            run[3 * my_run[k]] = (uint16_t)(3 * jd[col]);    // the same values from every column of the run
+            run[3 * my_run[k] + 1] = (uint16_t)(3 * jD[col]);
+            run[3 * my_run[k] + 2] = (uint16_t)(3 * js[col]);
+            atomicMax(&run_max[my_run[k]], __float_as_int(fabsf((float)pc[k])));
+        } else {
+            my_run[k] = 0;                                   // dead columns add a phase of 0 nobody reads
+        }
+    }
+    __syncthreads();
+    const int row_len = n_grid * 3, r3 = runs * 3;
+    const int wt = min(32, REDUCE_DM_BYTES / (r3 * 8));
     const int64_t w0 = (int64_t)blockIdx.y * per_block;
     const int64_t w1 = min(n_walkers, w0 + per_block);
     for (int64_t wb = w0; wb < w1; wb += wt) {
         const int nw = (int)min((int64_t)wt, w1 - wb);
-        __syncthreads();
-        const double* src = Y + (size_t)wb * row_len;
-        for (int i = threadIdx.x; i < nw * row_len; i += REDUCE_THREADS) sy[i] = src[i];
-        __syncthreads();
-        for (int w = 0; w < nw; ++w) {
-            const double* y = sy + w * row_len;
+        bool big = false;
+        for (int i = tid; i < nw * r3; i += THREADS) {
+            const int w = i / r3, j = i - w * r3, t = j / 3, ax = j - 3 * t;
+            const double* y = Y + (size_t)(wb + w) * row_len + ax;
+            const double dm = __dsub_rn(__dadd_rn(y[run[3 * t]], y[run[3 * t + 1]]), y[run[3 * t + 2]]);
+            dM[i] = dm;
+            big |= !(fabsf((float)dm) * __int_as_float(run_max[t]) < 127.0f);
+        }
+        if (!__syncthreads_or(big)) {
+            for (int w = 0; w < nw; ++w) {
 #pragma unroll
-            for (int k = 0; k < REDUCE_CPT; ++k) {
+                for (int k = 0; k < REDUCE_CPT; ++k) {
+                    if (k >= kmax) break;
+                    const double* m = dM + w * r3 + 3 * my_run[k];
 #pragma unroll
-                for (int ax = 0; ax < 3; ++ax) {
-                    const double dm = __dsub_rn(__dadd_rn(y[a[k] + ax], y[b[k] + ax]), y[c[k] + ax]);
-                    double s, co;
-                    sincos(__dmul_rn(pc[k], dm), &s, &co);
-                    cs[k] += co;
-                    sn[k] += s;
+                    for (int ax = 0; ax < 3; ++ax) add_cos_sin(__fma_rn(pc[k], m[ax], REDUCE_MAGIC), tab, ac[k], as[k]);
                 }
             }
+        } else {
+#pragma unroll
+            for (int k = 0; k < REDUCE_CPT; ++k) {
+                const int i = k * THREADS + tid;
+                if (i >= cols) break;
+                const double co = coef[col0 + i];
+                double cs = 0.0, sn = 0.0;
+                for (int j = 0; j < nw * 3; ++j) {
+                    double s, c;
+                    sincos(__dmul_rn(co, dM[j / 3 * r3 + 3 * my_run[k] + j % 3]), &s, &c);
+                    cs += c;
+                    sn += s;
+                }
+                ac[k] += __double2ll_rn(cs * (double)(1ll << REDUCE_Q));
+                as[k] += __double2ll_rn(sn * (double)(1ll << REDUCE_Q));
+            }
         }
+        __syncthreads();                                     // dM is rewritten
     }
+    const long long half = shift > 0 ? 1ll << (shift - 1) : 0ll;
 #pragma unroll
     for (int k = 0; k < REDUCE_CPT; ++k) {
-        const int col = blockIdx.x * REDUCE_COLS + k * REDUCE_THREADS + threadIdx.x;
-        if (col < n_cols && w1 > w0) {
-            atomicAdd(&accum[col], (unsigned long long)__double2ll_rn(cs[k] * 4294967296.0));
-            atomicAdd(&accum[n_cols + col], (unsigned long long)__double2ll_rn(sn[k] * 4294967296.0));
+        const int i = k * THREADS + tid;
+        if (i < cols && w1 > w0) {
+            atomicAdd(&accum[col0 + i], (unsigned long long)((ac[k] + half) >> shift));
+            atomicAdd(&accum[n_cols + col0 + i], (unsigned long long)((as[k] + half) >> shift));
         }
     }
 }
 
-__global__ void reduce_Y_finish_kernel(const long long* accum, int n_cols, double* cos_sum, double* sin_sum) {
+__global__ void reduce_Y_finish_kernel(const long long* accum, int n_cols, double unit, double* cos_sum, double* sin_sum) {
     const int col = blockIdx.x * blockDim.x + threadIdx.x;
     if (col >= n_cols) return;
-    cos_sum[col] = (double)accum[col] * 0x1p-32;
-    sin_sum[col] = (double)accum[n_cols + col] * 0x1p-32;
+    cos_sum[col] = (double)accum[col] * unit;
+    sin_sum[col] = (double)accum[n_cols + col] * unit;
 }
 
 }  // namespace madi
@@ -1019,30 +1150,38 @@ extern "C" madi_status madi_reduce_Y(const double* Y, int64_t n_walkers, int32_t
     unsigned long long* accum = static_cast<unsigned long long*>(scratch);
     cudaError_t e = cudaMemsetAsync(accum, 0, (size_t)madi_reduce_Y_scratch_bytes(n_cols), s);
     if (e != cudaSuccess) return host::cuda_fail(e, "reduce_Y memset");
+    // fraction bits of the column totals: 3 n_walkers 2^q < 2^63
+    int q = REDUCE_Q;
+    while (3.0 * (double)n_walkers * std::ldexp(1.0, q) >= 0x1p63) --q;
     if (n_walkers > 0) {
-        // walker rows staged per round: up to 96 KB of shared memory
-        const int row_bytes = n_grid * 3 * 8;
-        const int wt = std::max(1, std::min(32, (96 * 1024) / row_bytes));
-        const size_t smem = (size_t)wt * row_bytes;
-        e = cudaFuncSetAttribute(reduce_Y_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        // 512 threads hide the chain of a term better (31,125 columns x 50,000
+        // walkers: 12.0 ms against 13.0 ms at 256 threads x 4 columns); up to 512
+        // columns, 256 threads leave fewer of them idle (200 columns: 0.16 ms
+        // against 0.24 ms).
+        const int threads = n_cols <= 256 * REDUCE_CPT ? 256 : 512;
+        const auto kernel = threads == 256 ? reduce_Y_kernel<256> : reduce_Y_kernel<512>;
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, REDUCE_SMEM);
         if (e != cudaSuccess) return host::cuda_fail(e, "reduce_Y attribute");
         int dev = 0, sms = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        const int gx = (n_cols + REDUCE_COLS - 1) / REDUCE_COLS;
-        // about 4 CTAs per SM over all column blocks, each walker range a multiple of wt
-        const int64_t want = std::max<int64_t>(1, (4ll * sms + gx - 1) / gx);
-        int64_t per = (n_walkers + want - 1) / want;
-        per = std::max<int64_t>(wt, (per + wt - 1) / wt * wt);
-        const int64_t gy = (n_walkers + per - 1) / per;
-        if (gy > 65535) return host::fail(MADI_ERR_UNSUPPORTED, "reduce_Y: too many walker blocks");
-        reduce_Y_kernel<<<dim3((unsigned)gx, (unsigned)gy), REDUCE_THREADS, smem, s>>>(Y, n_walkers, n_grid, wt, per, jd, jD,
-                                                                                       js, coef, n_cols, accum);
+        const int gx = (n_cols + threads * REDUCE_CPT - 1) / (threads * REDUCE_CPT);
+        // Whole waves of two CTAs an SM; more waves even out the last one as long
+        // as a CTA keeps enough walkers to pay for its table (~3 us).
+        int64_t gy = 1;
+        for (int waves = 1; waves <= 4; waves *= 2) {
+            const int64_t y = std::max<int64_t>(1, (int64_t)waves * 2 * sms / gx);
+            if (waves == 1 || n_walkers / y >= 64) gy = y;
+        }
+        int64_t per = std::min<int64_t>((n_walkers + gy - 1) / gy, REDUCE_WALKERS);
+        gy = (n_walkers + per - 1) / per;
+        kernel<<<dim3((unsigned)gx, (unsigned)gy), threads, REDUCE_SMEM, s>>>(
+            Y, n_walkers, n_grid, per, jd, jD, js, coef, n_cols, REDUCE_Q - q, accum);
         e = cudaGetLastError();
         if (e != cudaSuccess) return host::cuda_fail(e, "reduce_Y launch");
     }
     reduce_Y_finish_kernel<<<(n_cols + 255) / 256, 256, 0, s>>>(reinterpret_cast<const long long*>(accum), n_cols,
-                                                                cos_sum, sin_sum);
+                                                                std::ldexp(1.0, -q), cos_sum, sin_sum);
     e = cudaGetLastError();
     if (e != cudaSuccess) return host::cuda_fail(e, "reduce_Y finish");
     return MADI_OK;
