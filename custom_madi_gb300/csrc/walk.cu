@@ -641,20 +641,64 @@ __global__ void __launch_bounds__(256, MINB) walk_f32_kernel(const madi_walk_des
 
 // ---------------------------------------------------------------------------
 // fp64 walker (madi/walker_gpu.py:520-585 design and :698-840 arithmetic:
-// separately rounded fp64, reference origin L/2, exact KD rule at every step,
-// Y stored).  One thread per walker of jobs[0]; it replays a fixed random
-// stream (golden check) or walks the fp32 walker's Philox numbers.
+// separately rounded fp64, reference origin L/2, Y stored).  One thread per
+// walker of jobs[0]; it replays a fixed random stream (golden check) or walks
+// the fp32 walker's Philox numbers.
+//
+// Labels are the exact KD rule's at every step.  The rule itself (a stackless
+// fp64 descent, a chain of dependent loads and fp64 operations per node) took
+// 97 % of the walk, so the label comes from the fp32 walker's facet planes where
+// their margins clear the error band (its allowance of 2^-21 L covers rounding
+// the fp64 point to fp32, sqrt(3) 2^-24 L), and from the KD rule in the rest
+// (~0.04 % of steps).  What remains is bound by the fp64 pipe: Box-Muller in
+// fp64, once per pair of steps.  16,000 walkers x 4,600 steps in a 64-cell box:
+// 888 ms before, 34 ms now.
 // ---------------------------------------------------------------------------
-// Normals of step `step` of walker widx from the Philox stream of the fp32
-// walker, in fp64 (Box-Muller: u1 = (w + 1/2) 2^-32, u2 = (w' >> 8) 2^-24), and
-// the step's acceptance word: the fp32 walker's random numbers, evaluated in
-// the reference's precision.
-MADI_DEV void normals_f64(uint32_t widx, int step, uint32_t k0, uint32_t k1, double (&n)[3], uint32_t& word) {
-    const uint32_t pair = (uint32_t)step >> 1;
+constexpr int F64_THREADS = 128;
+
+// Label of a point from the walker's cache: true when the three cached planes
+// decide (inside the cached sphere, no margin within its band).  Otherwise
+// `start` becomes the cell beyond the cached cell's nearest facet when the point
+// lies across it (an exact plane of that cell).
+template <bool PERIODIC>
+MADI_DEV bool cached_label(const TileShared& ts, float L, float qx, float qy, float qz, int& in, int& cell, int& start) {
+    const float4 sp = FC(3), ce = FC(4), f1 = FC(0), th = FC(5);
+    float wx = qx - ce.x, wy = qy - ce.y, wz = qz - ce.z;
+    if (PERIODIC) {
+        const float hl = 0.5f * L;
+        wx = wx > hl ? wx - L : (wx < -hl ? wx + L : wx);
+        wy = wy > hl ? wy - L : (wy < -hl ? wy + L : wy);
+        wz = wz > hl ? wz - L : (wz < -hl ? wz + L : wz);
+    }
+    const float m1 = facet_m(f1, wx, wy, wz);
+    const float ux = wx - sp.x, uy = wy - sp.y, uz = wz - sp.z;
+    if (fmaf(ux, ux, fmaf(uy, uy, uz * uz)) < sp.w) {
+        const float4 f2 = FC(1), f3 = FC(2);
+        const float mm = fminf(m1, fminf(facet_m(f2, wx, wy, wz), facet_m(f3, wx, wy, wz)));
+        if (mm > ce.w) { in = 1; cell = __float_as_int(th.z); return true; }
+        if (mm > th.y && mm < th.x) { in = 0; cell = __float_as_int(th.z); return true; }
+    }
+    const int nb1 = __float_as_int(th.w);
+    if (m1 < -th.y && nb1 >= 0) start = nb1;
+    return false;
+}
+
+// Empties the walker's label cache.
+MADI_DEV void clear_cache(const TileShared& ts) {
+    FC(0) = make_float4(0.f, 0.f, 0.f, 3.0e38f);
+    FC(3) = make_float4(0.f, 0.f, 0.f, 0.f);
+    FC(4) = make_float4(0.f, 0.f, 0.f, 0.f);
+    FC(5) = make_float4(0.f, 0.f, __int_as_float(-1), __int_as_float(-1));
+}
+
+// The six normals of step pair `pair` of walker widx from the Philox stream of
+// the fp32 walker, in fp64 (Box-Muller: u1 = (w + 1/2) 2^-32, u2 = (w' >> 8)
+// 2^-24; the first three are the even step's), and the two acceptance words: the
+// fp32 walker's random numbers, evaluated in the reference's precision.
+MADI_DEV void normals_f64(uint32_t widx, uint32_t pair, uint32_t k0, uint32_t k1, double (&gv)[6], uint32_t (&word)[2]) {
     const U4 ra = philox10(U4{widx, pair, 0u, 0u}, k0, k1);
     const U4 rb = philox10(U4{widx, pair, 1u, 0u}, k0, k1);
     const uint32_t wd[6] = {ra.x, ra.y, ra.z, ra.w, rb.x, rb.y};
-    double gv[6];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         const double u1 = __dadd_rn(__dmul_rn((double)wd[2 * k], 2.3283064365386963e-10), 1.1641532182693481e-10);
@@ -665,23 +709,27 @@ MADI_DEV void normals_f64(uint32_t widx, int step, uint32_t k0, uint32_t k1, dou
         gv[2 * k] = __dmul_rn(r, cs);
         gv[2 * k + 1] = __dmul_rn(r, sn);
     }
-    const bool odd = (step & 1) != 0;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) n[k] = odd ? gv[3 + k] : gv[k];
-    word = (step & 1) ? rb.w : rb.z;
+    word[0] = rb.z;
+    word[1] = rb.w;
 }
 
-__global__ void __launch_bounds__(128) walk_f64_kernel(const madi_walk_desc d) {
+__global__ void __launch_bounds__(F64_THREADS) walk_f64_kernel(const madi_walk_desc d) {
+    __shared__ float4 s_fc[FC_BYTES_PER_WALKER / 16 * F64_THREADS];
+    TileShared ts{};
+    ts.fc = s_fc;
     const madi_walk_job job = d.jobs[0];
-    const int w = blockIdx.x * blockDim.x + threadIdx.x;
-    if (w >= job.n_walkers) return;
+    const int lane = threadIdx.x & 31;
+    const int w0 = blockIdx.x * blockDim.x + threadIdx.x;
+    if (w0 - lane >= job.n_walkers) return;                  // whole warps only: the facet pass is warp-wide
+    const bool active = w0 < job.n_walkers;
+    const int w = active ? w0 : job.n_walkers - 1;           // spare lanes shadow the last walker, write nothing
     const madi_geometry gd = d.geoms[job.geom];
     const Geo g = make_geo(gd, reinterpret_cast<const unsigned char*>(gd.stage));
     const bool periodic = gd.boundary == MADI_BOUNDARY_PERIODIC;
     const bool cells = gd.has_cells != 0;
     const bool stream = d.rng == MADI_RNG_STREAM;
     const uint32_t widx = job.walker_base + (uint32_t)w;
-    const double L = gd.L, half_L = gd.L / 2.0, ts = d.ts, pp = job.pp;
+    const double L = gd.L, half_L = gd.L / 2.0, ts_ms = d.ts, pp = job.pp;
     const size_t row = (size_t)job.y_row + w;
     double px, py, pz;
     if (stream) {
@@ -698,6 +746,9 @@ __global__ void __launch_bounds__(128) walk_f64_kernel(const madi_walk_desc d) {
             if (pz >= L) pz = 0.0;
         }
     }
+    const bool facets = cells && gd.n_cells > 0;
+    const float Lf = (float)L;
+    clear_cache(ts);
     int cell = 0, inside = 0, escaped = 0, cerr = 0;
     uint32_t n_acc = 0, n_rej = 0, n_full = 0;
     if (cells) {
@@ -711,23 +762,35 @@ __global__ void __launch_bounds__(128) walk_f64_kernel(const madi_walk_desc d) {
     double Yx = 0.0, Yy = 0.0, Yz = 0.0;
     double* Yo = d.Y + row * d.n_grid * 3;
     int8_t* It = d.inside_trace + row * d.n_grid;
-    Yo[0] = Yo[1] = Yo[2] = 0.0;
-    It[0] = (int8_t)inside;
+    if (active) {
+        Yo[0] = Yo[1] = Yo[2] = 0.0;
+        It[0] = (int8_t)inside;
+    }
+    double gv[6];
+    uint32_t words[2] = {0u, 0u};
     for (int step = 0; step < d.n_steps; ++step) {
-        if (!escaped && !cerr) {
-            double inc[3], u = 0.0;
-            uint32_t word = 0;
+        const bool alive = active && !escaped && !cerr;
+        double qx = px, qy = py, qz = pz, u = 0.0;
+        int qkx = kx, qky = ky, qkz = kz;
+        uint32_t word = 0;
+        bool ok = alive;
+        if (alive) {
+            double inc[3];
             if (stream) {
                 const size_t o = (size_t)step * job.n_walkers + w;
                 inc[0] = d.incr[3 * o]; inc[1] = d.incr[3 * o + 1]; inc[2] = d.incr[3 * o + 2];
                 u = d.unif[o];
             } else {
-                normals_f64(widx, step, job.key0, job.key1, inc, word);
-                inc[0] = __dmul_rn(inc[0], d.sigma); inc[1] = __dmul_rn(inc[1], d.sigma); inc[2] = __dmul_rn(inc[2], d.sigma);
+                if ((step & 1) == 0) {
+                    normals_f64(widx, (uint32_t)step >> 1, job.key0, job.key1, gv, words);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 3; ++i) gv[i] = gv[3 + i];
+                }
+                word = words[step & 1];
+                inc[0] = __dmul_rn(gv[0], d.sigma); inc[1] = __dmul_rn(gv[1], d.sigma); inc[2] = __dmul_rn(gv[2], d.sigma);
             }
-            double qx = __dadd_rn(px, inc[0]), qy = __dadd_rn(py, inc[1]), qz = __dadd_rn(pz, inc[2]);
-            int qkx = kx, qky = ky, qkz = kz;
-            bool ok = true;
+            qx = __dadd_rn(px, inc[0]); qy = __dadd_rn(py, inc[1]); qz = __dadd_rn(pz, inc[2]);
             if (periodic) {
                 if (qx < 0.0) { qx = __dadd_rn(qx, L); --qkx; }
                 if (qx >= L) { qx = __dsub_rn(qx, L); ++qkx; }
@@ -739,61 +802,79 @@ __global__ void __launch_bounds__(128) walk_f64_kernel(const madi_walk_desc d) {
                 escaped = 1;
                 ok = false;
             }
-            if (ok) {
-                int ncell = 0, nin = 0;
-                if (cells) {
-                    int s1 = 0;
-                    if (classify_kd_f64(g, qx, qy, qz, s1, nin) != CLS_OK) { cerr = 1; }
-                    ncell = g.cell[s1];
-                    ++n_full;
-                }
-                if (!cerr) {
-                    int m = 0;
-                    if (inside && !nin) m = 1;
-                    else if (!inside && nin) m = 1;
-                    else if (inside && nin && cell != ncell) m = 2;
-                    bool accept = true;
-                    if (m > 0 && pp < 1.0) {
-                        if (stream) {
-                            const double thr = m == 1 ? pp : __dmul_rn(pp, pp);
-                            accept = !(u >= thr);
-                        } else {            // 64-bit uniform against floor(pp^m 2^64), as the fp32 walker
-                            const uint64_t thr = m == 1 ? job.thr1 : job.thr2;
-                            const uint32_t th = (uint32_t)(thr >> 32);
-                            if (word != th) {
-                                accept = word < th;
-                            } else {
-                                const U4 rc = philox10(U4{widx, (uint32_t)step, 2u, 0u}, job.key0, job.key1);
-                                accept = rc.x < (uint32_t)thr;
-                            }
+        }
+        // ---- label: facet planes (cache, then a warp-wide pass), else the KD rule ----
+        int ncell = 0, nin = 0;
+        bool known = !cells;
+        if (facets) {
+            const float fx = (float)qx, fy = (float)qy, fz = (float)qz;
+            // a step longer than the box leaves a periodic point outside after one wrap
+            const bool boxed = ok && fminf(fx, fminf(fy, fz)) >= 0.f && fmaxf(fx, fmaxf(fy, fz)) <= Lf;
+            int start = cell;
+            if (boxed) known = periodic ? cached_label<true>(ts, Lf, fx, fy, fz, nin, ncell, start)
+                                        : cached_label<false>(ts, Lf, fx, fy, fz, nin, ncell, start);
+            const bool miss = boxed && !known;
+            if (__any_sync(MADI_FULL, miss)) {
+                int cq = start;
+                const int r = periodic ? coop_facets<true>(g, ts, miss, fx, fy, fz, start, lane, cq)
+                                       : coop_facets<false>(g, ts, miss, fx, fy, fz, start, lane, cq);
+                if (miss && r >= 0) { known = true; nin = r; ncell = cq; }
+            }
+        }
+        if (ok) {
+            if (!known) {
+                int s1 = 0;
+                if (classify_kd_f64(g, qx, qy, qz, s1, nin) != CLS_OK) { cerr = 1; }
+                ncell = g.cell[s1];
+            }
+            if (cells) ++n_full;
+            if (!cerr) {
+                int m = 0;
+                if (inside && !nin) m = 1;
+                else if (!inside && nin) m = 1;
+                else if (inside && nin && cell != ncell) m = 2;
+                bool accept = true;
+                if (m > 0 && pp < 1.0) {
+                    if (stream) {
+                        const double thr = m == 1 ? pp : __dmul_rn(pp, pp);
+                        accept = !(u >= thr);
+                    } else {            // 64-bit uniform against floor(pp^m 2^64), as the fp32 walker
+                        const uint64_t thr = m == 1 ? job.thr1 : job.thr2;
+                        const uint32_t th = (uint32_t)(thr >> 32);
+                        if (word != th) {
+                            accept = word < th;
+                        } else {
+                            const U4 rc = philox10(U4{widx, (uint32_t)step, 2u, 0u}, job.key0, job.key1);
+                            accept = rc.x < (uint32_t)thr;
                         }
-                        if (accept) ++n_acc; else ++n_rej;
                     }
-                    if (accept) {
-                        px = qx; py = qy; pz = qz; kx = qkx; ky = qky; kz = qkz;
-                        cell = ncell; inside = nin;
-                    }
-                    double xn = __dsub_rn(px, half_L), yn = __dsub_rn(py, half_L), zn = __dsub_rn(pz, half_L);
-                    if (periodic) {
-                        xn = __dadd_rn(xn, __dmul_rn((double)kx, L));
-                        yn = __dadd_rn(yn, __dmul_rn((double)ky, L));
-                        zn = __dadd_rn(zn, __dmul_rn((double)kz, L));
-                    }
-                    Yx = __dadd_rn(Yx, __dmul_rn(__dmul_rn(0.5, __dadd_rn(xp, xn)), ts));
-                    Yy = __dadd_rn(Yy, __dmul_rn(__dmul_rn(0.5, __dadd_rn(yp, yn)), ts));
-                    Yz = __dadd_rn(Yz, __dmul_rn(__dmul_rn(0.5, __dadd_rn(zp, zn)), ts));
-                    xp = xn; yp = yn; zp = zn;
+                    if (accept) ++n_acc; else ++n_rej;
                 }
+                if (accept) {
+                    px = qx; py = qy; pz = qz; kx = qkx; ky = qky; kz = qkz;
+                    cell = ncell; inside = nin;
+                }
+                double xn = __dsub_rn(px, half_L), yn = __dsub_rn(py, half_L), zn = __dsub_rn(pz, half_L);
+                if (periodic) {
+                    xn = __dadd_rn(xn, __dmul_rn((double)kx, L));
+                    yn = __dadd_rn(yn, __dmul_rn((double)ky, L));
+                    zn = __dadd_rn(zn, __dmul_rn((double)kz, L));
+                }
+                Yx = __dadd_rn(Yx, __dmul_rn(__dmul_rn(0.5, __dadd_rn(xp, xn)), ts_ms));
+                Yy = __dadd_rn(Yy, __dmul_rn(__dmul_rn(0.5, __dadd_rn(yp, yn)), ts_ms));
+                Yz = __dadd_rn(Yz, __dmul_rn(__dmul_rn(0.5, __dadd_rn(zp, zn)), ts_ms));
+                xp = xn; yp = yn; zp = zn;
             }
         }
         const int si = step + 1;
-        if (si % d.steps_per_h == 0) {
+        if (active && si % d.steps_per_h == 0) {
             const int j = si / d.steps_per_h;
             Yo[3 * j] = Yx; Yo[3 * j + 1] = Yy; Yo[3 * j + 2] = Yz;
             It[j] = (int8_t)inside;
             if (inside) atomicAdd(reinterpret_cast<unsigned long long*>(&d.occupancy[(size_t)job.slot * d.n_grid + j]), 1ull);
         }
     }
+    if (!active) return;
     uint64_t* cnt = d.counters + (size_t)job.slot * MADI_CNT_N;
     atomicAdd(reinterpret_cast<unsigned long long*>(&cnt[MADI_CNT_WALKERS]), 1ull);
     if (escaped) atomicAdd(reinterpret_cast<unsigned long long*>(&cnt[MADI_CNT_ESCAPED]), 1ull);
@@ -1094,7 +1175,7 @@ extern "C" madi_status madi_walk(const madi_walk_desc* d, void* stream) {
         if (!d->Y || !d->inside_trace) return host::fail(MADI_ERR_INVALID, "fp64 walker writes Y and inside_trace");
         // The job is read on the device; the host only needs its walker count, passed as n_tiles * 128 bound.
         const int blocks = d->n_tiles;
-        walk_f64_kernel<<<blocks, 128, 0, s>>>(*d);
+        walk_f64_kernel<<<blocks, F64_THREADS, 0, s>>>(*d);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return host::cuda_fail(e, "fp64 walker launch");
         return MADI_OK;

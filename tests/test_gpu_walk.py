@@ -366,3 +366,35 @@ def test_reference_design_path_matches_oracle_signal():
     assert not np.isnan(want).any()
     assert np.max(np.abs(got - want)) <= 1e-9 * 1000, np.max(np.abs(got - want))
     assert np.array_equal(r["occupancy"], out["occupancy"])
+
+
+@pytest.mark.parametrize("n_walkers, n_cells, rho, V", [
+    (1, 2, 2.0e5, 4.0),        # one lane of a warp; two cells, cells that face their own images
+    (33, 27, 5.0e7, 0.017),    # one lane past a warp; steps a sixth of the cell spacing
+    (161, 64, 2.0e5, 2.6),     # past a block; thick extracellular space
+])
+def test_f64_walker_labels_equal_kd_rule(n_walkers, n_cells, rho, V):
+    """The fp64 walk labels every step as the fp64 KD rule does: with the facet
+    table taken away (n_cells = 0) the same walk runs on the KD rule alone, and
+    every stored Y, inside flag and crossing count is the same bit for bit."""
+    import torch
+    from custom_madi_gb300 import _native as N
+    from custom_madi_gb300.config import SimConfig
+    from custom_madi_gb300.ensemble import create_ensemble
+    from custom_madi_gb300.walker_gpu import WalkBatch, WalkJob
+    cfg = SimConfig(boundary_mode="periodic", n_cells=n_cells, n_walkers=n_walkers, n_ensembles=1, ts=0.01, T_max_ms=4.0,
+                    small_deltas=[1.0], big_deltas=[2.0], b_values=[0.0, 1000.0])
+    ens = create_ensemble(rho, V, cfg, seed=5, verify_vi=False, measure_vi=False)
+    out = []
+    for table in (True, False):
+        ens._device.clear()
+        dev = ens.device()
+        if not table:
+            dev.struct.n_cells = 0
+        b = WalkBatch([WalkJob(ens, 0.2, 11, n_walkers)], cfg, out_mode=N.MADI_OUT_Y, precision=64)
+        b.launch()
+        torch.cuda.synchronize()
+        out.append((b.Y.cpu().numpy(), b.inside_trace.cpu().numpy(), b.counters_np(), b.occupancy.cpu().numpy()))
+    ens._device.clear()
+    for x, y in zip(*out):
+        assert np.array_equal(x, y)
