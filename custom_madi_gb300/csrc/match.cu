@@ -1,86 +1,51 @@
 // Library match (MAP nearest library entry per voxel), replacing
 // _map_kernel_fixed / _map_kernel_free_s0 (madi/fitters_gpu.py:96-154).
 //
-// FP32 path: exhaustive fp32 scan on the CUDA cores, library streamed through
-// shared memory in chunks, one voxel per thread.  Fixed S0 scores the centred
-// pair (m - mu, L_j - mu), mu the library column mean: the uncentred expanded
-// form |L_j|^2 - 2 m.L_j rounds at ~|L|^2 2^-24, coarser than the gap between
+// FP32 path, fp32 scores on the CUDA cores.  Fixed S0 scores the centred pair
+// (m - mu, L_j - mu), mu the library column mean: the uncentred expanded form
+// |L_j|^2 - 2 m.L_j rounds at ~|L|^2 2^-24, coarser than the gap between
 // near-tied entries of a dense library, while the centred form rounds at
-// ~|L - mu|^2 2^-24.
+// ~|L - mu|^2 2^-24.  The choice is the lowest score, the lowest index among
+// equal ones, whichever kernel finds it:
+//   match_pruned_kernel  large fits: library tiles that cannot hold the winner
+//                        are skipped (prune.cuh);
+//   match_scan_kernel    every pair; small fits split the library over CTAs.
+#include <algorithm>
 #include <cstdint>
 #include "madi_device.cuh"
 #include "madi_host.h"
+#include "prune.cuh"
 
 namespace madi {
 
-constexpr int MATCH_THREADS = 256;
+constexpr int MATCH_THREADS = 128;
 constexpr int MATCH_CHUNK = 128;
+constexpr float NO_SCORE = 3.0e38f;
 
-// fixed S0: score_j = |L_j - mu|^2 - 2 (m - mu).(L_j - mu) = |m - L_j|^2 - |m - mu|^2 ;
-// free S0: score_j = -(m.r)^2/|r|^2 when m.r > 0 (mu unused).
-template <int FMAX, int MODE>
-__global__ void __launch_bounds__(MATCH_THREADS) match_fp32_kernel(const float* __restrict__ meas,
-                                                                   const float* __restrict__ lib,
-                                                                   const float* __restrict__ mu, int64_t n_vox,
-                                                                   int n_lib, int n_feat, int32_t* best_idx,
-                                                                   float* best_resid, float* best_s0) {
-    __shared__ float sl[MATCH_CHUNK][FMAX];
-    __shared__ float sn[MATCH_CHUNK];
-    __shared__ float smu[FMAX];
-    const int64_t v = (int64_t)blockIdx.x * MATCH_THREADS + threadIdx.x;
-    if (threadIdx.x < FMAX)
-        smu[threadIdx.x] = (MODE == MADI_MATCH_FIXED_S0 && (int)threadIdx.x < n_feat) ? mu[threadIdx.x] : 0.f;
-    __syncthreads();
-    float m[FMAX];
-#pragma unroll
-    for (int f = 0; f < FMAX; ++f) m[f] = (v < n_vox && f < n_feat) ? meas[v * n_feat + f] - smu[f] : 0.f;
-    float best = 3.0e38f;
-    int bj = 0;
-    for (int base = 0; base < n_lib; base += MATCH_CHUNK) {
-        const int cnt = min(MATCH_CHUNK, n_lib - base);
-        __syncthreads();
-        for (int t = threadIdx.x; t < MATCH_CHUNK * FMAX; t += MATCH_THREADS) {
-            const int e = t / FMAX, f = t - e * FMAX;
-            sl[e][f] = (e < cnt && f < n_feat) ? lib[(int64_t)(base + e) * n_feat + f] - smu[f] : 0.f;
-        }
-        __syncthreads();
-        if (threadIdx.x < MATCH_CHUNK) {
-            float s = 0.f;
-#pragma unroll
-            for (int f = 0; f < FMAX; ++f) s = fmaf(sl[threadIdx.x][f], sl[threadIdx.x][f], s);
-            sn[threadIdx.x] = MODE == MADI_MATCH_FREE_S0 ? fmaxf(s, 1e-30f) : s;
-        }
-        __syncthreads();
-        for (int e = 0; e < cnt; ++e) {
-            float dot = 0.f;
-#pragma unroll
-            for (int f = 0; f < FMAX; ++f) dot = fmaf(m[f], sl[e][f], dot);
-            float score;
-            if (MODE == MADI_MATCH_FIXED_S0) {
-                score = fmaf(-2.f, dot, sn[e]);
-            } else {
-                score = dot > 0.f ? -(dot * dot) / sn[e] : 3.0e38f;
-            }
-            if (score < best) { best = score; bj = base + e; }
-        }
-    }
-    if (v >= n_vox) return;
-    // Residual of the chosen entry from the direct difference of the raw data.
-#pragma unroll
-    for (int f = 0; f < FMAX; ++f) m[f] = f < n_feat ? meas[v * n_feat + f] : 0.f;
+// (score, index) as one word that orders like the pair; -0 and 0 are equal scores.
+MADI_DEV unsigned long long match_key(float score, int j) {
+    const uint32_t o = (uint32_t)f2o(score + 0.0f) ^ 0x80000000u;
+    return ((unsigned long long)o << 32) | (uint32_t)j;
+}
+
+// Residual of the chosen entry from the direct difference of the raw data.
+template <int N, int MODE>
+MADI_DEV void match_write(const float* __restrict__ meas, const float* __restrict__ lib, int64_t v, int bj, int n_feat,
+                          int32_t* best_idx, float* best_resid, float* best_s0) {
+    const float* M = meas + v * n_feat;
     const float* L = lib + (int64_t)bj * n_feat;
     float dot = 0.f, rr = 0.f;
 #pragma unroll
-    for (int f = 0; f < FMAX; ++f) {
-        if (f < n_feat) { dot = fmaf(m[f], L[f], dot); rr = fmaf(L[f], L[f], rr); }
+    for (int f = 0; f < N; ++f) {
+        if (f < n_feat) { dot = fmaf(M[f], L[f], dot); rr = fmaf(L[f], L[f], rr); }
     }
     float s0 = 1.f;
     if (MODE == MADI_MATCH_FREE_S0) s0 = dot / fmaxf(rr, 1e-30f);
     float res = 0.f;
 #pragma unroll
-    for (int f = 0; f < FMAX; ++f) {
+    for (int f = 0; f < N; ++f) {
         if (f < n_feat) {
-            const float r = m[f] - s0 * L[f];
+            const float r = M[f] - s0 * L[f];
             res = fmaf(r, r, res);
         }
     }
@@ -90,18 +55,374 @@ __global__ void __launch_bounds__(MATCH_THREADS) match_fp32_kernel(const float* 
     if (MODE == MADI_MATCH_FREE_S0 && best_s0) best_s0[v] = s0;
 }
 
-template <int FMAX>
-static madi_status launch_fp32(const madi_match_desc* d, float* mu, cudaStream_t s) {
-    const int64_t blocks = (d->n_vox + MATCH_THREADS - 1) / MATCH_THREADS;
-    if (d->mode == MADI_MATCH_FIXED_S0)
-        match_fp32_kernel<FMAX, MADI_MATCH_FIXED_S0><<<(unsigned)blocks, MATCH_THREADS, 0, s>>>(
-            d->measured, d->lib, mu, d->n_vox, d->n_lib, d->n_feat, d->best_idx, d->best_resid, d->best_s0);
-    else
-        match_fp32_kernel<FMAX, MADI_MATCH_FREE_S0><<<(unsigned)blocks, MATCH_THREADS, 0, s>>>(
-            d->measured, d->lib, nullptr, d->n_vox, d->n_lib, d->n_feat, d->best_idx, d->best_resid, d->best_s0);
+// Fixed S0 score_j = |L_j - mu|^2 - 2 (m - mu).(L_j - mu) = |m - L_j|^2 - |m - mu|^2;
+// free S0 score_j = -(m.r)^2 / |r|^2 when m.r > 0.  The free score's division is
+// only made for pairs that may reach the best so far: dot^2 >= bar |r|^2, bar
+// 4e-7 below the best (the rounding on both sides is below 2e-7), 0 where the
+// best is subnormal or there is none.
+MADI_DEV float free_bar(float best) { return best < -1e-36f ? -best * (1.f - 4e-7f) : 0.f; }
+MADI_DEV bool free_may_win(float dot, float sn, float bar) {
+    return dot > 0.f && fmaxf(dot * dot, 1e-36f) >= bar * sn;
+}
+
+template <int MODE>
+MADI_DEV void match_pair(float dot, float sn, int j, float& best, int& bj, float& bar) {
+    if (MODE == MADI_MATCH_FIXED_S0) {
+        const float score = fmaf(-2.f, dot, sn);
+        if (score < best) { best = score; bj = j; }
+    } else if (free_may_win(dot, sn, bar)) {
+        const float score = -(dot * dot) / sn;
+        if (score < best) { best = score; bj = j; bar = free_bar(best); }
+    }
+}
+
+// Every pair: the library (or the part blockIdx.y of it) streams through shared
+// memory, V voxels per thread so that one 16-byte shared load feeds 4 V fused
+// multiply-adds (with one voxel a thread the shared-memory pipe, not the FMA
+// pipe, was the limit).  keys != null: the part's winners meet in a 64-bit
+// minimum per voxel and match_finish_kernel writes the results.
+template <int N, int MODE, int V>
+__global__ void __launch_bounds__(MATCH_THREADS) match_scan_kernel(const float* __restrict__ meas,
+                                                                   const float* __restrict__ lib,
+                                                                   const float* __restrict__ mu, int64_t n_vox,
+                                                                   int n_lib, int n_feat, int part,
+                                                                   unsigned long long* keys, int32_t* best_idx,
+                                                                   float* best_resid, float* best_s0) {
+    __shared__ float4 sl[MATCH_CHUNK][N / 4];
+    __shared__ float sn[MATCH_CHUNK];
+    __shared__ float smu[N];
+    const int64_t v0 = (int64_t)blockIdx.x * (MATCH_THREADS * V) + threadIdx.x;
+    if (threadIdx.x < N)
+        smu[threadIdx.x] = (MODE == MADI_MATCH_FIXED_S0 && (int)threadIdx.x < n_feat) ? mu[threadIdx.x] : 0.f;
+    __syncthreads();
+    float m[V][N];
+    float best[V], bar[V];
+    int bj[V];
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+        const int64_t v = v0 + i * MATCH_THREADS;
+#pragma unroll
+        for (int f = 0; f < N; ++f) m[i][f] = (v < n_vox && f < n_feat) ? meas[v * n_feat + f] - smu[f] : 0.f;
+        best[i] = NO_SCORE;
+        bar[i] = 0.f;
+        bj[i] = 0;
+    }
+    const int j0 = blockIdx.y * part, j1 = min(n_lib, j0 + part);
+    for (int base = j0; base < j1; base += MATCH_CHUNK) {
+        const int cnt = min(MATCH_CHUNK, j1 - base);
+        __syncthreads();
+        float* flat = reinterpret_cast<float*>(sl);
+        for (int t = threadIdx.x; t < cnt * n_feat; t += MATCH_THREADS) {
+            const int e = t / n_feat, f = t - e * n_feat;
+            flat[e * N + f] = lib[(int64_t)base * n_feat + t] - smu[f];
+        }
+        for (int t = threadIdx.x; t < cnt * (N - n_feat); t += MATCH_THREADS) {
+            const int e = t / (N - n_feat), f = n_feat + t - e * (N - n_feat);
+            flat[e * N + f] = 0.f;
+        }
+        __syncthreads();
+        if ((int)threadIdx.x < cnt) {
+            float s = 0.f;
+#pragma unroll
+            for (int f = 0; f < N / 4; ++f) {
+                const float4 l = sl[threadIdx.x][f];
+                s = fmaf(l.x, l.x, s); s = fmaf(l.y, l.y, s); s = fmaf(l.z, l.z, s); s = fmaf(l.w, l.w, s);
+            }
+            sn[threadIdx.x] = MODE == MADI_MATCH_FREE_S0 ? fmaxf(s, 1e-30f) : s;
+        }
+        __syncthreads();
+#pragma unroll 2
+        for (int e = 0; e < cnt; ++e) {
+            float dot[V];
+#pragma unroll
+            for (int i = 0; i < V; ++i) dot[i] = 0.f;
+#pragma unroll
+            for (int f = 0; f < N / 4; ++f) {
+                const float4 l = sl[e][f];
+#pragma unroll
+                for (int i = 0; i < V; ++i) {
+                    dot[i] = fmaf(m[i][4 * f], l.x, dot[i]);
+                    dot[i] = fmaf(m[i][4 * f + 1], l.y, dot[i]);
+                    dot[i] = fmaf(m[i][4 * f + 2], l.z, dot[i]);
+                    dot[i] = fmaf(m[i][4 * f + 3], l.w, dot[i]);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < V; ++i) match_pair<MODE>(dot[i], sn[e], base + e, best[i], bj[i], bar[i]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+        const int64_t v = v0 + i * MATCH_THREADS;
+        if (v >= n_vox) continue;
+        if (keys) atomicMin(&keys[v], match_key(best[i], bj[i]));
+        else match_write<N, MODE>(meas, lib, v, bj[i], n_feat, best_idx, best_resid, best_s0);
+    }
+}
+
+template <int N, int MODE>
+__global__ void __launch_bounds__(256) match_finish_kernel(const float* __restrict__ meas, const float* __restrict__ lib,
+                                                           const unsigned long long* __restrict__ keys, int64_t n_vox,
+                                                           int n_feat, int32_t* best_idx, float* best_resid,
+                                                           float* best_s0) {
+    const int64_t v = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    if (v < n_vox) match_write<N, MODE>(meas, lib, v, (int)(uint32_t)keys[v], n_feat, best_idx, best_resid, best_s0);
+}
+
+// ---------------------------------------------------------------------------
+// Pruned search.  A warp takes 64 voxels that are neighbours in the index's
+// order (two per lane), scans the tile nearest to them, then every tile that
+// some voxel still needs: first by the box of the warp's voxels (32 tiles at a
+// time, one per lane), then voxel by voxel.
+//
+// Why nothing is missed: with d the box distance in the embedding, every entry
+// of the tile has |m - L|^2 >= d^2 (1-Lipschitz), so its exact score is at least
+// d^2 - |m|^2 (fixed S0), and |cos| <= 1 - d^2 / 2 between unit rows (free S0).
+// The fp32 score is off by at most (F + 2) 2^-24 (|m|^2 + 2 |L|^2) (two dot
+// products), the fp32 embedding by (F + 8) 2^-23 (|m| + |L|) per coordinate, and
+// the directions are orthonormal to 1e-5: 0.998 d^2 and the margin E = (F + 8)
+// 2^-21 (|m|^2 + max |L|^2) cover them together ((a + b)^2 <= 1.001 a^2 + 1001
+// b^2).  A tile is skipped only if the bound lies strictly above the best score,
+// so ties keep the lowest index.  Where fp32 scores can overflow, or the free
+// score's dot^2 become subnormal, the bound says nothing: those voxels (and ones
+// that are not finite) skip nothing.
+// ---------------------------------------------------------------------------
+struct PrunedVoxel {
+    float m2, e, limit, best;
+    int bj;
+    bool bounded;
+};
+
+template <int MODE>
+MADI_DEV void set_limit(PrunedVoxel& v) {
+    if (MODE == MADI_MATCH_FIXED_S0) {
+        v.limit = v.best + v.m2 + v.e;
+    } else {
+        const float s = v.best < 0.f ? fmaxf(-v.best / v.m2 - v.e, 0.f) : 0.f;     // cos^2 to beat
+        v.limit = 2.f * (1.f - sqrtf(s)) + 4e-6f;
+    }
+    if (!v.bounded || !(v.limit < NO_SCORE)) v.limit = __int_as_float(0x7f800000);
+}
+
+MADI_DEV float warp_minf32(float v) { float r; asm("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v)); return r; }
+MADI_DEV float warp_maxf32(float v) { float r; asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v)); return r; }
+
+// Squared distance between the boxes [lo, hi] and the tile's.
+MADI_DEV float box_distance2(const float4* __restrict__ b, const float (&lo)[6], const float (&hi)[6]) {
+    const float4 l0 = b[0], l1 = b[1], h0 = b[2], h1 = b[3];
+    const float tl[6] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y}, th[6] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y};
+    float d2 = 0.f;
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+        const float d = fmaxf(fmaxf(tl[k] - hi[k], lo[k] - th[k]), 0.f);
+        d2 = fmaf(d, d, d2);
+    }
+    return d2;
+}
+
+template <int N, int MODE>
+MADI_DEV void scan_tile(const float4* __restrict__ rows, const float (&ma)[N], const float (&mb)[N], PrunedVoxel& a,
+                        PrunedVoxel& b) {
+    // winners of the tile alone (its entries are in index order), then against the
+    // best so far; the free score's bar starts from the best so far
+    float ta = NO_SCORE, tb = NO_SCORE;
+    float bara = MODE == MADI_MATCH_FIXED_S0 ? 0.f : free_bar(a.best), barb = MODE == MADI_MATCH_FIXED_S0 ? 0.f : free_bar(b.best);
+    int ja = -1, jb = -1;
+#pragma unroll 2
+    for (int e = 0; e < prune::TILE; ++e) {
+        const float4* r = rows + e * (N / 4 + 1);
+        float da = 0.f, db = 0.f;
+#pragma unroll
+        for (int f = 0; f < N / 4; ++f) {
+            const float4 l = r[f];
+            da = fmaf(ma[4 * f], l.x, da); da = fmaf(ma[4 * f + 1], l.y, da);
+            da = fmaf(ma[4 * f + 2], l.z, da); da = fmaf(ma[4 * f + 3], l.w, da);
+            db = fmaf(mb[4 * f], l.x, db); db = fmaf(mb[4 * f + 1], l.y, db);
+            db = fmaf(mb[4 * f + 2], l.z, db); db = fmaf(mb[4 * f + 3], l.w, db);
+        }
+        const float4 x = r[N / 4];
+        const int j = __float_as_int(x.y);
+        match_pair<MODE>(da, x.x, j, ta, ja, bara);
+        match_pair<MODE>(db, x.x, j, tb, jb, barb);
+    }
+    if (ja >= 0 && (ta < a.best || (ta == a.best && ja < a.bj))) { a.best = ta; a.bj = ja; }
+    if (jb >= 0 && (tb < b.best || (tb == b.best && jb < b.bj))) { b.best = tb; b.bj = jb; }
+    set_limit<MODE>(a);
+    set_limit<MODE>(b);
+}
+
+template <int N, int MODE>
+__global__ void __launch_bounds__(MATCH_THREADS, N <= 16 ? 4 : 3) match_pruned_kernel(const float* __restrict__ meas,
+                                                                        const float* __restrict__ lib,
+                                                                        const prune::Index ix, int32_t* best_idx,
+                                                                        float* best_resid, float* best_s0) {
+    __shared__ float sv[prune::B_FLOATS], smu[N];
+    for (int i = threadIdx.x; i < prune::B_FLOATS; i += MATCH_THREADS) sv[i] = ix.basis[i];
+    if (threadIdx.x < N)
+        smu[threadIdx.x] = (MODE == MADI_MATCH_FIXED_S0 && (int)threadIdx.x < ix.F) ? ix.mu[threadIdx.x] : 0.f;
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    const int64_t p0 = ((int64_t)blockIdx.x * (MATCH_THREADS / 32) + (threadIdx.x >> 5)) * 64;
+    if (p0 >= ix.n_vox) return;
+    const float slack = (float)(ix.F + 8) * 4.76837158203125e-07f;             // (F + 8) 2^-21
+    const float lmax = ix.lmax[0], inv_lmin = ix.lmax[1];
+    int64_t vox[2];
+    float m[2][N], phi[2][6];
+    PrunedVoxel pv[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        vox[i] = ix.vperm[min(p0 + 32 * i + lane, ix.n_vox - 1)];
+        PrunedVoxel& v = pv[i];
+        v.m2 = 0.f;
+#pragma unroll
+        for (int f = 0; f < N; ++f) {
+            m[i][f] = f < ix.F ? meas[vox[i] * ix.F + f] - smu[f] : 0.f;
+            v.m2 = fmaf(m[i][f], m[i][f], v.m2);
+        }
+        prune::Phi e;
+        if (MODE == MADI_MATCH_FIXED_S0) {
+            e = prune::embed(m[i], sv);
+            v.e = slack * (v.m2 + lmax);
+            v.bounded = v.m2 + lmax < 1e36f;
+        } else {
+            float u[N];
+            const float sc = v.m2 > 0.f ? rsqrtf(v.m2) : 0.f;
+#pragma unroll
+            for (int f = 0; f < N; ++f) u[f] = f < ix.F ? fmaf(m[i][f], sc, -sv[prune::B_CENTRE + f]) : 0.f;
+            e = prune::embed(u, sv);
+            v.e = slack;
+            v.bounded = v.m2 < 1e36f && v.m2 * lmax < 1e36f && v.m2 > 1e-32f * inv_lmin;
+        }
+#pragma unroll
+        for (int k = 0; k < prune::KDIR; ++k) phi[i][k] = e.p[k];
+        phi[i][5] = e.q;
+        v.best = NO_SCORE;
+        v.bj = 0;
+        set_limit<MODE>(v);
+    }
+    const float4* boxes = reinterpret_cast<const float4*>(ix.box);
+    const float4* rows = reinterpret_cast<const float4*>(ix.rows);
+    const int tile_rows = prune::TILE * (N / 4 + 1);
+    // ---- the tile nearest to one of the warp's voxels ----
+    float c[6], glo[6], ghi[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+        c[k] = __shfl_sync(MADI_FULL, phi[0][k], 16);
+        glo[k] = warp_minf32(fminf(phi[0][k], phi[1][k]));
+        ghi[k] = warp_maxf32(fmaxf(phi[0][k], phi[1][k]));
+    }
+    float near = NO_SCORE;
+    int t0 = 0;
+    for (int t = lane; t < ix.n_tiles; t += 32) {
+        const float d = box_distance2(boxes + 4ll * t, c, c);
+        if (d < near) { near = d; t0 = t; }
+    }
+    {
+        const float best = warp_minf32(near);
+        const unsigned who = __ballot_sync(MADI_FULL, near == best);
+        t0 = __shfl_sync(MADI_FULL, t0, who ? __ffs(who) - 1 : 0);
+    }
+    scan_tile<N, MODE>(rows + (int64_t)t0 * tile_rows, m[0], m[1], pv[0], pv[1]);
+    // ---- every other tile some voxel still needs ----
+    for (int base = 0; base < ix.n_tiles; base += 32) {
+        const float top = warp_maxf32(fmaxf(pv[0].limit, pv[1].limit));
+        const int mine = base + lane;
+        bool want = false;
+        if (mine < ix.n_tiles && mine != t0) want = !(0.998f * box_distance2(boxes + 4ll * mine, glo, ghi) > top);
+        for (unsigned mask = __ballot_sync(MADI_FULL, want); mask; mask &= mask - 1) {
+            const int t = base + __ffs(mask) - 1;
+            const float4* b = boxes + 4ll * t;
+            const bool need = !(0.998f * box_distance2(b, phi[0], phi[0]) > pv[0].limit) ||
+                              !(0.998f * box_distance2(b, phi[1], phi[1]) > pv[1].limit);
+            if (__any_sync(MADI_FULL, need)) scan_tile<N, MODE>(rows + (int64_t)t * tile_rows, m[0], m[1], pv[0], pv[1]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+        if (p0 + 32 * i + lane < ix.n_vox)
+            match_write<N, MODE>(meas, lib, vox[i], pv[i].bj, ix.F, best_idx, best_resid, best_s0);
+}
+
+// ---------------------------------------------------------------------------
+// Which kernel (fp32)
+// ---------------------------------------------------------------------------
+struct MatchPlan {
+    bool pruned;
+    int parts;                  // library parts of the exhaustive scan
+    int part;                   // entries a part
+    int64_t bytes;              // scratch beyond the column means
+};
+
+static MatchPlan match_plan(int64_t n_vox, int32_t n_lib, int32_t n_feat) {
+    MatchPlan p{false, 1, n_lib, 0};
+    // The index costs ~0.1 ms; below ~4e9 products the scan is done by then.
+    if (n_vox >= 4096 && n_lib >= 1024 && (double)n_vox * n_lib * n_feat >= 4e9 && n_vox < 0x7fffffff) {
+        p.pruned = true;
+        prune::Index ix;
+        p.bytes = prune::layout(ix, nullptr, n_vox, n_lib, n_feat);
+        return p;
+    }
+    // Small fits leave most SMs idle with one CTA per 128 voxels: about eight
+    // CTAs an SM (1,216 of 152 SMs), a part no shorter than a chunk.
+    const int64_t blocks = (n_vox + MATCH_THREADS - 1) / MATCH_THREADS;
+    const int64_t chunks = (n_lib + MATCH_CHUNK - 1) / MATCH_CHUNK;
+    const int64_t want = std::min<int64_t>(std::min<int64_t>(chunks, 65535), blocks > 0 ? 1216 / blocks : 1);
+    if (want > 1) {
+        p.part = (int)((chunks + want - 1) / want * MATCH_CHUNK);
+        p.parts = (n_lib + p.part - 1) / p.part;
+        p.bytes = 8 * n_vox;
+    }
+    return p;
+}
+
+template <int N, int MODE>
+static madi_status launch_fp32(const madi_match_desc* d, const MatchPlan& p, float* mu, unsigned char* scratch, cudaStream_t s) {
+    if (p.pruned) {
+        prune::Index ix;
+        prune::layout(ix, scratch, d->n_vox, d->n_lib, d->n_feat);
+        ix.mu = MODE == MADI_MATCH_FIXED_S0 ? mu : nullptr;
+        ix.free_s0 = MODE == MADI_MATCH_FREE_S0;
+        const madi_status st = prune::build(ix, d->measured, d->lib, true, s);
+        if (st != MADI_OK) return st;
+        constexpr int per = MATCH_THREADS * 2;
+        match_pruned_kernel<N, MODE><<<(unsigned)((d->n_vox + per - 1) / per), MATCH_THREADS, 0, s>>>(
+            d->measured, d->lib, ix, d->best_idx, d->best_resid, d->best_s0);
+    } else {
+        unsigned long long* keys = p.parts > 1 ? reinterpret_cast<unsigned long long*>(scratch) : nullptr;
+        if (keys) {
+            const cudaError_t e = cudaMemsetAsync(keys, 0xff, 8 * d->n_vox, s);
+            if (e != cudaSuccess) return host::cuda_fail(e, "match fp32 memset");
+        }
+        const int64_t blocks = (d->n_vox + MATCH_THREADS - 1) / MATCH_THREADS;
+        // two voxels a thread once that still fills the chip
+        if (blocks >= 2 * 1216) {
+            const dim3 grid((unsigned)((d->n_vox + 2 * MATCH_THREADS - 1) / (2 * MATCH_THREADS)), (unsigned)p.parts);
+            match_scan_kernel<N, MODE, 2><<<grid, MATCH_THREADS, 0, s>>>(d->measured, d->lib, mu, d->n_vox, d->n_lib, d->n_feat,
+                                                                        p.part, keys, d->best_idx, d->best_resid, d->best_s0);
+        } else {
+            match_scan_kernel<N, MODE, 1><<<dim3((unsigned)blocks, (unsigned)p.parts), MATCH_THREADS, 0, s>>>(
+                d->measured, d->lib, mu, d->n_vox, d->n_lib, d->n_feat, p.part, keys, d->best_idx, d->best_resid, d->best_s0);
+        }
+        if (keys)
+            match_finish_kernel<N, MODE><<<(unsigned)((d->n_vox + 255) / 256), 256, 0, s>>>(
+                d->measured, d->lib, keys, d->n_vox, d->n_feat, d->best_idx, d->best_resid, d->best_s0);
+    }
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return host::cuda_fail(e, "match fp32 launch");
     return MADI_OK;
+}
+
+template <int MODE>
+static madi_status launch_fp32_mode(const madi_match_desc* d, const MatchPlan& p, float* mu, unsigned char* scratch, cudaStream_t s) {
+    switch ((d->n_feat + 3) / 4) {
+        case 1: case 2: return launch_fp32<8, MODE>(d, p, mu, scratch, s);
+        case 3: return launch_fp32<12, MODE>(d, p, mu, scratch, s);
+        case 4: return launch_fp32<16, MODE>(d, p, mu, scratch, s);
+        case 5: return launch_fp32<20, MODE>(d, p, mu, scratch, s);
+        case 6: return launch_fp32<24, MODE>(d, p, mu, scratch, s);
+        case 7: return launch_fp32<28, MODE>(d, p, mu, scratch, s);
+        default: return launch_fp32<32, MODE>(d, p, mu, scratch, s);
+    }
 }
 
 }  // namespace madi
@@ -113,13 +434,15 @@ const int* madi_match_bf16_status_word(const madi_match_desc* d);
 int64_t madi_match_bf16_scratch(int64_t n_vox, int32_t n_lib, int32_t n_feat, int32_t topk);
 void madi_match_column_mean(const float* lib, int32_t n_lib, int32_t n_feat, float* mu, cudaStream_t s);
 
-// fp32 needs room for the column means (either mode, so one size fits both).
+// fp32 needs room for the column means (fixed S0); with the plan's scratch behind
+// them it splits or prunes the scan.
 static constexpr int64_t FP32_SCRATCH = 256;
 
 extern "C" int64_t madi_match_scratch_bytes(int64_t n_vox, int32_t n_lib, int32_t n_feat, int32_t precision,
                                             int32_t topk) {
     if (precision == MADI_MATCH_BF16) return madi_match_bf16_scratch(n_vox, n_lib, n_feat, topk);
-    return FP32_SCRATCH;
+    if (n_vox <= 0 || n_lib < 1 || n_feat < 1 || n_feat > 32) return FP32_SCRATCH;
+    return FP32_SCRATCH + match_plan(n_vox, n_lib, n_feat).bytes;
 }
 
 extern "C" madi_status madi_match(const madi_match_desc* d, void* stream) {
@@ -144,10 +467,14 @@ extern "C" madi_status madi_match(const madi_match_desc* d, void* stream) {
         mu = static_cast<float*>(d->scratch);
         madi_match_column_mean(d->lib, d->n_lib, d->n_feat, mu, s);
     }
-    if (d->n_feat <= 8) return launch_fp32<8>(d, mu, s);
-    if (d->n_feat <= 16) return launch_fp32<16>(d, mu, s);
-    if (d->n_feat <= 24) return launch_fp32<24>(d, mu, s);
-    return launch_fp32<32>(d, mu, s);
+    MatchPlan plan = match_plan(d->n_vox, d->n_lib, d->n_feat);
+    unsigned char* scratch = nullptr;
+    if (d->scratch && (reinterpret_cast<uintptr_t>(d->scratch) & 255) == 0 && d->scratch_bytes >= FP32_SCRATCH + plan.bytes)
+        scratch = static_cast<unsigned char*>(d->scratch) + FP32_SCRATCH;
+    else
+        plan = MatchPlan{false, 1, d->n_lib, 0};            // the caller's scratch holds the column means only
+    return d->mode == MADI_MATCH_FIXED_S0 ? launch_fp32_mode<MADI_MATCH_FIXED_S0>(d, plan, mu, scratch, s)
+                                          : launch_fp32_mode<MADI_MATCH_FREE_S0>(d, plan, mu, scratch, s);
 }
 
 extern "C" madi_status madi_match_wait(const madi_match_desc* d, void* stream) {
