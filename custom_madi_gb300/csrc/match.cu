@@ -170,10 +170,13 @@ __global__ void __launch_bounds__(256) match_finish_kernel(const float* __restri
 }
 
 // ---------------------------------------------------------------------------
-// Pruned search.  A warp takes 64 voxels that are neighbours in the index's
-// order (two per lane), scans the tile nearest to them, then every tile that
-// some voxel still needs: first by the box of the warp's voxels (32 tiles at a
-// time, one per lane), then voxel by voxel.
+// Pruned search.  A group of 64 voxels that are neighbours in the index's order
+// (two per lane) has the tile nearest to it scanned, then every tile that some
+// voxel still needs: first by the box of the group's voxels (32 tiles at a time,
+// one per lane), then voxel by voxel.  A tile's rows (6 KB at 20 features) come
+// to shared memory by one bulk copy while the tile before is scanned: read in
+// place, each entry waited for its 6 broadcast loads.  WARPS warps share a
+// group's tiles and merge their winners, so that small fits fill the chip.
 //
 // Why nothing is missed: with d the box distance in the embedding, every entry
 // of the tile has |m - L|^2 >= d^2 (1-Lipschitz), so its exact score is at least
@@ -220,8 +223,28 @@ MADI_DEV float box_distance2(const float4* __restrict__ b, const float (&lo)[6],
     return d2;
 }
 
+// Two fp32 fused multiply-adds in one instruction, each rounded as fmaf().
+MADI_DEV uint64_t pair2(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+MADI_DEV float2 split2(uint64_t v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+MADI_DEV uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// Scores a tile for the two voxels of every lane.  Rows come in pairs of entries,
+// feature by feature, so one packed instruction advances both entries' dot
+// products (m holds each feature twice).
 template <int N, int MODE>
-MADI_DEV void scan_tile(const float4* __restrict__ rows, const float (&ma)[N], const float (&mb)[N], PrunedVoxel& a,
+MADI_DEV void scan_tile(const ulonglong2* rows, const uint64_t (&ma)[N], const uint64_t (&mb)[N], PrunedVoxel& a,
                         PrunedVoxel& b) {
     // winners of the tile alone (its entries are in index order), then against the
     // best so far; the free score's bar starts from the best so far
@@ -229,21 +252,21 @@ MADI_DEV void scan_tile(const float4* __restrict__ rows, const float (&ma)[N], c
     float bara = MODE == MADI_MATCH_FIXED_S0 ? 0.f : free_bar(a.best), barb = MODE == MADI_MATCH_FIXED_S0 ? 0.f : free_bar(b.best);
     int ja = -1, jb = -1;
 #pragma unroll 2
-    for (int e = 0; e < prune::TILE; ++e) {
-        const float4* r = rows + e * (N / 4 + 1);
-        float da = 0.f, db = 0.f;
+    for (int e = 0; e < prune::TILE / 2; ++e) {
+        const ulonglong2* r = rows + e * (N / 2 + 2);
+        uint64_t da = 0, db = 0;
 #pragma unroll
-        for (int f = 0; f < N / 4; ++f) {
-            const float4 l = r[f];
-            da = fmaf(ma[4 * f], l.x, da); da = fmaf(ma[4 * f + 1], l.y, da);
-            da = fmaf(ma[4 * f + 2], l.z, da); da = fmaf(ma[4 * f + 3], l.w, da);
-            db = fmaf(mb[4 * f], l.x, db); db = fmaf(mb[4 * f + 1], l.y, db);
-            db = fmaf(mb[4 * f + 2], l.z, db); db = fmaf(mb[4 * f + 3], l.w, db);
+        for (int f = 0; f < N / 2; ++f) {
+            const ulonglong2 l = r[f];
+            da = fma2(ma[2 * f], l.x, da); da = fma2(ma[2 * f + 1], l.y, da);
+            db = fma2(mb[2 * f], l.x, db); db = fma2(mb[2 * f + 1], l.y, db);
         }
-        const float4 x = r[N / 4];
-        const int j = __float_as_int(x.y);
-        match_pair<MODE>(da, x.x, j, ta, ja, bara);
-        match_pair<MODE>(db, x.x, j, tb, jb, barb);
+        const ulonglong2 x = r[N / 2];
+        const float2 sn = split2(x.x), id = split2(x.y), ea = split2(da), eb = split2(db);
+        match_pair<MODE>(ea.x, sn.x, __float_as_int(id.x), ta, ja, bara);
+        match_pair<MODE>(eb.x, sn.x, __float_as_int(id.x), tb, jb, barb);
+        match_pair<MODE>(ea.y, sn.y, __float_as_int(id.y), ta, ja, bara);
+        match_pair<MODE>(eb.y, sn.y, __float_as_int(id.y), tb, jb, barb);
     }
     if (ja >= 0 && (ta < a.best || (ta == a.best && ja < a.bj))) { a.best = ta; a.bj = ja; }
     if (jb >= 0 && (tb < b.best || (tb == b.best && jb < b.bj))) { b.best = tb; b.bj = jb; }
@@ -251,96 +274,185 @@ MADI_DEV void scan_tile(const float4* __restrict__ rows, const float (&ma)[N], c
     set_limit<MODE>(b);
 }
 
-template <int N, int MODE>
-__global__ void __launch_bounds__(MATCH_THREADS, N <= 16 ? 4 : 3) match_pruned_kernel(const float* __restrict__ meas,
+// Bulk copy of one tile's rows into shared memory, completing on `bar`.
+MADI_DEV void tile_fetch(float4* dst, const float4* src, uint32_t bytes, uint64_t* bar) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst), b = (uint32_t)__cvta_generic_to_shared(bar);
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(b), "r"(bytes) : "memory");
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 :: "r"(d), "l"(src), "r"(bytes), "r"(b) : "memory");
+}
+
+// Waits for phase `parity` of a tile copy, ~1 s at most (20 us suspends); false
+// if it ran out.
+MADI_DEV bool tile_wait(uint64_t* bar, uint32_t parity) {
+    const uint32_t b = (uint32_t)__cvta_generic_to_shared(bar);
+    for (int i = 0; i < 50000; ++i) {
+        uint32_t done;
+        asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n selp.u32 %0, 1, 0, p;\n}"
+                     : "=r"(done) : "r"(b), "r"(parity), "r"(20000u) : "memory");
+        if (done) return true;
+    }
+    return false;
+}
+
+template <int N, int MODE, int WARPS>
+__global__ void __launch_bounds__(MATCH_THREADS, N <= 12 ? 4 : N <= 24 ? 3 : 2) match_pruned_kernel(const float* __restrict__ meas,
                                                                         const float* __restrict__ lib,
                                                                         const prune::Index ix, int32_t* best_idx,
                                                                         float* best_resid, float* best_s0) {
+    constexpr int NW = MATCH_THREADS / 32, GROUPS = NW / WARPS;
+    constexpr int TILE4 = prune::TILE * (N / 4 + 1);                           // float4 of a tile's rows
+    extern __shared__ __align__(128) float4 stage[];                           // [warp][2][TILE4]
     __shared__ float sv[prune::B_FLOATS], smu[N];
+    __shared__ uint64_t bars[NW][2];
+    __shared__ unsigned long long merged[WARPS > 1 ? GROUPS : 1][64];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int i = threadIdx.x; i < prune::B_FLOATS; i += MATCH_THREADS) sv[i] = ix.basis[i];
     if (threadIdx.x < N)
         smu[threadIdx.x] = (MODE == MADI_MATCH_FIXED_S0 && (int)threadIdx.x < ix.F) ? ix.mu[threadIdx.x] : 0.f;
+    if (WARPS > 1)
+        for (int i = threadIdx.x; i < GROUPS * 64; i += MATCH_THREADS) merged[i >> 6][i & 63] = ~0ull;
+    if (lane < 2) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"((uint32_t)__cvta_generic_to_shared(&bars[warp][lane])) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     __syncthreads();
-    const int lane = threadIdx.x & 31;
-    const int64_t p0 = ((int64_t)blockIdx.x * (MATCH_THREADS / 32) + (threadIdx.x >> 5)) * 64;
-    if (p0 >= ix.n_vox) return;
+    const int64_t p0 = ((int64_t)blockIdx.x * GROUPS + warp / WARPS) * 64;
+    const int part = warp % WARPS;
+    const bool live = p0 < ix.n_vox;                                           // a whole group
+    if (WARPS == 1 && !live) return;
     const float slack = (float)(ix.F + 8) * 4.76837158203125e-07f;             // (F + 8) 2^-21
     const float lmax = ix.lmax[0], inv_lmin = ix.lmax[1];
     int64_t vox[2];
-    float m[2][N], phi[2][6];
     PrunedVoxel pv[2];
+    if (live) {
+        uint64_t mm[2][N];
+        float phi[2][6];
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        vox[i] = ix.vperm[min(p0 + 32 * i + lane, ix.n_vox - 1)];
-        PrunedVoxel& v = pv[i];
-        v.m2 = 0.f;
+        for (int i = 0; i < 2; ++i) {
+            float m[N];
+            vox[i] = ix.vperm[min(p0 + 32 * i + lane, ix.n_vox - 1)];
+            PrunedVoxel& v = pv[i];
+            v.m2 = 0.f;
 #pragma unroll
-        for (int f = 0; f < N; ++f) {
-            m[i][f] = f < ix.F ? meas[vox[i] * ix.F + f] - smu[f] : 0.f;
-            v.m2 = fmaf(m[i][f], m[i][f], v.m2);
+            for (int f = 0; f < N; ++f) {
+                m[f] = f < ix.F ? meas[vox[i] * ix.F + f] - smu[f] : 0.f;
+                v.m2 = fmaf(m[f], m[f], v.m2);
+            }
+            prune::Phi e;
+            if (MODE == MADI_MATCH_FIXED_S0) {
+                e = prune::embed(m, sv);
+                v.e = slack * (v.m2 + lmax);
+                v.bounded = v.m2 + lmax < 1e36f;
+            } else {
+                float u[N];
+                const float sc = v.m2 > 0.f ? rsqrtf(v.m2) : 0.f;
+#pragma unroll
+                for (int f = 0; f < N; ++f) u[f] = f < ix.F ? fmaf(m[f], sc, -sv[prune::B_CENTRE + f]) : 0.f;
+                e = prune::embed(u, sv);
+                v.e = slack;
+                v.bounded = v.m2 < 1e36f && v.m2 * lmax < 1e36f && v.m2 > 1e-32f * inv_lmin;
+            }
+#pragma unroll
+            for (int k = 0; k < prune::KDIR; ++k) phi[i][k] = e.p[k];
+            phi[i][5] = e.q;
+#pragma unroll
+            for (int f = 0; f < N; ++f) mm[i][f] = pair2(m[f], m[f]);
+            v.best = NO_SCORE;
+            v.bj = 0;
+            set_limit<MODE>(v);
         }
-        prune::Phi e;
-        if (MODE == MADI_MATCH_FIXED_S0) {
-            e = prune::embed(m[i], sv);
-            v.e = slack * (v.m2 + lmax);
-            v.bounded = v.m2 + lmax < 1e36f;
-        } else {
-            float u[N];
-            const float sc = v.m2 > 0.f ? rsqrtf(v.m2) : 0.f;
+        const float4* boxes = reinterpret_cast<const float4*>(ix.box);
+        const float4* rows = reinterpret_cast<const float4*>(ix.rows);
+        float4* buf = stage + warp * 2 * TILE4;
+        uint32_t fetched = 0, scanned = 0;                                     // tiles so far: buffer = count & 1
+        bool stuck = false;
+        auto fetch = [&](int t) {
+            if (lane == 0) tile_fetch(buf + (fetched & 1) * TILE4, rows + (int64_t)t * TILE4, TILE4 * 16, &bars[warp][fetched & 1]);
+            ++fetched;
+        };
+        auto scan = [&]() {
+            const uint32_t i = scanned & 1;
+            if (!tile_wait(&bars[warp][i], (scanned >> 1) & 1)) stuck = true;
+            else scan_tile<N, MODE>(reinterpret_cast<const ulonglong2*>(buf + i * TILE4), mm[0], mm[1], pv[0], pv[1]);
+            ++scanned;
+            __syncwarp();                                                      // read before it is fetched over
+        };
+        // ---- the tile nearest to one of the group's voxels ----
+        float c[6], glo[6], ghi[6];
 #pragma unroll
-            for (int f = 0; f < N; ++f) u[f] = f < ix.F ? fmaf(m[i][f], sc, -sv[prune::B_CENTRE + f]) : 0.f;
-            e = prune::embed(u, sv);
-            v.e = slack;
-            v.bounded = v.m2 < 1e36f && v.m2 * lmax < 1e36f && v.m2 > 1e-32f * inv_lmin;
+        for (int k = 0; k < 6; ++k) {
+            c[k] = __shfl_sync(MADI_FULL, phi[0][k], 16);
+            glo[k] = warp_minf32(fminf(phi[0][k], phi[1][k]));
+            ghi[k] = warp_maxf32(fmaxf(phi[0][k], phi[1][k]));
         }
+        float near = NO_SCORE;
+        int t0 = 0;
+        for (int t = lane; t < ix.n_tiles; t += 32) {
+            const float d = box_distance2(boxes + 4ll * t, c, c);
+            if (d < near) { near = d; t0 = t; }
+        }
+        {
+            const float best = warp_minf32(near);
+            const unsigned who = __ballot_sync(MADI_FULL, near == best);
+            t0 = __shfl_sync(MADI_FULL, t0, who ? __ffs(who) - 1 : 0);
+        }
+        fetch(t0);
+        scan();
+        // ---- every other tile some voxel still needs (this warp's share), one
+        // in flight while the one before is scanned ----
+        unsigned share = 0xffffffffu;
+        if (WARPS > 1) share = (0x11111111u * ((1u << (4 / WARPS)) - 1u)) << (part * (4 / WARPS));
+        for (int base = 0; base < ix.n_tiles; base += 32) {
+            const float top = warp_maxf32(fmaxf(pv[0].limit, pv[1].limit));
+            const int mine = base + lane;
+            bool want = false;
+            if (mine < ix.n_tiles && mine != t0) want = !(0.998f * box_distance2(boxes + 4ll * mine, glo, ghi) > top);
+            for (unsigned mask = __ballot_sync(MADI_FULL, want) & share; mask; mask &= mask - 1) {
+                const int t = base + __ffs(mask) - 1;
+                const float4* b = boxes + 4ll * t;
+                const bool need = !(0.998f * box_distance2(b, phi[0], phi[0]) > pv[0].limit) ||
+                                  !(0.998f * box_distance2(b, phi[1], phi[1]) > pv[1].limit);
+                if (!__any_sync(MADI_FULL, need)) continue;
+                fetch(t);
+                if (fetched - scanned == 2) scan();
+            }
+        }
+        while (fetched != scanned) scan();
+        // a copy that never completed (not seen; the wait is bounded): no result
+        // is better than a wrong one
+        if (stuck) pv[0].bj = pv[1].bj = -1;
+    }
+    if (WARPS > 1) {
+        const int g = warp / WARPS;
+        if (live) {
 #pragma unroll
-        for (int k = 0; k < prune::KDIR; ++k) phi[i][k] = e.p[k];
-        phi[i][5] = e.q;
-        v.best = NO_SCORE;
-        v.bj = 0;
-        set_limit<MODE>(v);
-    }
-    const float4* boxes = reinterpret_cast<const float4*>(ix.box);
-    const float4* rows = reinterpret_cast<const float4*>(ix.rows);
-    const int tile_rows = prune::TILE * (N / 4 + 1);
-    // ---- the tile nearest to one of the warp's voxels ----
-    float c[6], glo[6], ghi[6];
+            for (int i = 0; i < 2; ++i) atomicMin(&merged[g][32 * i + lane], pv[i].bj < 0 ? 0ull : match_key(pv[i].best, pv[i].bj));
+        }
+        __syncthreads();
+        if (!live || part != 0) return;
 #pragma unroll
-    for (int k = 0; k < 6; ++k) {
-        c[k] = __shfl_sync(MADI_FULL, phi[0][k], 16);
-        glo[k] = warp_minf32(fminf(phi[0][k], phi[1][k]));
-        ghi[k] = warp_maxf32(fmaxf(phi[0][k], phi[1][k]));
-    }
-    float near = NO_SCORE;
-    int t0 = 0;
-    for (int t = lane; t < ix.n_tiles; t += 32) {
-        const float d = box_distance2(boxes + 4ll * t, c, c);
-        if (d < near) { near = d; t0 = t; }
-    }
-    {
-        const float best = warp_minf32(near);
-        const unsigned who = __ballot_sync(MADI_FULL, near == best);
-        t0 = __shfl_sync(MADI_FULL, t0, who ? __ffs(who) - 1 : 0);
-    }
-    scan_tile<N, MODE>(rows + (int64_t)t0 * tile_rows, m[0], m[1], pv[0], pv[1]);
-    // ---- every other tile some voxel still needs ----
-    for (int base = 0; base < ix.n_tiles; base += 32) {
-        const float top = warp_maxf32(fmaxf(pv[0].limit, pv[1].limit));
-        const int mine = base + lane;
-        bool want = false;
-        if (mine < ix.n_tiles && mine != t0) want = !(0.998f * box_distance2(boxes + 4ll * mine, glo, ghi) > top);
-        for (unsigned mask = __ballot_sync(MADI_FULL, want); mask; mask &= mask - 1) {
-            const int t = base + __ffs(mask) - 1;
-            const float4* b = boxes + 4ll * t;
-            const bool need = !(0.998f * box_distance2(b, phi[0], phi[0]) > pv[0].limit) ||
-                              !(0.998f * box_distance2(b, phi[1], phi[1]) > pv[1].limit);
-            if (__any_sync(MADI_FULL, need)) scan_tile<N, MODE>(rows + (int64_t)t * tile_rows, m[0], m[1], pv[0], pv[1]);
+        for (int i = 0; i < 2; ++i) {
+            const unsigned long long key = merged[g][32 * i + lane];
+            pv[i].bj = key == 0ull ? -1 : (int)(uint32_t)key;
         }
     }
 #pragma unroll
     for (int i = 0; i < 2; ++i)
-        if (p0 + 32 * i + lane < ix.n_vox)
-            match_write<N, MODE>(meas, lib, vox[i], pv[i].bj, ix.F, best_idx, best_resid, best_s0);
+        if (p0 + 32 * i + lane < ix.n_vox) {
+            if (pv[i].bj < 0) best_idx[vox[i]] = -1;
+            else match_write<N, MODE>(meas, lib, vox[i], pv[i].bj, ix.F, best_idx, best_resid, best_s0);
+        }
+}
+
+template <int N, int MODE, int WARPS>
+static cudaError_t launch_pruned(const madi_match_desc* d, const prune::Index& ix, cudaStream_t s) {
+    const auto kernel = match_pruned_kernel<N, MODE, WARPS>;
+    constexpr int smem = MATCH_THREADS / 32 * 2 * prune::TILE * (N / 4 + 1) * 16;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    constexpr int per = 64 * (MATCH_THREADS / 32) / WARPS;
+    kernel<<<(unsigned)((d->n_vox + per - 1) / per), MATCH_THREADS, smem, s>>>(d->measured, d->lib, ix, d->best_idx,
+                                                                              d->best_resid, d->best_s0);
+    return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------------------
@@ -355,7 +467,8 @@ struct MatchPlan {
 
 static MatchPlan match_plan(int64_t n_vox, int32_t n_lib, int32_t n_feat) {
     MatchPlan p{false, 1, n_lib, 0};
-    // The index costs ~0.1 ms; below ~4e9 products the scan is done by then.
+    // The index costs ~0.1 ms: 20,000 voxels x 20,000 entries x 20 take 1.73 ms
+    // scanned by one part, 0.20 ms pruned; 4,096 voxels 0.15 ms split over parts.
     if (n_vox >= 4096 && n_lib >= 1024 && (double)n_vox * n_lib * n_feat >= 4e9 && n_vox < 0x7fffffff) {
         p.pruned = true;
         prune::Index ix;
@@ -384,9 +497,15 @@ static madi_status launch_fp32(const madi_match_desc* d, const MatchPlan& p, flo
         ix.free_s0 = MODE == MADI_MATCH_FREE_S0;
         const madi_status st = prune::build(ix, d->measured, d->lib, true, s);
         if (st != MADI_OK) return st;
-        constexpr int per = MATCH_THREADS * 2;
-        match_pruned_kernel<N, MODE><<<(unsigned)((d->n_vox + per - 1) / per), MATCH_THREADS, 0, s>>>(
-            d->measured, d->lib, ix, d->best_idx, d->best_resid, d->best_s0);
+        // Warps a group: more shorten the longest group's chain of tiles while the
+        // groups alone do not fill the chip, but each repeats the group's set-up and
+        // holds a staler bound (20,000 entries, ms at 1 / 2 / 4 warps, before the
+        // packed multiply-adds: 100,000 voxels 0.83 / 0.53 / 0.47, 150,000 0.76 /
+        // 0.65 / 0.67, 300,000 1.06 / 1.07 / 1.14, 1e6 2.97 / 3.15 / 3.48).
+        const cudaError_t e = d->n_vox < 125000 ? launch_pruned<N, MODE, 4>(d, ix, s)
+                              : d->n_vox < 300000 ? launch_pruned<N, MODE, 2>(d, ix, s)
+                                                  : launch_pruned<N, MODE, 1>(d, ix, s);
+        if (e != cudaSuccess) return host::cuda_fail(e, "match fp32 pruned launch");
     } else {
         unsigned long long* keys = p.parts > 1 ? reinterpret_cast<unsigned long long*>(scratch) : nullptr;
         if (keys) {

@@ -8,6 +8,7 @@ namespace madi {
 namespace prune {
 
 constexpr int BASIS_THREADS = 1024;
+constexpr int ITERATIONS = 6;
 constexpr int SROW = FMAX + 1;                  // sample row stride in shared memory (bank spread)
 
 // Directions from a strided sample of the library: covariance, then orthogonal
@@ -62,30 +63,38 @@ __global__ void __launch_bounds__(BASIS_THREADS) basis_kernel(const float* __res
     __syncthreads();
     if (warp == 0) {
         float x[KDIR];
+#pragma unroll
         for (int k = 0; k < KDIR; ++k) x[k] = lane < F ? cosf(0.7f * (k + 1) * lane) + (lane == k ? 1.f : 0.f) : 0.f;
-        for (int it = 0; it < 17; ++it) {
+        for (int it = 0; it <= ITERATIONS; ++it) {
             if (it > 0) {
                 float y[KDIR] = {};
                 for (int b = 0; b < F; ++b) {
                     const float c = cov[lane * FMAX + b];
+#pragma unroll
                     for (int k = 0; k < KDIR; ++k) y[k] = fmaf(c, __shfl_sync(MADI_FULL, x[k], b), y[k]);
                 }
+#pragma unroll
                 for (int k = 0; k < KDIR; ++k) x[k] = y[k];
             }
-            // Gram-Schmidt, twice in the last round; a direction that vanishes becomes 0
-            for (int rep = 0; rep < (it == 16 ? 2 : 1); ++rep)
+            // Gram-Schmidt (each vector's sums together), twice in the last round; a
+            // direction that vanishes becomes 0
+            for (int rep = 0; rep < (it == ITERATIONS ? 2 : 1); ++rep) {
+#pragma unroll
                 for (int k = 0; k < KDIR; ++k) {
-                    float n0 = x[k] * x[k];
-                    for (int o = 16; o > 0; o >>= 1) n0 += __shfl_xor_sync(MADI_FULL, n0, o);
-                    for (int j = 0; j < k; ++j) {
-                        float d = x[k] * x[j];
-                        for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(MADI_FULL, d, o);
-                        x[k] = fmaf(-d, x[j], x[k]);
-                    }
+                    float d[KDIR];
+#pragma unroll
+                    for (int j = 0; j <= k; ++j) d[j] = x[k] * x[j];
+                    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                        for (int j = 0; j <= k; ++j) d[j] += __shfl_xor_sync(MADI_FULL, d[j], o);
+                    const float n0 = d[k];
+#pragma unroll
+                    for (int j = 0; j < k; ++j) x[k] = fmaf(-d[j], x[j], x[k]);
                     float n2 = x[k] * x[k];
                     for (int o = 16; o > 0; o >>= 1) n2 += __shfl_xor_sync(MADI_FULL, n2, o);
                     x[k] = (n2 > 1e-6f * n0 && n2 > 1e-30f) ? x[k] * (1.f / sqrtf(n2)) : 0.f;
                 }
+            }
         }
         for (int k = 0; k < KDIR; ++k) v[k][lane] = x[k];
     }
@@ -190,38 +199,41 @@ __global__ void __launch_bounds__(256) embed_kernel(const float* __restrict__ me
     }
 }
 
-// Exclusive scan of the bins: CTA 0 the library's, CTA 1 the voxels'.
+// Exclusive scan of the bins: CTA 0 the library's, CTA 1 the voxels'.  A warp
+// takes a contiguous 32nd, 128 bins per coalesced step.
 __global__ void __launch_bounds__(1024) scan_kernel(uint32_t* bins) {
+    static_assert(LIB_BINS % 4096 == 0 && VOX_BINS % 4096 == 0, "whole steps");
+    constexpr int MAX_STEPS = (LIB_BINS > VOX_BINS ? LIB_BINS : VOX_BINS) / 4096;
     __shared__ uint32_t part[32];
     uint32_t* b = blockIdx.x == 0 ? bins : bins + LIB_BINS;
-    const int per = (blockIdx.x == 0 ? LIB_BINS : VOX_BINS) / 1024;
+    const int steps = (blockIdx.x == 0 ? LIB_BINS : VOX_BINS) / 4096;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint4* mine = reinterpret_cast<uint4*>(b + threadIdx.x * per);
+    uint4* mine = reinterpret_cast<uint4*>(b) + warp * steps * 32 + lane;
+    uint4 x[MAX_STEPS];
     uint32_t sum = 0;
-    for (int i = 0; i < per / 4; ++i) { const uint4 x = mine[i]; sum += x.x + x.y + x.z + x.w; }
-    uint32_t inc = sum;
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t u = __shfl_up_sync(MADI_FULL, inc, o);
-        if (lane >= o) inc += u;
-    }
-    if (lane == 31) part[warp] = inc;
+#pragma unroll
+    for (int i = 0; i < MAX_STEPS; ++i)
+        if (i < steps) x[i] = mine[32 * i];
+#pragma unroll
+    for (int i = 0; i < MAX_STEPS; ++i)
+        if (i < steps) sum += x[i].x + x[i].y + x[i].z + x[i].w;
+    sum = __reduce_add_sync(MADI_FULL, sum);
+    if (lane == 0) part[warp] = sum;
     __syncthreads();
-    if (warp == 0) {
-        uint32_t p = part[lane];
+    uint32_t run = __reduce_add_sync(MADI_FULL, lane < warp ? part[lane] : 0u);
+#pragma unroll
+    for (int i = 0; i < MAX_STEPS; ++i) {
+        if (i >= steps) break;
+        const uint32_t s4 = x[i].x + x[i].y + x[i].z + x[i].w;
+        uint32_t inc = s4;
         for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t u = __shfl_up_sync(MADI_FULL, p, o);
-            if (lane >= o) p += u;
+            const uint32_t u = __shfl_up_sync(MADI_FULL, inc, o);
+            if (lane >= o) inc += u;
         }
-        part[lane] = p;
-    }
-    __syncthreads();
-    uint32_t run = inc - sum + (warp > 0 ? part[warp - 1] : 0u);
-    for (int i = 0; i < per / 4; ++i) {
-        const uint4 x = mine[i];
         uint4 y;
-        y.x = run; y.y = y.x + x.x; y.z = y.y + x.y; y.w = y.z + x.z;
-        run = y.w + x.w;
-        mine[i] = y;
+        y.x = run + inc - s4; y.y = y.x + x[i].x; y.z = y.y + x[i].y; y.w = y.z + x[i].z;
+        mine[32 * i] = y;
+        run += __shfl_sync(MADI_FULL, inc, 31);
     }
 }
 
@@ -240,7 +252,7 @@ __global__ void __launch_bounds__(256) scatter_kernel(const Index ix, int lib_bl
 // |row|^2 as the exhaustive scan computes it, and the box of their Phi.
 __global__ void __launch_bounds__(TILE) tile_kernel(const float* __restrict__ lib, const Index ix) {
     __shared__ int idx[TILE], sorted[TILE];
-    __shared__ float red[2][6][2];
+    __shared__ float red[2][6][TILE / 32];
     const int t = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int e = ix.lperm[t * TILE + tid];
     const int key = e < 0 ? 0x7fffffff : e;
@@ -252,18 +264,20 @@ __global__ void __launch_bounds__(TILE) tile_kernel(const float* __restrict__ li
     __syncthreads();
     const int j = sorted[tid];
     ix.lperm[t * TILE + tid] = j;
-    float* out = ix.rows + (int64_t)(t * TILE + tid) * ix.stride;
-    const int w = ix.stride - 4;
+    // pairs of entries, feature by feature: (x_0[f], x_1[f]), then (|x_0|^2, |x_1|^2,
+    // index, index)
+    const int w = ix.stride - 4, half = tid & 1;
+    float* out = ix.rows + (int64_t)(t * (TILE / 2) + (tid >> 1)) * (2 * ix.stride);
     float s = 0.f;
     for (int f = 0; f < w; ++f) {
         const float x = (j >= 0 && f < ix.F) ? lib[(int64_t)j * ix.F + f] - (ix.mu ? ix.mu[f] : 0.f) : 0.f;
         s = fmaf(x, x, s);
-        out[f] = x;
+        out[2 * f + half] = x;
     }
-    // padding entries score 3e38 / NaN and never win
-    out[w] = j >= 0 ? (ix.free_s0 ? fmaxf(s, 1e-30f) : s) : __int_as_float(0x7fc00000);
-    out[w + 1] = __int_as_float(j);
-    out[w + 2] = out[w + 3] = 0.f;
+    // padding entries score NaN (free S0: no positive dot product) and never win
+    out[2 * w + half] = j >= 0 ? (ix.free_s0 ? fmaxf(s, 1e-30f) : s) : __int_as_float(0x7fc00000);
+    out[2 * w + 2 + half] = __int_as_float(j);
+    out[2 * w + 4 + half] = out[2 * w + 6 + half] = 0.f;
     for (int k = 0; k < 6; ++k) {
         float lo = j >= 0 ? ix.phi[8ll * j + k] : 3.0e38f, hi = j >= 0 ? lo : -3.0e38f;
         for (int o = 16; o > 0; o >>= 1) {
@@ -274,8 +288,10 @@ __global__ void __launch_bounds__(TILE) tile_kernel(const float* __restrict__ li
     }
     __syncthreads();
     if (tid < 6) {
-        ix.box[16ll * t + tid] = fminf(red[0][tid][0], red[0][tid][1]);
-        ix.box[16ll * t + 8 + tid] = fmaxf(red[1][tid][0], red[1][tid][1]);
+        float lo = red[0][tid][0], hi = red[1][tid][0];
+        for (int w = 1; w < TILE / 32; ++w) { lo = fminf(lo, red[0][tid][w]); hi = fmaxf(hi, red[1][tid][w]); }
+        ix.box[16ll * t + tid] = lo;
+        ix.box[16ll * t + 8 + tid] = hi;
     }
 }
 

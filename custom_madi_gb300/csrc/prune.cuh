@@ -20,11 +20,11 @@
 namespace madi {
 namespace prune {
 
-constexpr int TILE = 64;                        // library entries per tile
+constexpr int TILE = 32;                        // library entries per tile
 constexpr int KDIR = 5;                         // directions of the embedding
 constexpr int FMAX = 32;
-constexpr int SAMPLE = 1024;                    // rows sampled for the directions and ranges
-constexpr int LIB_FINE = 1024;                  // v_2 buckets of a slab
+constexpr int SAMPLE = 512;                     // rows sampled for the directions and ranges
+constexpr int LIB_FINE = 512;                   // v_2 buckets of a slab
 constexpr int MAX_SLABS = 64;
 constexpr int LIB_BINS = MAX_SLABS * LIB_FINE;
 constexpr int VOX_BINS = 64 * 32 * 16;          // (v_1, v_2, v_3) buckets

@@ -66,7 +66,7 @@ KINDS = ("decays", "random", "ties", "constant", "masked", "scales", "nonfinite"
 @pytest.mark.parametrize("free", (False, True))
 @pytest.mark.parametrize("kind", KINDS)
 def test_pruned_search_equals_scan(kind, free):
-    for n_vox, n_lib, F in ((50_001, 4_099, 20), (130_000, 1_025, 31)):
+    for n_vox, n_lib, F in ((50_001, 4_099, 20), (130_000, 1_025, 31), (300_001, 1_025, 14)):   # 4, 2, 1 warps a group
         vox, lib = _data(kind, n_vox, n_lib, F, np.random.default_rng(n_lib + F))
         need, a = _match(vox, lib, free)
         assert need > 256 + 8 * n_vox           # the index: this size is pruned
