@@ -46,7 +46,7 @@ MADI_CNT_N = len(CNT_NAMES)
 EXPORTED = (
     "madi_abi_version", "madi_last_error_string", "madi_classify", "madi_walk",
     "madi_walk_smem_bytes", "madi_reduce_Y", "madi_reduce_Y_scratch_bytes", "madi_match", "madi_match_wait", "madi_match_scratch_bytes",
-    "madi_bayes", "madi_bayes_scratch_bytes",
+    "madi_bayes", "madi_bayes_scratch_bytes", "madi_bayes_work_bytes",
     "madi_kdtree_build", "madi_grid_build", "madi_facets_build", "madi_walk_blocks_per_sm", "madi_walk_noalloc",
     "madi_walk_batched", "madi_autotune_load", "madi_autotune_store",
     "madi_serve_arena_bytes", "madi_serve_create", "madi_serve_submit", "madi_serve_poll",
@@ -184,6 +184,8 @@ def _declare(lib):
     lib.madi_bayes.argtypes = [C.POINTER(MadiBayesDesc), P]
     lib.madi_bayes_scratch_bytes.argtypes = [C.c_int32, C.c_int32]
     lib.madi_bayes_scratch_bytes.restype = C.c_int64
+    lib.madi_bayes_work_bytes.argtypes = [C.c_int64, C.c_int32, C.c_int32]
+    lib.madi_bayes_work_bytes.restype = C.c_int64
     lib.madi_match_scratch_bytes.argtypes = [C.c_int64, C.c_int32, C.c_int32, C.c_int32, C.c_int32]
     lib.madi_match_scratch_bytes.restype = C.c_int64
     lib.madi_kdtree_build.argtypes = [P, C.c_int32, P, P, P, P, P]

@@ -9,8 +9,8 @@
 // deviations of (kio, rho, V), the weighted residual, n_eff = W^2 / sum w^2 and
 // (free S0) the weighted S0.
 //
-// One voxel per thread, the library streamed through shared memory twice:
-//   pass 1: the fp32 scores of every entry (the match kernel's centred fixed-S0
+// One voxel per lane, the library in index order, twice:
+//   pass 1: the fp32 scores of the entries (the match kernel's centred fixed-S0
 //           score, or the free-S0 projection), argmax of e_j -> j*; e_j* is then
 //           recomputed from the direct difference and is the shift S (the
 //           reference shifts by the minimum residual or the maximum log-weight;
@@ -22,15 +22,26 @@
 //           (d = parameter minus that of j*, so narrow posteriors keep their
 //           variance), w r, w^2 and w s0.  Entries below the cut weigh less
 //           than e^-CUT of entry j*.
+//
+// Most of the time went into fp64: d took three fp64 subtractions and conversions
+// per (warp, entry) that passed, at two fp64 lanes per SM and cycle, and with
+// voxels in file order nearly every entry passed for some lane.  Here
+//   - voxels are taken in the order of the search index (prune.cuh), so that the
+//     32 voxels of a warp need the same entries;
+//   - a warp tests 32 entries at a time, one per lane, against the box of its
+//     voxels in the index's embedding and only visits those that can matter;
+//   - d is formed in pairs of floats (48 bits), then rounded to fp32 as before.
+// The entries a voxel sums, and their order, are unchanged.  100,000 voxels x
+// 20,000 entries x 20 features, sigma_m 0.02: 33.2 ms before, @@BAYES@@.
 #include <cstdint>
 #include "madi_device.cuh"
 #include "madi_host.h"
+#include "prune.cuh"
 
 namespace madi {
 namespace bayes {
 
-constexpr int THREADS = 256;
-constexpr int CHUNK = 128;
+constexpr int CHUNK = 128;           // entries staged at a time
 constexpr float CUT = 60.f;          // exp(-60) ~ 9e-27 of the shift entry's weight
 
 struct Kahan {
@@ -57,10 +68,34 @@ struct Plan {
     int n_lib, F;
     float inv2s2;
     double* out;
+    prune::Index ix;                 // indexed plans only
+    float* blocks;                   // [n_lib][Entry floats], indexed plans only
 };
 
+// One entry in shared memory: centred (fixed S0) or raw (free S0) row, raw row,
+// then |row|^2, log q, and kio, rho, V as pairs of floats.
+template <int N>
+struct Entry {
+    static constexpr int RAW = N, AUX = 2 * N, FLOATS = 2 * N + 8;
+};
+
+// x as hi + lo (48 bits).
+MADI_DEV float2 pair_of(double x) {
+    const float h = (float)x;
+    return make_float2(h, isfinite(h) ? (float)(x - (double)h) : 0.f);
+}
+
+// a - b of two pairs, rounded to fp32.
+MADI_DEV float pair_diff(float ah, float al, float2 b) {
+    const float s = ah - b.x;
+    const float t = s - ah;
+    const float e = (ah - (s - t)) - (b.x + t);              // exact error of s
+    return s + (e + (al - b.y));
+}
+
 // Screened log-weight of one entry from the fp32 score, and its error bound.
-template <int FMAX, bool FREE>
+// The error bound counts FERR features (the row rounded up to a multiple of 8).
+template <int FMAX, int FERR, bool FREE>
 MADI_DEV void screen(const float* m, const float* l, float sn, float lq, float m2, float inv2s2, float& e,
                      float& err) {
     float dot = 0.f;
@@ -70,14 +105,14 @@ MADI_DEV void screen(const float* m, const float* l, float sn, float lq, float m
         // centred: r = |m~|^2 + |L~|^2 - 2 m~.L~ ; fp32 error <= (F + 4) 2^-23 (|m~|^2 + |L~|^2)
         const float r = fmaxf(fmaf(-2.f, dot, sn) + m2, 0.f);
         e = lq - r * inv2s2;
-        err = ((float)(FMAX + 4) * 1.2e-7f * (m2 + sn)) * inv2s2 + 1e-3f;
+        err = ((float)(FERR + 4) * 1.2e-7f * (m2 + sn)) * inv2s2 + 1e-3f;
     } else {
         // rw = |L|^2 (|m|^2 |L|^2 / (m.L)^2 - 1) when m.L > 0
         if (!(dot > 0.f)) { e = -3.0e38f; err = 0.f; return; }
         const float ratio = m2 * sn / (dot * dot);
         const float rw = fmaxf(sn * (ratio - 1.f), 0.f);
         e = lq - rw * inv2s2;
-        err = (sn * ratio * (float)(FMAX + 8) * 2.4e-7f) * inv2s2 + 1e-3f;
+        err = (sn * ratio * (float)(FERR + 8) * 2.4e-7f) * inv2s2 + 1e-3f;
     }
 }
 
@@ -108,118 +143,238 @@ MADI_DEV bool exact(const float* mr, const float* L, int F, float& resid, float&
     return true;
 }
 
-template <int FMAX, bool FREE>
-__global__ void __launch_bounds__(THREADS) bayes_kernel(const Plan P) {
-    __shared__ float sl[CHUNK][FMAX];        // centred (fixed) or raw (free) library rows
-    __shared__ float sraw[CHUNK][FMAX];      // raw rows for the exact residual
-    __shared__ float sn[CHUNK];              // |L~|^2
-    __shared__ float slq[CHUNK];
-    __shared__ double spar[3][CHUNK];
-    __shared__ float smu[FMAX];
-    const int F = P.F;
-    const int64_t v = (int64_t)blockIdx.x * THREADS + threadIdx.x;
-    const bool live = v < P.n_vox;
-    if (threadIdx.x < FMAX) smu[threadIdx.x] = (!FREE && (int)threadIdx.x < F) ? P.mu[threadIdx.x] : 0.f;
+// Entry e of the library in the staged form.
+template <int N, bool FREE>
+MADI_DEV void make_entry(const Plan& P, int64_t e, const float* smu, float* o) {
+    float sn = 0.f;
+    for (int f = 0; f < N; ++f) {
+        const float x = f < P.F ? P.lib[e * P.F + f] : 0.f;
+        const float c = f < P.F ? x - smu[f] : 0.f;
+        o[f] = c;
+        o[Entry<N>::RAW + f] = x;
+        sn = fmaf(c, c, sn);
+    }
+    float* a = o + Entry<N>::AUX;
+    a[0] = FREE ? fmaxf(sn, 1e-30f) : sn;
+    a[1] = (float)P.logq[e];
+    const float2 k = pair_of(P.kio[e]), r = pair_of(P.rho[e]), v = pair_of(P.V[e]);
+    a[2] = k.x; a[3] = k.y; a[4] = r.x; a[5] = r.y; a[6] = v.x; a[7] = v.y;
+}
+
+// The library in the staged form, and (|row|^2, log q) beside its embedding.
+template <int N, bool FREE>
+__global__ void __launch_bounds__(128) bayes_prep_kernel(const Plan P) {
+    __shared__ float smu[N];
+    if (threadIdx.x < N) smu[threadIdx.x] = (!FREE && (int)threadIdx.x < P.F) ? P.mu[threadIdx.x] : 0.f;
     __syncthreads();
-    float m[FMAX], mr[FMAX];
+    const int64_t e = (int64_t)blockIdx.x * 128 + threadIdx.x;
+    if (e >= P.n_lib) return;
+    float* o = P.blocks + e * Entry<N>::FLOATS;
+    make_entry<N, FREE>(P, e, smu, o);
+    P.ix.phi[8 * e + 6] = o[Entry<N>::AUX];
+    P.ix.phi[8 * e + 7] = o[Entry<N>::AUX + 1];
+}
+
+// Largest of a warp's values (no NaN).
+MADI_DEV float warp_maxf_bits(float v) { return o2f(__reduce_max_sync(MADI_FULL, f2o(v))); }
+
+// Least residual rw an entry with embedding distance^2 d2 and |row|^2 sn can
+// have, and more than the screen and its error bound are off, in rw units.
+// Fixed S0: d2 >= |m - L|^2 bounds from below, fp32 scores are off by at most e
+// (see match_pruned_kernel).  Free S0: cos <= 1 - d2 / 2 and rw = sn (1 / cos^2 - 1).
+template <bool FREE>
+MADI_DEV float least_rw(float d2, float sn, float e) {
+    if (!FREE) return 0.998f * d2 - e;
+    const float c = fmaxf(1.f - 0.499f * d2, 0.05f);
+    return sn * ((1.f / (c * c) - 1.f) * 0.998f - 1e-4f);
+}
+
+template <int N, bool FREE, int THREADS, bool INDEXED>
+__global__ void __launch_bounds__(THREADS) bayes_kernel(const __grid_constant__ Plan P) {
+    constexpr int FERR = (N + 7) / 8 * 8, EF = Entry<N>::FLOATS;
+    extern __shared__ __align__(16) float sent[];            // [CHUNK][EF]
+    __shared__ float smu[N], sv[INDEXED ? prune::B_FLOATS : 1];
+    const int F = P.F, lane = threadIdx.x & 31;
+    const int64_t slot = (int64_t)blockIdx.x * THREADS + threadIdx.x;
+    const bool live = slot < P.n_vox;
+    const int64_t v = INDEXED ? (int64_t)P.ix.vperm[min(slot, P.n_vox - 1)] : min(slot, P.n_vox - 1);
+    if (threadIdx.x < N) smu[threadIdx.x] = (!FREE && (int)threadIdx.x < F) ? P.mu[threadIdx.x] : 0.f;
+    if (INDEXED)
+        for (int i = threadIdx.x; i < prune::B_FLOATS; i += THREADS) sv[i] = P.ix.basis[i];
+    __syncthreads();
+    float m[N], mr[N];
     float m2 = 0.f;
 #pragma unroll
-    for (int f = 0; f < FMAX; ++f) {
-        mr[f] = (live && f < F) ? P.meas[v * F + f] : 0.f;
+    for (int f = 0; f < N; ++f) {
+        mr[f] = f < F ? P.meas[v * F + f] : 0.f;
         m[f] = f < F ? mr[f] - smu[f] : 0.f;
         m2 = fmaf(m[f], m[f], m2);
     }
-    auto stage = [&](int base, int cnt) {
-        __syncthreads();
-        for (int t = threadIdx.x; t < CHUNK * FMAX; t += THREADS) {
-            const int e = t / FMAX, f = t - e * FMAX;
-            const float x = (e < cnt && f < F) ? P.lib[(int64_t)(base + e) * F + f] : 0.f;
-            sraw[e][f] = x;
-            sl[e][f] = f < F ? x - smu[f] : 0.f;
-        }
-        for (int e = threadIdx.x; e < CHUNK; e += THREADS) {
-            const bool ok = e < cnt;
-            slq[e] = ok ? (float)P.logq[base + e] : -3.0e38f;
-            spar[0][e] = ok ? P.kio[base + e] : 0.0;
-            spar[1][e] = ok ? P.rho[base + e] : 0.0;
-            spar[2][e] = ok ? P.V[base + e] : 0.0;
-        }
-        __syncthreads();
-        if (threadIdx.x < CHUNK) {
-            float s = 0.f;
+    // box of the warp's voxels in the embedding; e: margin on a residual (fixed S0)
+    float glo[6], ghi[6], e_max = 0.f;
+    bool bounded = false;
+    if (INDEXED) {
+        prune::Phi ph;
+        if (!FREE) {
+            ph = prune::embed(m, sv);
+        } else {
+            float u[N];
+            const float sc = m2 > 0.f ? rsqrtf(m2) : 0.f;
 #pragma unroll
-            for (int f = 0; f < FMAX; ++f) s = fmaf(sl[threadIdx.x][f], sl[threadIdx.x][f], s);
-            sn[threadIdx.x] = FREE ? fmaxf(s, 1e-30f) : s;
+            for (int f = 0; f < N; ++f) u[f] = f < F ? fmaf(m[f], sc, -sv[prune::B_CENTRE + f]) : 0.f;
+            ph = prune::embed(u, sv);
         }
-        __syncthreads();
+        const float lmax = P.ix.lmax[0];
+        const bool ok = FREE ? m2 < 1e30f && m2 * lmax < 1e30f && m2 > 1e-25f * P.ix.lmax[1] && P.ix.lmax[1] < 1e20f
+                             : m2 + lmax < 1e30f;
+        bounded = __all_sync(MADI_FULL, ok);
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+            const float x = k < 5 ? ph.p[k] : ph.q;
+            glo[k] = o2f(__reduce_min_sync(MADI_FULL, f2o(x)));
+            ghi[k] = o2f(__reduce_max_sync(MADI_FULL, f2o(x)));
+        }
+        // screen error (F + 8) 2^-21 (|m|^2 + |L|^2) twice, and the bound added to it
+        e_max = warp_maxf_bits((float)(FERR + 8) * 2e-6f * (m2 + lmax));
+    }
+    // Visits, in index order, the entries that may reach `floor` (a log-weight) for
+    // some voxel of the warp; visit(e, entry) runs warp-wide.
+    auto sweep = [&](auto floor, auto visit) {
+        for (int base = 0; base < P.n_lib; base += CHUNK) {
+            const int cnt = min(CHUNK, P.n_lib - base);
+            unsigned mask[CHUNK / 32];
+            unsigned any = 0;
+            const float lim = floor();
+#pragma unroll
+            for (int i = 0; i < CHUNK / 32; ++i) {
+                const int k = 32 * i + lane;
+                bool want = k < cnt;
+                if (INDEXED && bounded && want) {
+                    const float4* q = reinterpret_cast<const float4*>(P.ix.phi + 8 * (int64_t)(base + k));
+                    const float4 a = q[0], b = q[1];
+                    const float x[6] = {a.x, a.y, a.z, a.w, b.x, b.y};
+                    float d2 = 0.f;
+#pragma unroll
+                    for (int j = 0; j < 6; ++j) {
+                        const float d = fmaxf(fmaxf(x[j] - ghi[j], glo[j] - x[j]), 0.f);
+                        d2 = fmaf(d, d, d2);
+                    }
+                    want = !(b.w - least_rw<FREE>(d2, b.z, e_max) * P.inv2s2 + 3e-3f < lim);
+                }
+                mask[i] = __ballot_sync(MADI_FULL, want);
+                any |= mask[i];
+            }
+            if (THREADS > 32 ? !__syncthreads_or(any != 0u) : any == 0u) continue;
+            if (THREADS == 32) __syncwarp();
+            if (INDEXED) {
+                const float4* src = reinterpret_cast<const float4*>(P.blocks + (int64_t)base * EF);
+                float4* dst = reinterpret_cast<float4*>(sent);
+                for (int t = threadIdx.x; t < cnt * (EF / 4); t += THREADS) dst[t] = src[t];
+            } else {
+                for (int t = threadIdx.x; t < cnt; t += THREADS) make_entry<N, FREE>(P, base + t, smu, sent + t * EF);
+            }
+            if (THREADS > 32) __syncthreads(); else __syncwarp();
+#pragma unroll
+            for (int i = 0; i < CHUNK / 32; ++i)
+                for (unsigned w = mask[i]; w; w &= w - 1) {
+                    const int k = 32 * i + __ffs(w) - 1;
+                    visit(base + k, sent + k * EF);
+                }
+            if (THREADS > 32) __syncthreads(); else __syncwarp();
+        }
     };
     // ---- pass 1: argmax of the screened log-weight ----
     float best = -3.0e38f;
     int bj = -1;
-    for (int base = 0; base < P.n_lib; base += CHUNK) {
-        const int cnt = min(CHUNK, P.n_lib - base);
-        stage(base, cnt);
-        for (int e = 0; e < cnt; ++e) {
-            float ee, err;
-            screen<FMAX, FREE>(m, sl[e], sn[e], slq[e], m2, P.inv2s2, ee, err);
-            if (ee > best) { best = ee; bj = base + e; }
+    float known = -3.0e38f;                                  // a log-weight every voxel of the warp reaches
+    if (INDEXED && bounded) {
+        // the screened weight of the entry that looks best for one of the voxels
+        float c[6], top = -3.0e38f;
+#pragma unroll
+        for (int k = 0; k < 6; ++k) c[k] = 0.5f * (glo[k] + ghi[k]);
+        int tj = 0;
+        for (int e = lane; e < P.n_lib; e += 32) {
+            const float4* q = reinterpret_cast<const float4*>(P.ix.phi + 8 * (int64_t)e);
+            const float4 a = q[0], b = q[1];
+            const float x[6] = {a.x, a.y, a.z, a.w, b.x, b.y};
+            float d2 = 0.f;
+#pragma unroll
+            for (int j = 0; j < 6; ++j) d2 = fmaf(x[j] - c[j], x[j] - c[j], d2);
+            const float u = b.w - least_rw<FREE>(d2, b.z, 0.f) * P.inv2s2;
+            if (u > top) { top = u; tj = e; }
         }
+        const float w = warp_maxf_bits(top);
+        const unsigned who = __ballot_sync(MADI_FULL, top == w);
+        tj = __shfl_sync(MADI_FULL, tj, who ? __ffs(who) - 1 : 0);
+        const float* o = P.blocks + (int64_t)tj * EF;
+        float err;
+        screen<N, FERR, FREE>(m, o, o[Entry<N>::AUX], o[Entry<N>::AUX + 1], m2, P.inv2s2, known, err);
     }
+    sweep([&]() { return warp_minf(fmaxf(best, known)); },
+          [&](int e, const float* o) {
+              float ee, err;
+              screen<N, FERR, FREE>(m, o, o[Entry<N>::AUX], o[Entry<N>::AUX + 1], m2, P.inv2s2, ee, err);
+              if (ee > best) { best = ee; bj = e; }
+          });
     // shift and centre from the exact residual of j*
     float S = 0.f;
     double x0[3] = {0.0, 0.0, 0.0};
+    float2 xp[3] = {};
     bool any = bj >= 0;
     if (any) {
-        float Lj[FMAX];
+        float Lj[N];
 #pragma unroll
-        for (int f = 0; f < FMAX; ++f) Lj[f] = f < F ? P.lib[(int64_t)bj * F + f] : 0.f;
+        for (int f = 0; f < N; ++f) Lj[f] = f < F ? P.lib[(int64_t)bj * F + f] : 0.f;
         float resid, rw, s0;
-        any = exact<FMAX, FREE>(mr, Lj, F, resid, rw, s0);
+        any = exact<N, FREE>(mr, Lj, F, resid, rw, s0);
         S = (float)P.logq[bj] - rw * P.inv2s2;
         x0[0] = P.kio[bj];
         x0[1] = P.rho[bj];
         x0[2] = P.V[bj];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) xp[k] = pair_of(x0[k]);
     }
     // ---- pass 2: exp-weighted sums over the entries above the cut ----
     Kahan W, W2, R, S0, d1[3], d2[3];
-    for (int base = 0; base < P.n_lib; base += CHUNK) {
-        const int cnt = min(CHUNK, P.n_lib - base);
-        stage(base, cnt);
-        if (!any) continue;
-        for (int e = 0; e < cnt; ++e) {
-            float ee, err;
-            screen<FMAX, FREE>(m, sl[e], sn[e], slq[e], m2, P.inv2s2, ee, err);
-            if (!(ee + err - S > -CUT)) continue;
-            float resid, rw, s0;
-            if (!exact<FMAX, FREE>(mr, sraw[e], F, resid, rw, s0)) continue;
-            float x = slq[e] - rw * P.inv2s2 - S;
-            if (!(x > -CUT)) continue;
-            if (x > 0.f) {
-                // an entry above the screened maximum (within the screen's error):
-                // move the shift to it so that every weight stays <= 1
-                const float f = expf(-x);
-                W.scale(f);
-                W2.scale(f * f);
-                R.scale(f);
-                S0.scale(f);
+    sweep([&]() {
+              // entries below S - CUT of every voxel; a voxel without any entry sums none
+              const float s = warp_minf(any ? S : 3.0e38f);
+              return s - CUT - 1e-5f * fabsf(s);
+          },
+          [&](int, const float* o) {
+              const float* a = o + Entry<N>::AUX;
+              float ee, err;
+              screen<N, FERR, FREE>(m, o, a[0], a[1], m2, P.inv2s2, ee, err);
+              if (!any || !(ee + err - S > -CUT)) return;
+              float resid, rw, s0;
+              if (!exact<N, FREE>(mr, o + Entry<N>::RAW, F, resid, rw, s0)) return;
+              float x = a[1] - rw * P.inv2s2 - S;
+              if (!(x > -CUT)) return;
+              if (x > 0.f) {
+                  // an entry above the screened maximum (within the screen's error):
+                  // move the shift to it so that every weight stays <= 1
+                  const float f = expf(-x);
+                  W.scale(f);
+                  W2.scale(f * f);
+                  R.scale(f);
+                  S0.scale(f);
 #pragma unroll
-                for (int k = 0; k < 3; ++k) { d1[k].scale(f); d2[k].scale(f); }
-                S += x;
-                x = 0.f;
-            }
-            const float w = expf(x);
-            W.add(w);
-            W2.add(w * w);
-            R.add(w * resid);
-            if (FREE) S0.add(w * s0);
+                  for (int k = 0; k < 3; ++k) { d1[k].scale(f); d2[k].scale(f); }
+                  S += x;
+                  x = 0.f;
+              }
+              const float w = expf(x);
+              W.add(w);
+              W2.add(w * w);
+              R.add(w * resid);
+              if (FREE) S0.add(w * s0);
 #pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                const float d = (float)(spar[k][e] - x0[k]);
-                d1[k].add(w * d);
-                d2[k].add(w * d * d);
-            }
-        }
-    }
+              for (int k = 0; k < 3; ++k) {
+                  const float d = pair_diff(a[2 + 2 * k], a[3 + 2 * k], xp[k]);
+                  d1[k].add(w * d);
+                  d2[k].add(w * d * d);
+              }
+          });
     if (!live) return;
     const int64_t n = P.n_vox;
     double* o = P.out;
@@ -236,15 +391,40 @@ __global__ void __launch_bounds__(THREADS) bayes_kernel(const Plan P) {
     o[8 * n + v] = (FREE && Wv > 0.0) ? S0.value() / Wd : 0.0;
 }
 
-template <int FMAX>
-static madi_status launch(const madi_bayes_desc* d, const Plan& P, cudaStream_t s) {
-    const unsigned blocks = (unsigned)((d->n_vox + THREADS - 1) / THREADS);
-    if (d->mode == MADI_MATCH_FREE_S0) bayes_kernel<FMAX, true><<<blocks, THREADS, 0, s>>>(P);
-    else bayes_kernel<FMAX, false><<<blocks, THREADS, 0, s>>>(P);
-    const cudaError_t e = cudaGetLastError();
+template <int N, bool FREE, int THREADS, bool INDEXED>
+static madi_status launch_kernel(const Plan& P, cudaStream_t s) {
+    const auto kernel = bayes_kernel<N, FREE, THREADS, INDEXED>;
+    constexpr int smem = CHUNK * Entry<N>::FLOATS * 4;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return host::cuda_fail(e, "bayes attribute");
+    kernel<<<(unsigned)((P.n_vox + THREADS - 1) / THREADS), THREADS, smem, s>>>(P);
+    e = cudaGetLastError();
     if (e != cudaSuccess) return host::cuda_fail(e, "bayes launch");
     return MADI_OK;
 }
+
+template <int N, bool FREE>
+static madi_status launch(const madi_bayes_desc* d, const Plan& P, bool indexed, cudaStream_t s) {
+    if (!indexed) return launch_kernel<N, FREE, 128, false>(P, s);
+    const madi_status st = prune::build(P.ix, d->measured, d->lib, false, s);
+    if (st != MADI_OK) return st;
+    bayes_prep_kernel<N, FREE><<<(unsigned)((P.n_lib + 127) / 128), 128, 0, s>>>(P);
+    // one warp a CTA until 128-thread CTAs give every SM four warps
+    return P.n_vox < 152 * 128 ? launch_kernel<N, FREE, 32, true>(P, s) : launch_kernel<N, FREE, 128, true>(P, s);
+}
+
+template <bool FREE>
+static madi_status launch_mode(const madi_bayes_desc* d, const Plan& P, bool indexed, cudaStream_t s) {
+    switch ((d->n_feat + 3) / 4) {
+        case 1: case 2: return launch<8, FREE>(d, P, indexed, s);
+        case 3: case 4: return launch<16, FREE>(d, P, indexed, s);
+        case 5: return launch<20, FREE>(d, P, indexed, s);
+        case 6: return launch<24, FREE>(d, P, indexed, s);
+        default: return launch<32, FREE>(d, P, indexed, s);
+    }
+}
+
+static int entry_floats(int F) { return 2 * (F <= 8 ? 8 : F <= 16 ? 16 : F <= 20 ? 20 : F <= 24 ? 24 : 32) + 8; }
 
 }  // namespace bayes
 }  // namespace madi
@@ -252,6 +432,15 @@ static madi_status launch(const madi_bayes_desc* d, const Plan& P, cudaStream_t 
 using namespace madi;
 
 void madi_match_column_mean(const float* lib, int32_t n_lib, int32_t n_feat, float* mu, cudaStream_t s);
+
+// The index pays for its ~0.1 ms from about here on.
+static bool bayes_indexed(int64_t n_vox, int32_t n_lib) { return n_vox >= 64 && n_lib >= 256 && n_vox < 0x7fffffff; }
+
+extern "C" int64_t madi_bayes_work_bytes(int64_t n_vox, int32_t n_lib, int32_t n_feat) {
+    if (n_vox <= 0 || n_lib < 1 || n_feat < 1 || n_feat > 32 || !bayes_indexed(n_vox, n_lib)) return 256;
+    prune::Index ix;
+    return 256 + prune::layout(ix, nullptr, n_vox, n_lib, n_feat) + 4ll * n_lib * bayes::entry_floats(n_feat);
+}
 
 extern "C" int64_t madi_bayes_scratch_bytes(int32_t n_lib, int32_t n_feat) {
     (void)n_lib;
@@ -295,8 +484,15 @@ extern "C" madi_status madi_bayes(const madi_bayes_desc* d, void* stream) {
     P.F = d->n_feat;
     P.inv2s2 = (float)inv;
     P.out = d->out;
-    if (d->n_feat <= 8) return bayes::launch<8>(d, P, s);
-    if (d->n_feat <= 16) return bayes::launch<16>(d, P, s);
-    if (d->n_feat <= 24) return bayes::launch<24>(d, P, s);
-    return bayes::launch<32>(d, P, s);
+    const bool indexed = bayes_indexed(d->n_vox, d->n_lib) &&
+                         d->scratch_bytes >= madi_bayes_work_bytes(d->n_vox, d->n_lib, d->n_feat);
+    if (indexed) {
+        unsigned char* base = static_cast<unsigned char*>(d->scratch) + 256;
+        const int64_t at = prune::layout(P.ix, base, d->n_vox, d->n_lib, d->n_feat);
+        P.blocks = reinterpret_cast<float*>(base + at);
+        P.ix.free_s0 = d->mode == MADI_MATCH_FREE_S0;
+        P.ix.mu = P.ix.free_s0 ? nullptr : mu;
+    }
+    return d->mode == MADI_MATCH_FREE_S0 ? bayes::launch_mode<true>(d, P, indexed, s)
+                                         : bayes::launch_mode<false>(d, P, indexed, s);
 }

@@ -300,22 +300,23 @@ static void launch_embed(const Index& ix, const float* meas, const float* lib, i
     embed_kernel<N><<<lib_blocks + vox_blocks, 256, 0, s>>>(meas, lib, ix, lib_blocks);
 }
 
-madi_status build(const Index& ix, const float* meas, const float* lib, bool with_library, cudaStream_t s) {
+madi_status build(const Index& ix, const float* meas, const float* lib, bool tiles, cudaStream_t s) {
     cudaError_t e = cudaMemsetAsync(ix.bins, 0, (LIB_BINS + VOX_BINS) * 4 + 256, s);
     if (e != cudaSuccess) return host::cuda_fail(e, "search index memset");
     constexpr int smem = (SAMPLE * SROW + FMAX * FMAX) * 4;
     e = cudaFuncSetAttribute(basis_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return host::cuda_fail(e, "search index attribute");
     basis_kernel<<<1, BASIS_THREADS, smem, s>>>(meas, lib, ix);
-    const int lib_blocks = with_library ? (ix.n_tiles * TILE + 255) / 256 : 0;
+    const int lib_blocks = (ix.n_tiles * TILE + 255) / 256;
     const int vox_blocks = (int)((ix.n_vox + 255) / 256);
     if (ix.F <= 8) launch_embed<8>(ix, meas, lib, lib_blocks, vox_blocks, s);
     else if (ix.F <= 16) launch_embed<16>(ix, meas, lib, lib_blocks, vox_blocks, s);
     else if (ix.F <= 24) launch_embed<24>(ix, meas, lib, lib_blocks, vox_blocks, s);
     else launch_embed<32>(ix, meas, lib, lib_blocks, vox_blocks, s);
     scan_kernel<<<2, 1024, 0, s>>>(ix.bins);
-    scatter_kernel<<<lib_blocks + vox_blocks, 256, 0, s>>>(ix, lib_blocks);
-    if (with_library) tile_kernel<<<ix.n_tiles, TILE, 0, s>>>(lib, ix);
+    const int sort_blocks = tiles ? lib_blocks : 0;
+    scatter_kernel<<<sort_blocks + vox_blocks, 256, 0, s>>>(ix, sort_blocks);
+    if (tiles) tile_kernel<<<ix.n_tiles, TILE, 0, s>>>(lib, ix);
     e = cudaGetLastError();
     if (e != cudaSuccess) return host::cuda_fail(e, "search index launch");
     return MADI_OK;

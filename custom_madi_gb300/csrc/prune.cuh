@@ -83,8 +83,9 @@ inline int64_t layout(Index& ix, unsigned char* base, int64_t n_vox, int32_t n_l
     return at;
 }
 
-// Enqueues the kernels that fill the index (library order, rows, boxes, voxel order).
-madi_status build(const Index& ix, const float* meas, const float* lib, bool with_library, cudaStream_t s);
+// Enqueues the kernels that fill the index: directions, embedding of the library,
+// voxel order and, with `tiles`, the library order, rows and boxes.
+madi_status build(const Index& ix, const float* meas, const float* lib, bool tiles, cudaStream_t s);
 
 // Embedding of a row x[0..F) (already centred / scaled); v = basis in shared memory.
 template <int N>

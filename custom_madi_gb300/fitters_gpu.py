@@ -150,7 +150,7 @@ def bayes_fit_gpu(measured_batch, lib_mat, kios_arr, rhos_arr, Vs_arr, sigma_m, 
     par = [torch.from_numpy(np.ascontiguousarray(a, np.float64)).to(dev)
            for a in (np.log(q), kios_arr, np.asarray(rhos_arr, np.float64), np.asarray(Vs_arr, np.float64))]
     out = torch.empty((N.MADI_BAYES_N_OUT, n_vox), dtype=torch.float64, device=dev)
-    scratch = torch.empty(int(N.lib().madi_bayes_scratch_bytes(n_lib, F)) + 256, dtype=torch.uint8, device=dev)
+    scratch = torch.empty(int(N.lib().madi_bayes_work_bytes(n_vox, n_lib, F)) + 256, dtype=torch.uint8, device=dev)
     d = N.MadiBayesDesc()
     d.measured, d.lib = N.ptr(M), N.ptr(Lm)
     d.log_weight, d.kio, d.rho, d.V = (N.ptr(t) for t in par)

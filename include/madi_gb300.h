@@ -340,7 +340,9 @@ madi_status madi_match_wait(const madi_match_desc* desc, void* stream);
  * screen the entries; the kept ones get a direct-difference fp32 residual
  * (error ~F ulp of the residual) and Kahan-compensated fp32 sums of
  * parameter differences from the best entry, combined in fp64.
- * scratch: 256-byte aligned, madi_bayes_scratch_bytes() bytes. */
+ * scratch: 256-byte aligned, at least madi_bayes_scratch_bytes() bytes; with
+ * madi_bayes_work_bytes() the fit orders the voxels and skips entries that
+ * cannot weigh in (the same sums, several times faster). */
 #define MADI_BAYES_N_OUT 9
 typedef struct madi_bayes_desc {
     const float* measured;         /* [n_vox][n_feat] (fixed: normalised; free: raw) */
@@ -360,6 +362,7 @@ typedef struct madi_bayes_desc {
 } madi_bayes_desc;
 
 int64_t madi_bayes_scratch_bytes(int32_t n_lib, int32_t n_feat);
+int64_t madi_bayes_work_bytes(int64_t n_vox, int32_t n_lib, int32_t n_feat);
 madi_status madi_bayes(const madi_bayes_desc* desc, void* stream);
 
 /* ------------------------------------------------------------------------ */
