@@ -41,8 +41,9 @@ struct TileShared {
     const Snap* snap;     // [n_grid] moment coefficients
     double* auxd;         // [3][blockDim.x] Y' at the last storage point (fp64)
     float* auxf;          // [3 + 3 NP][blockDim.x] interval-start displacement, moments dM
-    float4* fc;           // [5][blockDim.x] per-walker label cache (two facet planes + sphere)
-    uint32_t* auxc;       // [3][blockDim.x] rare counters: fp64 fallbacks, accepted, rejected crossings
+    float4* fc;           // [6][blockDim.x] per-walker label cache (three facet planes + sphere)
+    uint32_t* auxc;       // [2][blockDim.x] rare counters: accepted, rejected crossings
+    float4* queue;        // [blockDim.x / 32][NGRP] walkers of the facet pass in flight
 };
 
 // Per-walker state touched once per storage interval lives in shared memory
@@ -53,70 +54,63 @@ struct TileShared {
 #define AUX_C(k) ts.auxc[(k) * blockDim.x + threadIdx.x]
 #define FC(k) ts.fc[(k) * blockDim.x + threadIdx.x]
 
-// Per-walker label cache, built at a point q0 of cell c by a full facet pass
-// (facets k1, k2, k3 of smallest margin, every other facet's margin >= m4 as
-// computed; error bound T0 at q0):
-//   FC(0..2) = facets k1, k2, k3 (n, h);   FC(3) = (w0, R^2);
-//   FC(4) = (c, alpha_c + Tm);   FC(5) = (alpha_c - Tm, Tm, c, cell across k1),
-// Tm = 3 T0.  Every other facet k has exact m_k(q0) >= m4 - T0 and is
-// 1-Lipschitz, so for |w - w0| < R = m4 - alpha_c - 8 T0 it stays above
-// alpha_c + T(q) (T(q) <= Tm there, and the w rounding of both points adds at
-// most T(q) + T0): for q in the Voronoi cell of c (all cached margins > Tm)
-// the label follows from the three cached margins alone, by the facet-plane
-// rule.
-// A point across a cached facet goes to a full pass (the facet list of c does
-// not bound the seeds beyond it), started in the cell across k1 when k1 is
-// the facet crossed.
+// Per-walker label cache, built at a point q0 (w0 relative to the seed) by a full
+// facet pass of cell c: facets k1, k2, k3 of smallest margin, every other facet's
+// margin >= m4 as computed; T0 the error bound at q0, Tm = 3 T0.
+//   FC(0..2) = facets k1, k2, k3 (n, h);   FC(3) = (w0, M = m4 - 5 T0);
+//   FC(4) = (c, alpha_c + Tm);   FC(5) = (alpha_c - Tm, Tm, c, cell across k1).
+// Another facet k has exact m_k(q0) >= m4 - T0 and is 1-Lipschitz, and the
+// rounding of w and w0 moves |w - w0| by at most T(q) + T0, T(q) <= Tm while
+// |w - w0| < L: so exact m_k(q) >= M - |w - w0|.  With mm, ms the smallest and
+// second smallest cached margin at q (each within T(q)):
+//   inside c     if mm > alpha_c + Tm and M - |w - w0| > alpha_c + Tm;
+//   outside      if Tm <= mm < alpha_c - Tm and M - |w - w0| > Tm: q lies in the
+//                Voronoi cell of c, short of its shrunk cell;
+//   outside      if mm < Tm, mm > Tm - alpha_min, ms + mm > 2 Tm and M - |w - w0| >
+//                max(-mm, 0) + Tm: q is within delta = max(-mm, 0) + Tm < alpha_min
+//                of a point q' of the boundary of the cell of c (q moved back to
+//                the one plane it is across, the other margins staying >= 0).  At
+//                q' two seeds are nearest, so every seed i has a j with m_ij(q') <=
+//                0, hence m_ij(q) <= delta < alpha_i: q is in no shrunk cell.
+// (An extracellular walker's cell is never compared, so c serves for it.)
+// A facet pass costs a warp ~1,900 cycles of latency and was 72 % of the walk (a
+// free-water walk takes 73 ms where this one took 271: 64 entries x 25,000
+// walkers), so the rules above go for fewer of them.  Misses: 12.3 % of
+// walker-steps with the in / out rule of one sphere, 9.2 % with refused crossings
+// settled on one plane, 7.0 % with the rule across a plane, 5.9 % with M kept
+// instead of one radius; 216 ms.
 constexpr int FC_BYTES_PER_WALKER = 6 * 16;
 
-// Writes the cache of the walker in thread `w` (this CTA) from a full pass;
-// p1..p3 are the records of facets k1..k3.
-MADI_DEV void fc_build(const TileShared& ts, int w, const FacetTop& t, int c, float L, const float4& p1,
-                       const float4& p2, const float4& p3) {
-    const float Tm = 3.0f * t.T;
-    const float R = fminf(t.m4 - t.cc.w - 8.0f * t.T, L);
-    float4* f = ts.fc + w;
-    const int n = blockDim.x;
-    f[0] = p1;
-    f[n] = p2;
-    f[2 * n] = p3;
-    f[3 * n] = make_float4(t.wx, t.wy, t.wz, R > 0.f ? R * R * (1.0f - MADI_EPS19) : 0.f);
-    f[4 * n] = make_float4(t.cc.x, t.cc.y, t.cc.z, t.cc.w + Tm);
-    f[5 * n] = make_float4(t.cc.w - Tm, Tm, __int_as_float(c), __int_as_float(t.nb1));
-}
-
-// Order-preserving 32-bit key of a facet margin: the float's bits mapped to
-// unsigned order, the low KEY_BITS replaced by the facet's slot.  Dropping
-// those mantissa bits rounds the margin down (towards -inf) by at most
-// 2^(KEY_BITS - 23) relative; key_floor() returns that lower bound.
+// Sort key of a facet margin: the margin with the low KEY_BITS mantissa bits
+// replaced by the facet's slot, compared as a float.  That moves the margin by
+// at most 2^(KEY_BITS - 23) relative; key_floor() returns a lower bound of it.
 constexpr int KEY_BITS = 6;                      // slots per cell <= 64
 constexpr uint32_t KEY_SLOT = (1u << KEY_BITS) - 1u;
 
-MADI_DEV uint32_t margin_key(float m, uint32_t slot) {
-    const uint32_t b = __float_as_uint(m);
-    const uint32_t u = (b & 0x80000000u) ? ~b : (b | 0x80000000u);
-    return (u & ~KEY_SLOT) | slot;
+MADI_DEV float margin_key(float m, uint32_t slot) {
+    return __uint_as_float((__float_as_uint(m) & ~KEY_SLOT) | slot);
 }
 
-MADI_DEV float key_floor(uint32_t key) {
-    const uint32_t u = key & ~KEY_SLOT;
-    return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u);
+MADI_DEV float key_floor(float key) {
+    const uint32_t b = __float_as_uint(key);
+    return __uint_as_float((b & 0x80000000u) ? (b | KEY_SLOT) : (b & ~KEY_SLOT));
 }
 
-MADI_DEV void cx(uint32_t& a, uint32_t& b) {
-    const uint32_t lo = min(a, b), hi = max(a, b);
+MADI_DEV uint32_t key_slot(float key) { return __float_as_uint(key) & KEY_SLOT; }
+
+MADI_DEV void cx(float& a, float& b) {
+    const float lo = fminf(a, b), hi = fmaxf(a, b);
     a = lo; b = hi;
 }
 
 // ascending sort of four keys
-MADI_DEV void sort4(uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& d) {
+MADI_DEV void sort4(float& a, float& b, float& c, float& d) {
     cx(a, b); cx(c, d); cx(a, c); cx(b, d); cx(b, c);
 }
 
 // the four smallest of two ascending quadruples, ascending, into (a0..a3)
-MADI_DEV void merge4(uint32_t& a0, uint32_t& a1, uint32_t& a2, uint32_t& a3, uint32_t b0, uint32_t b1,
-                     uint32_t b2, uint32_t b3) {
-    a0 = min(a0, b3); a1 = min(a1, b2); a2 = min(a2, b1); a3 = min(a3, b0);   // bitonic
+MADI_DEV void merge4(float& a0, float& a1, float& a2, float& a3, float b0, float b1, float b2, float b3) {
+    a0 = fminf(a0, b3); a1 = fminf(a1, b2); a2 = fminf(a2, b1); a3 = fminf(a3, b0);   // bitonic
     cx(a0, a2); cx(a1, a3); cx(a0, a1); cx(a2, a3);
 }
 
@@ -131,105 +125,194 @@ MADI_DEV void merge4(uint32_t& a0, uint32_t& a1, uint32_t& a2, uint32_t& a3, uin
 // facet-plane rule and its first lane writes the walker's label cache.  A walker
 // whose point lies across a facet is queued again from the cell beyond the
 // most violated facet (at most three moves).  Called by all 32 lanes; `start`
-// is each walker's first cell.  Returns FACET_IN / FACET_OUT with cell_q
-// set, or a negative code when the voxel-grid classifier has to decide.
+// is each walker's first cell; `refuse` marks walkers inside `start` whose
+// acceptance number rejects any membrane crossing: a point outside that shrunk
+// cell ends their pass as FACET_OUT of the same cell, whatever its own label.
+// Returns FACET_IN / FACET_OUT with cell_q set, or a negative code when the
+// voxel-grid classifier has to decide.
+// The pending walkers go to their groups through a queue in shared memory:
+// (point, cell | lane << QLANE | refuse << QREFUSE).
 constexpr int FG = 4;
 constexpr int FU = 8;
+constexpr int NGRP = 32 / FG;
+constexpr int VERDICT_MOVE = 8;
+constexpr int QLANE = 24, QREFUSE = 29;          // a cell's slots take 640 B of a block < 4 GiB: cell < 2^23
 
 template <bool PERIODIC>
 MADI_DEV int coop_facets(const Geo& g, const TileShared& ts, bool need, float qx, float qy, float qz, int start,
-                         int lane, int& cell_q) {
+                         bool refuse, int lane, int& cell_q) {
     const int gid = lane / FG, sub = lane % FG;
     const int warp0 = threadIdx.x & ~31;
     const int S = g.fstride;
+    float4* queue = ts.queue + (threadIdx.x >> 5) * NGRP;
     int my_cell = start, hops = 0, r_mine = FACET_BAND;
     bool pend = need;
     unsigned pending = __ballot_sync(MADI_FULL, pend);
     while (pending) {
-        const unsigned src = __fns(pending, 0, gid + 1);      // walker of this group, ~0u if none
-        const bool act = src < 32u;
-        const int s = act ? (int)src : 0;
-        const float sx = __shfl_sync(MADI_FULL, qx, s);
-        const float sy = __shfl_sync(MADI_FULL, qy, s);
-        const float sz = __shfl_sync(MADI_FULL, qz, s);
-        const int sc = __shfl_sync(MADI_FULL, my_cell, s);
-        const uint32_t base = (uint32_t)sc * (uint32_t)S;
+        const int rank = __popc(pending & ((1u << lane) - 1u));
+        const bool mine = pend && rank < NGRP;
+        if (mine) {
+            const int tag = my_cell | (lane << QLANE) | ((refuse && hops == 0 ? 1 : 0) << QREFUSE);
+            queue[rank] = make_float4(qx, qy, qz, __int_as_float(tag));
+        }
+        __syncwarp();
+        const bool act = gid < __popc(pending);
+        float q0 = 3.4e38f, q1 = 3.4e38f, q2 = 3.4e38f, q3 = 3.4e38f;
         float4 cc = make_float4(0.f, 0.f, 0.f, 0.f);
         float wx = 0.f, wy = 0.f, wz = 0.f;
-        uint32_t q0 = 0xffffffffu, q1 = 0xffffffffu, q2 = 0xffffffffu, q3 = 0xffffffffu;
+        int tag = 0, sc = 0;
+        uint32_t base = 0;
         if (act) {
+            const float4 Q = queue[gid];
+            tag = __float_as_int(Q.w);
+            sc = tag & ((1 << QLANE) - 1);
+            base = (uint32_t)sc * (uint32_t)S;
             // the cell record and the cell's slots depend only on sc: one round trip
             cc = g.ccen[sc];
             for (int k0 = sub; k0 < S; k0 += FG * FU) {
                 float4 f[FU];
 #pragma unroll
                 for (int i = 0; i < FU; ++i) f[i] = g.fpl[base + k0 + FG * i];
-                wx = sx - cc.x; wy = sy - cc.y; wz = sz - cc.z;
+                wx = Q.x - cc.x; wy = Q.y - cc.y; wz = Q.z - cc.z;
                 if (PERIODIC) {
                     const float hl = 0.5f * g.L;
                     wx = wx > hl ? wx - g.L : (wx < -hl ? wx + g.L : wx);
                     wy = wy > hl ? wy - g.L : (wy < -hl ? wy + g.L : wy);
                     wz = wz > hl ? wz - g.L : (wz < -hl ? wz + g.L : wz);
                 }
-                uint32_t k[FU];
+                float k[FU];
 #pragma unroll
                 for (int i = 0; i < FU; ++i) k[i] = margin_key(facet_m(f[i], wx, wy, wz), (uint32_t)(k0 + FG * i));
                 sort4(k[0], k[1], k[2], k[3]);
                 sort4(k[4], k[5], k[6], k[7]);
                 merge4(k[0], k[1], k[2], k[3], k[4], k[5], k[6], k[7]);
-                merge4(q0, q1, q2, q3, k[0], k[1], k[2], k[3]);
+                if (k0 < FG) { q0 = k[0]; q1 = k[1]; q2 = k[2]; q3 = k[3]; }
+                else merge4(q0, q1, q2, q3, k[0], k[1], k[2], k[3]);
             }
         }
 #pragma unroll
         for (int o = 1; o < FG; o <<= 1) {
-            const uint32_t b0 = __shfl_xor_sync(MADI_FULL, q0, o);
-            const uint32_t b1 = __shfl_xor_sync(MADI_FULL, q1, o);
-            const uint32_t b2 = __shfl_xor_sync(MADI_FULL, q2, o);
-            const uint32_t b3 = __shfl_xor_sync(MADI_FULL, q3, o);
+            const float b0 = __shfl_xor_sync(MADI_FULL, q0, o);
+            const float b1 = __shfl_xor_sync(MADI_FULL, q1, o);
+            const float b2 = __shfl_xor_sync(MADI_FULL, q2, o);
+            const float b3 = __shfl_xor_sync(MADI_FULL, q3, o);
             merge4(q0, q1, q2, q3, b0, b1, b2, b3);
         }
-        int r = FACET_BAND, nb = -1;
+        int verdict = FACET_BAND;                     // FACET_*, or VERDICT_MOVE + the cell to go on in
         if (act) {
-            FacetTop t;
-            t.k1 = base + (q0 & KEY_SLOT);
-            t.k2 = base + (q1 & KEY_SLOT);
-            t.k3 = base + (q2 & KEY_SLOT);
-            t.m4 = key_floor(q3);
+            const uint32_t k1 = base + key_slot(q0), k2 = base + key_slot(q1), k3 = base + key_slot(q2);
             // the three candidates' records and neighbours, loaded together (L1)
-            const float4 p1 = g.fpl[t.k1], p2 = g.fpl[t.k2], p3 = g.fpl[t.k3];
-            const int n1 = g.fnbr[t.k1], n2 = g.fnbr[t.k2], n3 = g.fnbr[t.k3];
+            const float4 p1 = g.fpl[k1], p2 = g.fpl[k2], p3 = g.fpl[k3];
+            const int n1 = g.fnbr[k1], n2 = g.fnbr[k2], n3 = g.fnbr[k3];
             const float e1 = facet_m(p1, wx, wy, wz);
             const float e2 = facet_m(p2, wx, wy, wz);
             const float e3 = facet_m(p3, wx, wy, wz);
             const float m1 = fminf(e1, fminf(e2, e3));
-            t.m1 = m1;
-            t.wx = wx; t.wy = wy; t.wz = wz; t.cc = cc;
-            t.T = fmaf(2.0f * MADI_EPS21, fabsf(wx) + fabsf(wy) + fabsf(wz), g.ftol) + 7.62939453125e-6f * fabsf(m1);
-            t.nb1 = e1 <= e2 ? (e1 <= e3 ? n1 : n3) : (e2 <= e3 ? n2 : n3);
-            if (m1 > t.T) {
-                const float dd = m1 - cc.w;
-                r = dd > t.T ? FACET_IN : (dd < -t.T ? FACET_OUT : FACET_BAND);
-            } else if (m1 < -t.T) {
-                r = FACET_LEFT;
-                nb = t.nb1;
+            const float T = fmaf(2.0f * MADI_EPS21, fabsf(wx) + fabsf(wy) + fabsf(wz), g.ftol) + 7.62939453125e-6f * fabsf(m1);
+            const int nb1 = e1 <= e2 ? (e1 <= e3 ? n1 : n3) : (e2 <= e3 ? n2 : n3);
+            const float dd = m1 - cc.w;
+            if ((tag >> QREFUSE) && dd < -T && nb1 >= 0) {    // nb1 < 0: an open cell's marker, no plane
+                verdict = FACET_OUT;
+            } else if (m1 > T) {
+                verdict = dd > T ? FACET_IN : (dd < -T ? FACET_OUT : FACET_BAND);
+            } else if (m1 < -T) {
+                verdict = nb1 >= 0 ? VERDICT_MOVE + nb1 : FACET_LEFT;
             }
-            if (sub == 0 && r >= 0) fc_build(ts, warp0 + s, t, sc, g.L, p1, p2, p3);
+            if (sub == 0 && (verdict == FACET_IN || verdict == FACET_OUT)) {
+                const float Tm = 3.0f * T;
+                const float M = fminf(key_floor(q3) - 5.0f * T, g.L);
+                const int n = blockDim.x;
+                float4* fc = ts.fc + warp0 + ((tag >> QLANE) & 31);
+                fc[0] = p1;
+                fc[n] = p2;
+                fc[2 * n] = p3;
+                fc[3 * n] = make_float4(wx, wy, wz, M);
+                fc[4 * n] = make_float4(cc.x, cc.y, cc.z, cc.w + Tm);
+                fc[5 * n] = make_float4(cc.w - Tm, Tm, __int_as_float(sc), __int_as_float(nb1));
+            }
         }
         // each pending walker reads its group's verdict (group = its rank among the pending)
-        const int rank = __popc(pending & ((1u << lane) - 1u));
-        const bool mine = pend && rank < 32 / FG;
-        const int leader = (mine ? rank : 0) * FG;
-        const int rl = __shfl_sync(MADI_FULL, r, leader);
-        const int nbl = __shfl_sync(MADI_FULL, nb, leader);
+        const int v = __shfl_sync(MADI_FULL, verdict, (mine ? rank : 0) * FG);
         if (mine) {
-            if (rl == FACET_LEFT && nbl >= 0 && hops < 3) { my_cell = nbl; ++hops; }
-            else { r_mine = rl; pend = false; }
+            if (v >= VERDICT_MOVE && hops < 3) { my_cell = v - VERDICT_MOVE; ++hops; }
+            else { r_mine = v >= VERDICT_MOVE ? FACET_LEFT : v; pend = false; }
         }
+        __syncwarp();                                 // the queue is read before the next round writes it
         pending = __ballot_sync(MADI_FULL, pend);
     }
-    __syncwarp();
     cell_q = my_cell;
     return r_mine;
+}
+
+// Label of a point from the walker's cache (the rules above); true if they decide.
+// `refuse`: the walker is inside `cell` and its acceptance number rejects any
+// crossing, so a point outside that shrunk cell is as good as decided (reported
+// as outside, whatever its own label): one plane with m < alpha_c - T(q) does,
+// anywhere (t_any >= T(q)).  Otherwise `start` becomes the cell beyond the cached
+// cell's nearest facet when the point lies across it (an exact plane of it).
+template <bool PERIODIC>
+MADI_DEV bool cached_label(const TileShared& ts, float L, float qx, float qy, float qz, bool refuse, int cell, float t_any,
+                           float a_min, int& in, int& cell_q, int& start) {
+    const float4 sp = FC(3), ce = FC(4), f1 = FC(0), f2 = FC(1), f3 = FC(2), th = FC(5);
+    float wx = qx - ce.x, wy = qy - ce.y, wz = qz - ce.z;
+    if (PERIODIC) {
+        const float hl = 0.5f * L;
+        wx = wx > hl ? wx - L : (wx < -hl ? wx + L : wx);
+        wy = wy > hl ? wy - L : (wy < -hl ? wy + L : wy);
+        wz = wz > hl ? wz - L : (wz < -hl ? wz + L : wz);
+    }
+    const float m1 = facet_m(f1, wx, wy, wz), m2 = facet_m(f2, wx, wy, wz), m3 = facet_m(f3, wx, wy, wz);
+    const float mm = fminf(m1, fminf(m2, m3));
+    const float ms = fmaxf(fminf(m1, m2), fminf(fmaxf(m1, m2), m3));
+    const float ux = wx - sp.x, uy = wy - sp.y, uz = wz - sp.z;
+    const float d2 = fmaf(ux, ux, fmaf(uy, uy, uz * uz));
+    const bool in_c = mm > ce.w;
+    const float r = sp.w - (in_c ? ce.w : fmaxf(-mm, 0.f) + th.y);
+    const bool near = r > 0.f && d2 < r * r * (1.0f - MADI_EPS19);
+    const bool out = mm < th.x && (mm >= th.y || (mm > th.y - a_min && ms + mm > 2.0f * th.y));
+    const int cc = __float_as_int(th.z);
+    cell_q = cc;
+    in = in_c ? 1 : 0;
+    if (near && (in_c || out)) return true;
+    if (refuse && cc == cell && mm < th.x - t_any) { in = 0; return true; }
+    const int nb1 = __float_as_int(th.w);
+    if (!refuse && m1 < -th.y && nb1 >= 0) start = nb1;
+    return false;
+}
+
+// Voxel-grid rule for the lanes with `need`, one warp-cooperative pass each, the
+// fp64 rule where it cannot decide (a count in *fallbacks).  Rare (0.03 % of
+// walker-steps), so a function of its own: its registers stay out of the step loop.
+struct FullLabel { int status, seed, inside; };
+
+__device__ __noinline__ FullLabel full_labels(const Geo& g, bool need, float qx, float qy, float qz, int guess,
+                                              unsigned long long* fallbacks) {
+    const int lane = threadIdx.x & 31;
+    FullLabel mine{CLS_OK, 0, 0};
+    for (unsigned pend = __ballot_sync(MADI_FULL, need); pend; pend &= pend - 1) {
+        const int src = __ffs(pend) - 1;
+        const float sx = __shfl_sync(MADI_FULL, qx, src);
+        const float sy = __shfl_sync(MADI_FULL, qy, src);
+        const float sz = __shfl_sync(MADI_FULL, qz, src);
+        const int sg = __shfl_sync(MADI_FULL, guess, src);
+        int s1 = 0, in = 0;
+        const int st = coop_classify(g, sx, sy, sz, sg, lane, s1, in);
+        if (lane == src) mine = FullLabel{st, s1, in};
+    }
+    __syncwarp();
+    if (need && mine.status == CLS_FALLBACK) {
+        mine.status = classify_list_f64(g, qx, qy, qz, mine.seed, mine.inside);
+        atomicAdd(fallbacks, 1ull);
+    }
+    return mine;
+}
+
+// Empties the walker's label cache.
+MADI_DEV void clear_cache(const TileShared& ts) {
+    FC(0) = FC(1) = FC(2) = make_float4(0.f, 0.f, 0.f, 3.0e38f);
+    FC(3) = make_float4(0.f, 0.f, 0.f, -1.f);
+    FC(4) = make_float4(0.f, 0.f, 0.f, 0.f);
+    FC(5) = make_float4(0.f, 0.f, __int_as_float(-1), __int_as_float(-1));
 }
 
 // Walk one tile (blockDim.x walkers of one job) on geometry view g.
@@ -275,32 +358,17 @@ __device__ __forceinline__ void walk_tile(const madi_walk_desc& d, const madi_wa
     bool frozen = !active;
     uint32_t n_full = 0, n_t1 = 0, n_fp = 0, escaped = 0, cerr = 0;
 #pragma unroll
-    for (int k = 0; k < 3; ++k) { AUX_Y(k) = 0.0; AUX_A(k) = 0.f; AUX_C(k) = 0u; }
+    for (int k = 0; k < 3; ++k) { AUX_Y(k) = 0.0; AUX_A(k) = 0.f; }
+    AUX_C(0) = AUX_C(1) = 0u;
+    unsigned long long* const cnt = reinterpret_cast<unsigned long long*>(d.counters + (size_t)job.slot * MADI_CNT_N);
 #pragma unroll
     for (int p = 0; p < NP; ++p) { AUX_M(p, 0) = 0.f; AUX_M(p, 1) = 0.f; AUX_M(p, 2) = 0.f; }
-    FC(0) = make_float4(0.f, 0.f, 0.f, 3.0e38f);  // empty label cache
-    FC(3) = make_float4(0.f, 0.f, 0.f, 0.f);
-    FC(4) = make_float4(0.f, 0.f, 0.f, 0.f);
-    FC(5) = make_float4(0.f, 0.f, __int_as_float(-1), __int_as_float(-1));
+    clear_cache(ts);
     if (cells) {
-        int my_st = CLS_OK, my_s1 = 0, my_in = 0;
-        for (unsigned pend = __ballot_sync(MADI_FULL, active); pend; pend &= pend - 1) {
-            const int src = __ffs(pend) - 1;
-            const float sx = __shfl_sync(MADI_FULL, px, src);
-            const float sy = __shfl_sync(MADI_FULL, py, src);
-            const float sz = __shfl_sync(MADI_FULL, pz, src);
-            int s1 = 0, in = 0;
-            const int st = coop_classify(g, sx, sy, sz, -1, lane, s1, in);
-            if (lane == src) { my_st = st; my_s1 = s1; my_in = in; }
-        }
-        __syncwarp();
+        const FullLabel f = full_labels(g, active, px, py, pz, -1, &cnt[MADI_CNT_FALLBACK64]);
         if (active) {
-            if (my_st == CLS_FALLBACK) {
-                my_st = classify_list_f64(g, px, py, pz, my_s1, my_in);
-                ++AUX_C(0);
-            }
-            if (my_st != CLS_OK) { cerr = 1; dead = true; }
-            else { cell = cell_of(g, my_s1); inside = my_in; }
+            if (f.status != CLS_OK) { cerr = 1; dead = true; }
+            else { cell = cell_of(g, f.seed); inside = f.inside; }
             ++n_full;
         }
     }
@@ -318,10 +386,14 @@ __device__ __forceinline__ void walk_tile(const madi_walk_desc& d, const madi_wa
     }
     const bool always = job.pp >= 1.0;
     const uint32_t th1 = (uint32_t)(job.thr1 >> 32), th2 = (uint32_t)(job.thr2 >> 32);
+    // error bound of any facet margin in the box (|w|_1 <= 3 L)
+    const float t_any = fmaf(6.0f * MADI_EPS21, L, (float)gd.facet_tol);
+    const float a_min = gd.alpha_min;
     float g3 = 0.f, g4 = 0.f, g5 = 0.f;
     uint32_t acc_word_odd = 0;
     int h_left = d.steps_per_h;
     int jgrid = 0;
+#pragma unroll 1
     for (int step = 0; step < d.n_steps; ++step) {
         // ---- random numbers: one Philox call per step on average ----
         float nx, ny, nz;
@@ -370,67 +442,33 @@ __device__ __forceinline__ void walk_tile(const madi_walk_desc& d, const madi_wa
             }
         }
         const float ex = dx + nx, ey = dy + ny, ez = dz + nz;
-        // ---- label from the facet planes of the current cell (and its neighbours) ----
+        // ---- label from the cached facet planes ----
+        const bool refuse = inside && !always && (stream ? ustream >= job.pp : word > th1);
         bool t1 = false;
         int t1_in = 0, t1_cell = cell;
         int start = cell;
-        if (ok && facets) {
-            // inside the cached sphere three planes decide
-            const float4 sp = FC(3), ce = FC(4), f1 = FC(0), th = FC(5);
-            float wx = qx - ce.x, wy = qy - ce.y, wz = qz - ce.z;
-            if (PERIODIC) {
-                const float hl = 0.5f * L;
-                wx = wx > hl ? wx - L : (wx < -hl ? wx + L : wx);
-                wy = wy > hl ? wy - L : (wy < -hl ? wy + L : wy);
-                wz = wz > hl ? wz - L : (wz < -hl ? wz + L : wz);
-            }
-            const float m1 = facet_m(f1, wx, wy, wz);
-            const float ux = wx - sp.x, uy = wy - sp.y, uz = wz - sp.z;
-            if (fmaf(ux, ux, fmaf(uy, uy, uz * uz)) < sp.w) {
-                const float4 f2 = FC(1), f3 = FC(2);
-                const float mm = fminf(m1, fminf(facet_m(f2, wx, wy, wz), facet_m(f3, wx, wy, wz)));
-                if (mm > ce.w) { t1 = true; t1_in = 1; t1_cell = __float_as_int(th.z); }
-                else if (mm > th.y && mm < th.x) { t1 = true; t1_in = 0; t1_cell = __float_as_int(th.z); }
-            }
-            // across the cached cell's nearest facet (an exact plane of it): start
-            // the full pass in the cell beyond
-            const int nb1 = __float_as_int(th.w);
-            if (!t1 && m1 < -th.y && nb1 >= 0) start = nb1;
-        }
+        if (ok && facets)
+            t1 = cached_label<PERIODIC>(ts, L, qx, qy, qz, refuse, cell, t_any, a_min, t1_in, t1_cell, start);
         // ---- cache misses: cooperative full facet passes, which rebuild the caches ----
         const bool miss = ok && facets && !t1;
         n_fp += miss ? 1u : 0u;
         if (__any_sync(MADI_FULL, miss)) {
             int cq = start;
-            const int r = coop_facets<PERIODIC>(g, ts, miss, qx, qy, qz, start, lane, cq);
+            const int r = coop_facets<PERIODIC>(g, ts, miss, qx, qy, qz, start, refuse, lane, cq);
             if (miss && r >= 0) { t1 = true; t1_in = r; t1_cell = cq; }
         }
-        // ---- full classifications of this step, one warp-cooperative pass each ----
+        // ---- full classifications of this step ----
         const bool need = ok && cells && !t1;
-        int my_st = CLS_OK, my_s1 = 0, my_in = 0;
-        for (unsigned pend = __ballot_sync(MADI_FULL, need); pend; pend &= pend - 1) {
-            const int src = __ffs(pend) - 1;
-            const float sx = __shfl_sync(MADI_FULL, qx, src);
-            const float sy = __shfl_sync(MADI_FULL, qy, src);
-            const float sz = __shfl_sync(MADI_FULL, qz, src);
-            const int sg = __shfl_sync(MADI_FULL, cell, src);
-            int s1 = 0, in = 0;
-            const int st = coop_classify(g, sx, sy, sz, sg, lane, s1, in);
-            if (lane == src) { my_st = st; my_s1 = s1; my_in = in; }
-        }
-        __syncwarp();
+        FullLabel full{CLS_OK, 0, 0};
+        if (__any_sync(MADI_FULL, need)) full = full_labels(g, need, qx, qy, qz, cell, &cnt[MADI_CNT_FALLBACK64]);
         if (ok) {
             int ncell = 0, nin = 0;
             if (t1) {
                 ncell = t1_cell; nin = t1_in; ++n_t1;
             } else if (need) {
-                if (my_st == CLS_FALLBACK) {
-                    my_st = classify_list_f64(g, qx, qy, qz, my_s1, my_in);
-                    ++AUX_C(0);
-                }
                 ++n_full;
-                if (my_st != CLS_OK) { cerr = 1; dead = true; }
-                else { ncell = cell_of(g, my_s1); nin = my_in; }
+                if (full.status != CLS_OK) { cerr = 1; dead = true; }
+                else { ncell = cell_of(g, full.seed); nin = full.inside; }
             }
             if (!dead) {
                 int m = 0;
@@ -450,7 +488,7 @@ __device__ __forceinline__ void walk_tile(const madi_walk_desc& d, const madi_wa
                             accept = rc.x < (uint32_t)thr;
                         }
                     }
-                    ++AUX_C(accept ? 1 : 2);
+                    ++AUX_C(accept ? 0 : 1);
                 }
                 if (accept) {
                     px = qx; py = qy; pz = qz;
@@ -540,33 +578,29 @@ __device__ __forceinline__ void walk_tile(const madi_walk_desc& d, const madi_wa
     }
     // ---- counters ----
     {
-        uint64_t* cnt = d.counters + (size_t)job.slot * MADI_CNT_N;
         const uint32_t v0 = __reduce_add_sync(0xffffffffu, active ? 1u : 0u);
         const uint32_t v1 = __reduce_add_sync(0xffffffffu, escaped);
         const uint32_t v2 = __reduce_add_sync(0xffffffffu, cerr);
         const uint32_t v3 = __reduce_add_sync(0xffffffffu, n_full);
         const uint32_t v4 = __reduce_add_sync(0xffffffffu, n_t1);
-        const uint32_t v5 = __reduce_add_sync(0xffffffffu, AUX_C(0));
-        const uint32_t v6 = __reduce_add_sync(0xffffffffu, AUX_C(1));
-        const uint32_t v7 = __reduce_add_sync(0xffffffffu, AUX_C(2));
+        const uint32_t v6 = __reduce_add_sync(0xffffffffu, AUX_C(0));
+        const uint32_t v7 = __reduce_add_sync(0xffffffffu, AUX_C(1));
         const uint32_t v8 = __reduce_add_sync(0xffffffffu, n_fp);
         if (lane == 0) {
-            unsigned long long* c = reinterpret_cast<unsigned long long*>(cnt);
-            if (v0) atomicAdd(&c[0], (unsigned long long)v0);
-            if (v1) atomicAdd(&c[1], (unsigned long long)v1);
-            if (v2) atomicAdd(&c[2], (unsigned long long)v2);
-            if (v3) atomicAdd(&c[3], (unsigned long long)v3);
-            if (v4) atomicAdd(&c[4], (unsigned long long)v4);
-            if (v5) atomicAdd(&c[5], (unsigned long long)v5);
-            if (v6) atomicAdd(&c[6], (unsigned long long)v6);
-            if (v7) atomicAdd(&c[7], (unsigned long long)v7);
-            if (v8) atomicAdd(&c[MADI_CNT_FACET_PASS], (unsigned long long)v8);
+            if (v0) atomicAdd(&cnt[MADI_CNT_WALKERS], (unsigned long long)v0);
+            if (v1) atomicAdd(&cnt[MADI_CNT_ESCAPED], (unsigned long long)v1);
+            if (v2) atomicAdd(&cnt[MADI_CNT_CLASSIFIER_ERROR], (unsigned long long)v2);
+            if (v3) atomicAdd(&cnt[MADI_CNT_FULL], (unsigned long long)v3);
+            if (v4) atomicAdd(&cnt[MADI_CNT_TIER1], (unsigned long long)v4);
+            if (v6) atomicAdd(&cnt[MADI_CNT_CROSS_ACCEPT], (unsigned long long)v6);
+            if (v7) atomicAdd(&cnt[MADI_CNT_CROSS_REJECT], (unsigned long long)v7);
+            if (v8) atomicAdd(&cnt[MADI_CNT_FACET_PASS], (unsigned long long)v8);
         }
     }
 }
 
 template <int OUT, bool PERIODIC, int NP, int MINB>
-__global__ void __launch_bounds__(256, MINB) walk_f32_kernel(const madi_walk_desc d) {
+__global__ void __launch_bounds__(256, MINB) walk_f32_kernel(const __grid_constant__ madi_walk_desc d) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int s_item;
     const int nthr = blockDim.x;
@@ -584,6 +618,7 @@ __global__ void __launch_bounds__(256, MINB) walk_f32_kernel(const madi_walk_des
     ts.fc = reinterpret_cast<float4*>(aux + 24 * nthr);
     ts.auxf = reinterpret_cast<float*>(aux + (24 + FC_BYTES_PER_WALKER) * nthr);
     ts.auxc = reinterpret_cast<uint32_t*>(ts.auxf + (3 + 3 * NP) * nthr);
+    ts.queue = reinterpret_cast<float4*>(ts.auxc + 2 * nthr);    // 2 of the 4 bytes a walker left of the 12
 
     for (int j = tid; j < d.n_grid; j += nthr) {
         uint32_t code = 0, any = 0;
@@ -614,19 +649,14 @@ __global__ void __launch_bounds__(256, MINB) walk_f32_kernel(const madi_walk_des
         const madi_geometry gd = d.geoms[job.geom];
         const int local = (item - job.tile_begin) * nthr + tid;
         const bool here = d.stage_smem > 0 && (int)gd.stage_bytes <= d.stage_smem;
-        if (here) {
-            if (job.geom != cur_geom) {
-                const uint4* src = reinterpret_cast<const uint4*>(gd.stage);
-                uint4* dst = reinterpret_cast<uint4*>(stage);
-                for (uint32_t i = tid; i < gd.stage_bytes / 16u; i += nthr) dst[i] = src[i];
-                cur_geom = job.geom;
-                __syncthreads();
-            }
-            walk_tile<OUT, PERIODIC, NP>(d, job, gd, make_geo(gd, stage), local, ts);
-        } else {
-            walk_tile<OUT, PERIODIC, NP>(d, job, gd, make_geo(gd, reinterpret_cast<const unsigned char*>(gd.stage)),
-                                         local, ts);
+        if (here && job.geom != cur_geom) {
+            const uint4* src = reinterpret_cast<const uint4*>(gd.stage);
+            uint4* dst = reinterpret_cast<uint4*>(stage);
+            for (uint32_t i = tid; i < gd.stage_bytes / 16u; i += nthr) dst[i] = src[i];
+            cur_geom = job.geom;
         }
+        __syncthreads();
+        walk_tile<OUT, PERIODIC, NP>(d, job, gd, make_geo(gd, here ? stage : reinterpret_cast<const unsigned char*>(gd.stage)), local, ts);
         __syncthreads();
         if (OUT == MADI_OUT_FUSED) {
             long long* out = reinterpret_cast<long long*>(d.accum) + (size_t)job.slot * 2 * n_out;
@@ -656,41 +686,6 @@ __global__ void __launch_bounds__(256, MINB) walk_f32_kernel(const madi_walk_des
 // ---------------------------------------------------------------------------
 constexpr int F64_THREADS = 128;
 
-// Label of a point from the walker's cache: true when the three cached planes
-// decide (inside the cached sphere, no margin within its band).  Otherwise
-// `start` becomes the cell beyond the cached cell's nearest facet when the point
-// lies across it (an exact plane of that cell).
-template <bool PERIODIC>
-MADI_DEV bool cached_label(const TileShared& ts, float L, float qx, float qy, float qz, int& in, int& cell, int& start) {
-    const float4 sp = FC(3), ce = FC(4), f1 = FC(0), th = FC(5);
-    float wx = qx - ce.x, wy = qy - ce.y, wz = qz - ce.z;
-    if (PERIODIC) {
-        const float hl = 0.5f * L;
-        wx = wx > hl ? wx - L : (wx < -hl ? wx + L : wx);
-        wy = wy > hl ? wy - L : (wy < -hl ? wy + L : wy);
-        wz = wz > hl ? wz - L : (wz < -hl ? wz + L : wz);
-    }
-    const float m1 = facet_m(f1, wx, wy, wz);
-    const float ux = wx - sp.x, uy = wy - sp.y, uz = wz - sp.z;
-    if (fmaf(ux, ux, fmaf(uy, uy, uz * uz)) < sp.w) {
-        const float4 f2 = FC(1), f3 = FC(2);
-        const float mm = fminf(m1, fminf(facet_m(f2, wx, wy, wz), facet_m(f3, wx, wy, wz)));
-        if (mm > ce.w) { in = 1; cell = __float_as_int(th.z); return true; }
-        if (mm > th.y && mm < th.x) { in = 0; cell = __float_as_int(th.z); return true; }
-    }
-    const int nb1 = __float_as_int(th.w);
-    if (m1 < -th.y && nb1 >= 0) start = nb1;
-    return false;
-}
-
-// Empties the walker's label cache.
-MADI_DEV void clear_cache(const TileShared& ts) {
-    FC(0) = make_float4(0.f, 0.f, 0.f, 3.0e38f);
-    FC(3) = make_float4(0.f, 0.f, 0.f, 0.f);
-    FC(4) = make_float4(0.f, 0.f, 0.f, 0.f);
-    FC(5) = make_float4(0.f, 0.f, __int_as_float(-1), __int_as_float(-1));
-}
-
 // The six normals of step pair `pair` of walker widx from the Philox stream of
 // the fp32 walker, in fp64 (Box-Muller: u1 = (w + 1/2) 2^-32, u2 = (w' >> 8)
 // 2^-24; the first three are the even step's), and the two acceptance words: the
@@ -714,9 +709,10 @@ MADI_DEV void normals_f64(uint32_t widx, uint32_t pair, uint32_t k0, uint32_t k1
 }
 
 __global__ void __launch_bounds__(F64_THREADS) walk_f64_kernel(const madi_walk_desc d) {
-    __shared__ float4 s_fc[FC_BYTES_PER_WALKER / 16 * F64_THREADS];
+    __shared__ float4 s_fc[FC_BYTES_PER_WALKER / 16 * F64_THREADS], s_queue[F64_THREADS / 32 * NGRP];
     TileShared ts{};
     ts.fc = s_fc;
+    ts.queue = s_queue;
     const madi_walk_job job = d.jobs[0];
     const int lane = threadIdx.x & 31;
     const int w0 = blockIdx.x * blockDim.x + threadIdx.x;
@@ -747,7 +743,7 @@ __global__ void __launch_bounds__(F64_THREADS) walk_f64_kernel(const madi_walk_d
         }
     }
     const bool facets = cells && gd.n_cells > 0;
-    const float Lf = (float)L;
+    const float Lf = (float)L, a_min = gd.alpha_min;
     clear_cache(ts);
     int cell = 0, inside = 0, escaped = 0, cerr = 0;
     uint32_t n_acc = 0, n_rej = 0, n_full = 0;
@@ -811,13 +807,14 @@ __global__ void __launch_bounds__(F64_THREADS) walk_f64_kernel(const madi_walk_d
             // a step longer than the box leaves a periodic point outside after one wrap
             const bool boxed = ok && fminf(fx, fminf(fy, fz)) >= 0.f && fmaxf(fx, fmaxf(fy, fz)) <= Lf;
             int start = cell;
-            if (boxed) known = periodic ? cached_label<true>(ts, Lf, fx, fy, fz, nin, ncell, start)
-                                        : cached_label<false>(ts, Lf, fx, fy, fz, nin, ncell, start);
+            // (no early refusal here: `refuse` is false)
+            if (boxed) known = periodic ? cached_label<true>(ts, Lf, fx, fy, fz, false, cell, 0.f, a_min, nin, ncell, start)
+                                        : cached_label<false>(ts, Lf, fx, fy, fz, false, cell, 0.f, a_min, nin, ncell, start);
             const bool miss = boxed && !known;
             if (__any_sync(MADI_FULL, miss)) {
                 int cq = start;
-                const int r = periodic ? coop_facets<true>(g, ts, miss, fx, fy, fz, start, lane, cq)
-                                       : coop_facets<false>(g, ts, miss, fx, fy, fz, start, lane, cq);
+                const int r = periodic ? coop_facets<true>(g, ts, miss, fx, fy, fz, start, false, lane, cq)
+                                       : coop_facets<false>(g, ts, miss, fx, fy, fz, start, false, lane, cq);
                 if (miss && r >= 0) { known = true; nin = r; ncell = cq; }
             }
         }

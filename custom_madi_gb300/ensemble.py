@@ -479,6 +479,8 @@ class DeviceGeometry:
         s.facet_stride = self.facet_stride
         s.n_cells = n_cells
         s.facet_tol = self.facet_tol
+        # rounded down: a lower bound of every fp64 annulus
+        s.alpha_min = float(np.min(ann)) * (1.0 - 2.0 ** -22) if n_cells > 0 else 0.0
         self.struct = s
         self.stage_bytes = len(blob)
 

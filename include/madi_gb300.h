@@ -97,7 +97,7 @@ typedef struct madi_geometry {
     uint32_t off_facet_plane;      /* float4 [n_cells][facet_stride]: n, offset h */
     uint32_t off_facet_nbr;        /* int32 [n_cells][facet_stride]: cell across  */
     int32_t  n_cells;              /* cells in the table (0 = no table)           */
-    int32_t  pad1;
+    float    alpha_min;            /* <= every cell's alpha (0: not known)        */
     double   facet_tol;            /* fp32 error of h - n.w, without the |w| term */
 } madi_geometry;
 

@@ -398,3 +398,42 @@ def test_f64_walker_labels_equal_kd_rule(n_walkers, n_cells, rho, V):
     ens._device.clear()
     for x, y in zip(*out):
         assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("mode, n_cells, rho, V, pp", [
+    ("periodic", 2, 2.0e5, 4.0, 0.3),       # cells that face their own images
+    ("periodic", 27, 5.0e7, 0.017, 0.02),   # steps a sixth of the cell spacing
+    ("periodic", 64, 2.0e5, 2.6, 1.0),      # thick extracellular space, every crossing accepted
+    ("periodic", 64, 2.0e5, 4.9, 0.0),      # thin extracellular space, every crossing refused
+    ("si_fatal_escape", 0, 2.0e5, 3.0, 0.05),   # open outer cells
+])
+def test_f32_walker_equals_voxel_grid_rule(mode, n_cells, rho, V, pp):
+    """Label cache, early refusal and facet passes walk exactly as the voxel-grid
+    rule does on every step (the same walk with the facet table taken away): equal
+    phase sums, occupancy and crossing counts, bit for bit."""
+    import torch
+    from custom_madi_gb300 import signal as S
+    from custom_madi_gb300.ensemble import create_ensemble
+    from custom_madi_gb300.walker_gpu import WalkBatch, WalkJob, pair_layout
+    n = 225                                  # a ragged tile
+    over = dict(boundary_mode="periodic", n_cells=n_cells) if mode == "periodic" else {}
+    cfg = SimConfig(n_walkers=n, n_ensembles=1, ts=0.01, T_max_ms=6.0, small_deltas=[1.0], big_deltas=[3.0],
+                    b_values=[0.0, 1000.0, 3000.0], **over)
+    ens = create_ensemble(rho, V, cfg, seed=3, verify_vi=False, measure_vi=False)
+    c = S.build_columns(cfg)
+    lay = pair_layout(c.j_delta, c.j_Delta, c.j_sum, c.phase_coef)
+    out = []
+    for table in (True, False):
+        ens._device.clear()
+        dev = ens.device()
+        if not table:
+            dev.struct.n_cells = 0
+        b = WalkBatch([WalkJob(ens, pp, 11, n), WalkJob(ens, pp, 12, n, walker_base=77)], cfg, layout=lay)
+        b.launch()
+        torch.cuda.synchronize()
+        cnt = b.counters_np()
+        assert (cnt[:, 8] > 0).all() == table        # facet passes only with the table
+        out.append((b.accum.cpu().numpy(), b.occupancy.cpu().numpy(), cnt[:, [0, 1, 2, 6, 7]]))
+    ens._device.clear()
+    for x, y in zip(*out):
+        assert np.array_equal(x, y)
