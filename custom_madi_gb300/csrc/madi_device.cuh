@@ -69,6 +69,7 @@ struct Geo {
     const int32_t* fnbr;        // [n_cells][fstride] cell across the facet
     int n_cells;
     float ftol;                 // fp32 error of a facet margin, without the |w| term
+    bool sorted;                // every cell's slots are in ascending order of h
 };
 
 MADI_DEV Geo make_geo(const madi_geometry& g, const unsigned char* base) {
@@ -93,6 +94,7 @@ MADI_DEV Geo make_geo(const madi_geometry& g, const unsigned char* base) {
     v.fnbr = reinterpret_cast<const int32_t*>(base + g.off_facet_nbr);
     v.n_cells = g.n_cells;
     v.ftol = (float)g.facet_tol;
+    v.sorted = g.alpha_min > 0.f;
     return v;
 }
 
@@ -312,18 +314,6 @@ enum { FACET_OUT = 0, FACET_IN = 1, FACET_LEFT = -1, FACET_BAND = -2 };
 MADI_DEV float facet_m(const float4 f, float wx, float wy, float wz) {
     return fmaf(-f.z, wz, fmaf(-f.y, wy, fmaf(-f.x, wx, f.w)));
 }
-
-// Result of a full facet pass: the three facets of smallest margin (slots
-// k1..k3), the smallest margin m1, a lower bound m4 on every other facet's
-// margin, the cell across the most violated facet, the point w relative to the
-// cell centre cc, and the error bound T at w.
-struct FacetTop {
-    float m1, m4;
-    uint32_t k1, k2, k3;
-    int nb1;                    // cell across the facet of margin m1
-    float wx, wy, wz, T;
-    float4 cc;
-};
 
 // ---------------------------------------------------------------------------
 // fp64 rule on the voxel candidate list: nearest seed, then every seed within

@@ -58,7 +58,7 @@ struct TileShared {
 // facet pass of cell c: facets k1, k2, k3 of smallest margin, every other facet's
 // margin >= m4 as computed; T0 the error bound at q0, Tm = 3 T0.
 //   FC(0..2) = facets k1, k2, k3 (n, h);   FC(3) = (w0, M = m4 - 5 T0);
-//   FC(4) = (c, alpha_c + Tm);   FC(5) = (alpha_c - Tm, Tm, c, cell across k1).
+//   FC(4) = (c, cell across k2);   FC(5) = (alpha_c - Tm, Tm, c, cell across k1).
 // Another facet k has exact m_k(q0) >= m4 - T0 and is 1-Lipschitz, and the
 // rounding of w and w0 moves |w - w0| by at most T(q) + T0, T(q) <= Tm while
 // |w - w0| < L: so exact m_k(q) >= M - |w - w0|.  With mm, ms the smallest and
@@ -78,7 +78,8 @@ struct TileShared {
 // walkers), so the rules above go for fewer of them.  Misses: 12.3 % of
 // walker-steps with the in / out rule of one sphere, 9.2 % with refused crossings
 // settled on one plane, 7.0 % with the rule across a plane, 5.9 % with M kept
-// instead of one radius; 216 ms.
+// instead of one radius (216 ms), 6.3 % with the first 16 slots deciding where
+// they can, in half the loads and sorting (203 ms).
 constexpr int FC_BYTES_PER_WALKER = 6 * 16;
 
 // Sort key of a facet margin: the margin with the low KEY_BITS mantissa bits
@@ -115,25 +116,28 @@ MADI_DEV void merge4(float& a0, float& a1, float& a2, float& a3, float b0, float
 }
 
 // Full facet passes for the lanes with `need`, warp-cooperatively: a group of
-// FG lanes takes one walker, splits its cell's facet slots (FU loads per lane
-// in flight, coalesced), keeps each lane's four smallest margin keys with
-// sorting networks and merges the group's in log2(FG) butterfly rounds.  The
-// three smallest keys name the cached facets, whose margins are recomputed
-// exactly (the true smallest margin is among them unless four margins lie
-// within 2^-17 relative of each other, which the widened band covers); the
-// fourth key bounds every other facet from below.  The group decides by the
-// facet-plane rule and its first lane writes the walker's label cache.  A walker
-// whose point lies across a facet is queued again from the cell beyond the
-// most violated facet (at most three moves).  Called by all 32 lanes; `start`
-// is each walker's first cell; `refuse` marks walkers inside `start` whose
-// acceptance number rejects any membrane crossing: a point outside that shrunk
-// cell ends their pass as FACET_OUT of the same cell, whatever its own label.
-// Returns FACET_IN / FACET_OUT with cell_q set, or a negative code when the
-// voxel-grid classifier has to decide.
+// FG lanes takes one walker and FG FU of its cell's facet slots (FU coalesced
+// loads per lane in flight), keeps each lane's four smallest margin keys with a
+// sorting network and merges the group's in log2(FG) butterfly rounds.  The three
+// smallest keys name the cached facets, whose margins are recomputed exactly (the
+// true smallest margin is among them unless four margins lie within 2^-17 relative
+// of each other, which the widened band covers); the fourth key bounds every other
+// facet from below.  Slots are in order of h and m_k >= h_k - |w|, so the first 16
+// slots decide whenever the last of them has h - |w| above the smallest margin
+// (`rest`, which then bounds the slots not read); else the next 16 follow.  The
+// group decides by the facet-plane rule and its first lane writes the walker's
+// label cache.  A walker whose point lies across a facet is queued again from the
+// cell beyond the most violated facet (at most three moves).  Called by all 32
+// lanes; `start` is each walker's first cell; `refuse` marks walkers inside
+// `start` whose acceptance number rejects any membrane crossing: a point outside
+// that shrunk cell ends their pass as FACET_OUT of the same cell, whatever its own
+// label.  Results: FACET_IN / FACET_OUT with cell_q set, or a negative code when
+// the voxel-grid classifier has to decide.
 // The pending walkers go to their groups through a queue in shared memory:
-// (point, cell | lane << QLANE | refuse << QREFUSE).
+// (point, cell | lane << QLANE | refuse << QREFUSE).  Groups without a walker work
+// on cell 0 and are ignored: a pass is one chain of ~1,000 cycles with no branch.
 constexpr int FG = 4;
-constexpr int FU = 8;
+constexpr int FU = 4;
 constexpr int NGRP = 32 / FG;
 constexpr int VERDICT_MOVE = 8;
 constexpr int QLANE = 24, QREFUSE = 29;          // a cell's slots take 640 B of a block < 4 GiB: cell < 2^23
@@ -157,22 +161,22 @@ MADI_DEV int coop_facets(const Geo& g, const TileShared& ts, bool need, float qx
         }
         __syncwarp();
         const bool act = gid < __popc(pending);
-        float q0 = 3.4e38f, q1 = 3.4e38f, q2 = 3.4e38f, q3 = 3.4e38f;
-        float4 cc = make_float4(0.f, 0.f, 0.f, 0.f);
-        float wx = 0.f, wy = 0.f, wz = 0.f;
-        int tag = 0, sc = 0;
-        uint32_t base = 0;
-        if (act) {
-            const float4 Q = queue[gid];
-            tag = __float_as_int(Q.w);
-            sc = tag & ((1 << QLANE) - 1);
-            base = (uint32_t)sc * (uint32_t)S;
-            // the cell record and the cell's slots depend only on sc: one round trip
-            cc = g.ccen[sc];
-            for (int k0 = sub; k0 < S; k0 += FG * FU) {
-                float4 f[FU];
+        const float4 Q = queue[gid];
+        const int tag = act ? __float_as_int(Q.w) : 0;
+        const int sc = tag & ((1 << QLANE) - 1);
+        const uint32_t base = (uint32_t)sc * (uint32_t)S;
+        // the cell record and its first slots depend only on sc: one round trip
+        const float4 cc = g.ccen[sc];
+        float wx = 0.f, wy = 0.f, wz = 0.f, m1 = 0.f, T = 0.f, rest = 0.f;
+        float q0 = 0.f, q1 = 0.f, q2 = 0.f, q3 = 0.f;
+        float4 p1, p2, p3;
+        int nb1 = -1, nb2 = -1, k0 = 0;
+        bool more;
+        do {
+            float4 f[FU];
 #pragma unroll
-                for (int i = 0; i < FU; ++i) f[i] = g.fpl[base + k0 + FG * i];
+            for (int i = 0; i < FU; ++i) f[i] = g.fpl[base + k0 + sub + FG * i];
+            if (k0 == 0) {
                 wx = Q.x - cc.x; wy = Q.y - cc.y; wz = Q.z - cc.z;
                 if (PERIODIC) {
                     const float hl = 0.5f * g.L;
@@ -180,56 +184,55 @@ MADI_DEV int coop_facets(const Geo& g, const TileShared& ts, bool need, float qx
                     wy = wy > hl ? wy - g.L : (wy < -hl ? wy + g.L : wy);
                     wz = wz > hl ? wz - g.L : (wz < -hl ? wz + g.L : wz);
                 }
-                float k[FU];
-#pragma unroll
-                for (int i = 0; i < FU; ++i) k[i] = margin_key(facet_m(f[i], wx, wy, wz), (uint32_t)(k0 + FG * i));
-                sort4(k[0], k[1], k[2], k[3]);
-                sort4(k[4], k[5], k[6], k[7]);
-                merge4(k[0], k[1], k[2], k[3], k[4], k[5], k[6], k[7]);
-                if (k0 < FG) { q0 = k[0]; q1 = k[1]; q2 = k[2]; q3 = k[3]; }
-                else merge4(q0, q1, q2, q3, k[0], k[1], k[2], k[3]);
             }
-        }
+            float k[FU];
 #pragma unroll
-        for (int o = 1; o < FG; o <<= 1) {
-            const float b0 = __shfl_xor_sync(MADI_FULL, q0, o);
-            const float b1 = __shfl_xor_sync(MADI_FULL, q1, o);
-            const float b2 = __shfl_xor_sync(MADI_FULL, q2, o);
-            const float b3 = __shfl_xor_sync(MADI_FULL, q3, o);
-            merge4(q0, q1, q2, q3, b0, b1, b2, b3);
-        }
-        int verdict = FACET_BAND;                     // FACET_*, or VERDICT_MOVE + the cell to go on in
-        if (act) {
+            for (int i = 0; i < FU; ++i) k[i] = margin_key(facet_m(f[i], wx, wy, wz), (uint32_t)(k0 + sub + FG * i));
+            sort4(k[0], k[1], k[2], k[3]);
+#pragma unroll
+            for (int o = 1; o < FG; o <<= 1) {
+                const float b0 = __shfl_xor_sync(MADI_FULL, k[0], o);
+                const float b1 = __shfl_xor_sync(MADI_FULL, k[1], o);
+                const float b2 = __shfl_xor_sync(MADI_FULL, k[2], o);
+                const float b3 = __shfl_xor_sync(MADI_FULL, k[3], o);
+                merge4(k[0], k[1], k[2], k[3], b0, b1, b2, b3);
+            }
+            if (k0 == 0) { q0 = k[0]; q1 = k[1]; q2 = k[2]; q3 = k[3]; }
+            else merge4(q0, q1, q2, q3, k[0], k[1], k[2], k[3]);
+            const float h_last = __shfl_sync(MADI_FULL, f[FU - 1].w, lane | (FG - 1));
             const uint32_t k1 = base + key_slot(q0), k2 = base + key_slot(q1), k3 = base + key_slot(q2);
             // the three candidates' records and neighbours, loaded together (L1)
-            const float4 p1 = g.fpl[k1], p2 = g.fpl[k2], p3 = g.fpl[k3];
+            p1 = g.fpl[k1]; p2 = g.fpl[k2]; p3 = g.fpl[k3];
             const int n1 = g.fnbr[k1], n2 = g.fnbr[k2], n3 = g.fnbr[k3];
             const float e1 = facet_m(p1, wx, wy, wz);
             const float e2 = facet_m(p2, wx, wy, wz);
             const float e3 = facet_m(p3, wx, wy, wz);
-            const float m1 = fminf(e1, fminf(e2, e3));
-            const float T = fmaf(2.0f * MADI_EPS21, fabsf(wx) + fabsf(wy) + fabsf(wz), g.ftol) + 7.62939453125e-6f * fabsf(m1);
-            const int nb1 = e1 <= e2 ? (e1 <= e3 ? n1 : n3) : (e2 <= e3 ? n2 : n3);
-            const float dd = m1 - cc.w;
-            if ((tag >> QREFUSE) && dd < -T && nb1 >= 0) {    // nb1 < 0: an open cell's marker, no plane
-                verdict = FACET_OUT;
-            } else if (m1 > T) {
-                verdict = dd > T ? FACET_IN : (dd < -T ? FACET_OUT : FACET_BAND);
-            } else if (m1 < -T) {
-                verdict = nb1 >= 0 ? VERDICT_MOVE + nb1 : FACET_LEFT;
-            }
-            if (sub == 0 && (verdict == FACET_IN || verdict == FACET_OUT)) {
-                const float Tm = 3.0f * T;
-                const float M = fminf(key_floor(q3) - 5.0f * T, g.L);
-                const int n = blockDim.x;
-                float4* fc = ts.fc + warp0 + ((tag >> QLANE) & 31);
-                fc[0] = p1;
-                fc[n] = p2;
-                fc[2 * n] = p3;
-                fc[3 * n] = make_float4(wx, wy, wz, M);
-                fc[4 * n] = make_float4(cc.x, cc.y, cc.z, cc.w + Tm);
-                fc[5 * n] = make_float4(cc.w - Tm, Tm, __int_as_float(sc), __int_as_float(nb1));
-            }
+            m1 = fminf(e1, fminf(e2, e3));
+            T = fmaf(2.0f * MADI_EPS21, fabsf(wx) + fabsf(wy) + fabsf(wz), g.ftol) + 7.62939453125e-6f * fabsf(m1);
+            nb1 = e1 <= e2 ? (e1 <= e3 ? n1 : n3) : (e2 <= e3 ? n2 : n3);
+            nb2 = n2;
+            // |w| to 2^-22 relative, which T covers
+            const float w2 = fmaf(wx, wx, fmaf(wy, wy, wz * wz));
+            rest = g.sorted ? h_last - w2 * rsqrtf(fmaxf(w2, 1e-30f)) - T : -3.0e38f;
+            k0 += FG * FU;
+            more = act && k0 < S && !(rest > m1 + 2.0f * T);
+        } while (__any_sync(MADI_FULL, more));
+        const float m4 = k0 < S ? fminf(key_floor(q3), rest) : key_floor(q3);
+        const float dd = m1 - cc.w;
+        int verdict = m1 > T ? (dd > T ? FACET_IN : (dd < -T ? FACET_OUT : FACET_BAND))
+                             : (m1 < -T ? (nb1 >= 0 ? VERDICT_MOVE + nb1 : FACET_LEFT) : FACET_BAND);
+        // nb1 < 0: an open cell's marker, no plane
+        if (((tag >> QREFUSE) & 1) && dd < -T && nb1 >= 0) verdict = FACET_OUT;
+        if (act && sub == 0 && (verdict == FACET_IN || verdict == FACET_OUT)) {
+            const float Tm = 3.0f * T;
+            const int n = blockDim.x;
+            float4* fc = ts.fc + warp0 + ((tag >> QLANE) & 31);
+            fc[0] = p1;
+            fc[n] = p2;
+            fc[2 * n] = p3;
+            fc[3 * n] = make_float4(wx, wy, wz, fminf(m4 - 5.0f * T, g.L));
+            fc[4 * n] = make_float4(cc.x, cc.y, cc.z, __int_as_float(nb2));
+            fc[5 * n] = make_float4(cc.w - Tm, Tm, __int_as_float(sc), __int_as_float(nb1));
         }
         // each pending walker reads its group's verdict (group = its rank among the pending)
         const int v = __shfl_sync(MADI_FULL, verdict, (mine ? rank : 0) * FG);
@@ -249,7 +252,7 @@ MADI_DEV int coop_facets(const Geo& g, const TileShared& ts, bool need, float qx
 // crossing, so a point outside that shrunk cell is as good as decided (reported
 // as outside, whatever its own label): one plane with m < alpha_c - T(q) does,
 // anywhere (t_any >= T(q)).  Otherwise `start` becomes the cell beyond the cached
-// cell's nearest facet when the point lies across it (an exact plane of it).
+// facet k1 or k2 that the point lies farther across (exact planes of the cell).
 template <bool PERIODIC>
 MADI_DEV bool cached_label(const TileShared& ts, float L, float qx, float qy, float qz, bool refuse, int cell, float t_any,
                            float a_min, int& in, int& cell_q, int& start) {
@@ -266,8 +269,9 @@ MADI_DEV bool cached_label(const TileShared& ts, float L, float qx, float qy, fl
     const float ms = fmaxf(fminf(m1, m2), fminf(fmaxf(m1, m2), m3));
     const float ux = wx - sp.x, uy = wy - sp.y, uz = wz - sp.z;
     const float d2 = fmaf(ux, ux, fmaf(uy, uy, uz * uz));
-    const bool in_c = mm > ce.w;
-    const float r = sp.w - (in_c ? ce.w : fmaxf(-mm, 0.f) + th.y);
+    const float a_up = fmaf(2.0f, th.y, th.x);           // alpha_c + Tm
+    const bool in_c = mm > a_up;
+    const float r = sp.w - (in_c ? a_up : fmaxf(-mm, 0.f) + th.y);
     const bool near = r > 0.f && d2 < r * r * (1.0f - MADI_EPS19);
     const bool out = mm < th.x && (mm >= th.y || (mm > th.y - a_min && ms + mm > 2.0f * th.y));
     const int cc = __float_as_int(th.z);
@@ -275,20 +279,22 @@ MADI_DEV bool cached_label(const TileShared& ts, float L, float qx, float qy, fl
     in = in_c ? 1 : 0;
     if (near && (in_c || out)) return true;
     if (refuse && cc == cell && mm < th.x - t_any) { in = 0; return true; }
-    const int nb1 = __float_as_int(th.w);
-    if (!refuse && m1 < -th.y && nb1 >= 0) start = nb1;
+    const int nb = __float_as_int(m1 <= m2 ? th.w : ce.w);
+    if (!refuse && fminf(m1, m2) < -th.y && nb >= 0) start = nb;
     return false;
 }
 
 // Voxel-grid rule for the lanes with `need`, one warp-cooperative pass each, the
 // fp64 rule where it cannot decide (a count in *fallbacks).  Rare (0.03 % of
-// walker-steps), so a function of its own: its registers stay out of the step loop.
-struct FullLabel { int status, seed, inside; };
+// walker-steps), so a function of its own that rebuilds its view of the geometry:
+// neither its registers nor the view's stay in the step loop.
+struct FullLabel { int status, cell, inside; };
 
-__device__ __noinline__ FullLabel full_labels(const Geo& g, bool need, float qx, float qy, float qz, int guess,
-                                              unsigned long long* fallbacks) {
+__device__ __noinline__ FullLabel full_labels(const madi_geometry* gd, const unsigned char* base, bool need, float qx,
+                                              float qy, float qz, int guess, unsigned long long* fallbacks) {
     const int lane = threadIdx.x & 31;
-    FullLabel mine{CLS_OK, 0, 0};
+    const Geo g = make_geo(*gd, base);
+    int status = CLS_OK, seed = 0, inside = 0;
     for (unsigned pend = __ballot_sync(MADI_FULL, need); pend; pend &= pend - 1) {
         const int src = __ffs(pend) - 1;
         const float sx = __shfl_sync(MADI_FULL, qx, src);
@@ -297,29 +303,31 @@ __device__ __noinline__ FullLabel full_labels(const Geo& g, bool need, float qx,
         const int sg = __shfl_sync(MADI_FULL, guess, src);
         int s1 = 0, in = 0;
         const int st = coop_classify(g, sx, sy, sz, sg, lane, s1, in);
-        if (lane == src) mine = FullLabel{st, s1, in};
+        if (lane == src) { status = st; seed = s1; inside = in; }
     }
     __syncwarp();
-    if (need && mine.status == CLS_FALLBACK) {
-        mine.status = classify_list_f64(g, qx, qy, qz, mine.seed, mine.inside);
+    if (need && status == CLS_FALLBACK) {
+        status = classify_list_f64(g, qx, qy, qz, seed, inside);
         atomicAdd(fallbacks, 1ull);
     }
-    return mine;
+    return FullLabel{status, need && status == CLS_OK ? cell_of(g, seed) : 0, inside};
 }
 
 // Empties the walker's label cache.
 MADI_DEV void clear_cache(const TileShared& ts) {
     FC(0) = FC(1) = FC(2) = make_float4(0.f, 0.f, 0.f, 3.0e38f);
     FC(3) = make_float4(0.f, 0.f, 0.f, -1.f);
-    FC(4) = make_float4(0.f, 0.f, 0.f, 0.f);
+    FC(4) = make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
     FC(5) = make_float4(0.f, 0.f, __int_as_float(-1), __int_as_float(-1));
 }
 
 // Walk one tile (blockDim.x walkers of one job) on geometry view g.
 template <int OUT, bool PERIODIC, int NP>
 __device__ __forceinline__ void walk_tile(const madi_walk_desc& d, const madi_walk_job& job,
-                                          const madi_geometry& gd, const Geo& g, int local, const TileShared& ts) {
+                                          const madi_geometry& gd, const unsigned char* base, int local,
+                                          const TileShared& ts) {
     const int lane = threadIdx.x & 31;
+    const Geo g = make_geo(gd, base);
     const bool active = local < job.n_walkers;
     const uint32_t widx = job.walker_base + (uint32_t)local;
     const float L = (float)gd.L;
@@ -365,10 +373,10 @@ __device__ __forceinline__ void walk_tile(const madi_walk_desc& d, const madi_wa
     for (int p = 0; p < NP; ++p) { AUX_M(p, 0) = 0.f; AUX_M(p, 1) = 0.f; AUX_M(p, 2) = 0.f; }
     clear_cache(ts);
     if (cells) {
-        const FullLabel f = full_labels(g, active, px, py, pz, -1, &cnt[MADI_CNT_FALLBACK64]);
+        const FullLabel f = full_labels(&gd, base, active, px, py, pz, -1, &cnt[MADI_CNT_FALLBACK64]);
         if (active) {
             if (f.status != CLS_OK) { cerr = 1; dead = true; }
-            else { cell = cell_of(g, f.seed); inside = f.inside; }
+            else { cell = f.cell; inside = f.inside; }
             ++n_full;
         }
     }
@@ -409,8 +417,11 @@ __device__ __forceinline__ void walk_tile(const madi_walk_desc& d, const madi_wa
             } else { nx = ny = nz = 0.f; }
         } else if ((step & 1) == 0) {
             const uint32_t pair = (uint32_t)step >> 1;
-            const U4 ra = philox10(U4{widx, pair, 0u, 0u}, job.key0, job.key1);
-            const U4 rb = philox10(U4{widx, pair, 1u, 0u}, job.key0, job.key1);
+            // the round keys are added up here: kept across steps they cost 20 registers
+            uint32_t k0 = job.key0, k1 = job.key1;
+            asm volatile("" : "+r"(k0), "+r"(k1));
+            const U4 ra = philox10(U4{widx, pair, 0u, 0u}, k0, k1);
+            const U4 rb = philox10(U4{widx, pair, 1u, 0u}, k0, k1);
             float g0, g1, g2;
             box_muller(ra.x, ra.y, g0, g1);
             box_muller(ra.z, ra.w, g2, g3);
@@ -460,7 +471,7 @@ __device__ __forceinline__ void walk_tile(const madi_walk_desc& d, const madi_wa
         // ---- full classifications of this step ----
         const bool need = ok && cells && !t1;
         FullLabel full{CLS_OK, 0, 0};
-        if (__any_sync(MADI_FULL, need)) full = full_labels(g, need, qx, qy, qz, cell, &cnt[MADI_CNT_FALLBACK64]);
+        if (__any_sync(MADI_FULL, need)) full = full_labels(&gd, base, need, qx, qy, qz, cell, &cnt[MADI_CNT_FALLBACK64]);
         if (ok) {
             int ncell = 0, nin = 0;
             if (t1) {
@@ -468,7 +479,7 @@ __device__ __forceinline__ void walk_tile(const madi_walk_desc& d, const madi_wa
             } else if (need) {
                 ++n_full;
                 if (full.status != CLS_OK) { cerr = 1; dead = true; }
-                else { ncell = cell_of(g, full.seed); nin = full.inside; }
+                else { ncell = full.cell; nin = full.inside; }
             }
             if (!dead) {
                 int m = 0;
@@ -656,7 +667,8 @@ __global__ void __launch_bounds__(256, MINB) walk_f32_kernel(const __grid_consta
             cur_geom = job.geom;
         }
         __syncthreads();
-        walk_tile<OUT, PERIODIC, NP>(d, job, gd, make_geo(gd, here ? stage : reinterpret_cast<const unsigned char*>(gd.stage)), local, ts);
+        walk_tile<OUT, PERIODIC, NP>(d, job, d.geoms[job.geom], here ? stage : reinterpret_cast<const unsigned char*>(gd.stage),
+                                     local, ts);
         __syncthreads();
         if (OUT == MADI_OUT_FUSED) {
             long long* out = reinterpret_cast<long long*>(d.accum) + (size_t)job.slot * 2 * n_out;

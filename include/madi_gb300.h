@@ -97,7 +97,9 @@ typedef struct madi_geometry {
     uint32_t off_facet_plane;      /* float4 [n_cells][facet_stride]: n, offset h */
     uint32_t off_facet_nbr;        /* int32 [n_cells][facet_stride]: cell across  */
     int32_t  n_cells;              /* cells in the table (0 = no table)           */
-    float    alpha_min;            /* <= every cell's alpha (0: not known)        */
+    float    alpha_min;            /* > 0: <= every cell's alpha, and each cell's slots
+                                    * are in ascending order of h (as madi_facets_build
+                                    * writes them); 0: neither is promised           */
     double   facet_tol;            /* fp32 error of h - n.w, without the |w| term */
 } madi_geometry;
 
