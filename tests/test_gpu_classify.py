@@ -75,3 +75,28 @@ def test_classify_random_stream_vs_oracle_large():
     oc, oi = O.classify_kd(O.geom_arrays(ens), pts)
     assert np.array_equal(i, oi) and np.array_equal(c, oc)
     assert np.mean(path == 1) < 0.01
+
+
+@pytest.mark.parametrize("mode, n_cells, rho, V", [("periodic", 2, 2.0e5, 4.0), ("periodic", 300, 5.0e7, 0.017),
+                                                   ("si_fatal_escape", 0, 1.0e5, 7.0)])
+def test_fp64_points_in_fp32_band(mode, n_cells, rho, V):
+    """fp64 points decided in fp32 where the band allows: the labels of the KD rule,
+    also on and within rounding of shifted facets, seeds and box faces."""
+    from custom_madi_gb300.config import SimConfig
+    from custom_madi_gb300.ensemble import create_ensemble
+    over = dict(boundary_mode="periodic", n_cells=n_cells) if mode == "periodic" else {}
+    cfg = SimConfig(n_ensembles=1, ts=0.01, T_max_ms=4.0, small_deltas=[1.0], big_deltas=[2.0], b_values=[0.0, 1000.0], **over)
+    ens = create_ensemble(rho, V, cfg, seed=9, verify_vi=False, measure_vi=False)
+    rng = np.random.default_rng(4)
+    p = rng.uniform(0.0, ens.L, size=(20_000, 3))
+    cs = ens.classifier_seeds if ens.classifier_seeds is not None else ens.seeds
+    an = ens.classifier_annulus if ens.classifier_annulus is not None else ens.annulus
+    i, j = rng.integers(0, len(cs), 5_000), rng.integers(0, len(cs), 5_000)
+    u = cs[j] - cs[i]
+    d = np.maximum(np.linalg.norm(u, axis=1, keepdims=True), 1e-12)
+    on = cs[i] + u * (0.5 - an[i][:, None] / d)                       # on the shifted facet of (i, j)
+    near = on + 10.0 ** rng.uniform(-13, -4, (len(on), 1)) * rng.standard_normal(on.shape)
+    q = np.concatenate([p, on, near, cs[i], np.where(rng.random(p.shape) < 0.3, 0.0, p)])
+    q = q[np.all((q >= 0.0) & (q < ens.L), axis=1)]
+    a, b = ens.classify(q, method="grid"), ens.classify(q, method="kd")
+    assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
