@@ -15,9 +15,9 @@
 //           recomputed from the direct difference and is the shift S (the
 //           reference shifts by the minimum residual or the maximum log-weight;
 //           any shift gives the same normalised weights).
-//   pass 2: entries whose screened e_j (with its fp32 error bound) is above
-//           S - CUT get the direct-difference residual (error ~F ulp of the
-//           residual itself, which is small where weights matter) and add
+//   pass 2: entries that can be above S - CUT get the direct-difference residual
+//           (error ~F ulp of the residual itself, which is small where weights
+//           matter); those that are above it add
 //           w = exp(e_j - S) to Kahan-compensated fp32 sums of w, w d, w d^2
 //           (d = parameter minus that of j*, so narrow posteriors keep their
 //           variance), w r, w^2 and w s0.  Entries below the cut weigh less
@@ -32,7 +32,8 @@
 //     voxels in the index's embedding and only visits those that can matter;
 //   - d is formed in pairs of floats (48 bits), then rounded to fp32 as before.
 // The entries a voxel sums, and their order, are unchanged.  100,000 voxels x
-// 20,000 entries x 20 features, sigma_m 0.02: 33.2 ms before, @@BAYES@@.
+// 20,000 entries x 20 features, sigma_m 0.02: 33.2 ms before, 6.8 ms now (5.6 ms of it this
+// kernel, bound by issue; the rest is host copies).
 #include <cstdint>
 #include "madi_device.cuh"
 #include "madi_host.h"
@@ -44,16 +45,19 @@ namespace bayes {
 constexpr int CHUNK = 128;           // entries staged at a time
 constexpr float CUT = 60.f;          // exp(-60) ~ 9e-27 of the shift entry's weight
 
-struct Kahan {
-    float s = 0.f, c = 0.f;
-    MADI_DEV void add(float x) {
-        const float y = x - c;
-        const float t = s + y;
-        c = (t - s) - y;
+// Two compensated sums of products in packed registers.  y = a b - c is one fused
+// operation; c is kept negated.
+struct Kahan2 {
+    uint64_t s = 0, nc = 0;
+    MADI_DEV void add(uint64_t a, uint64_t b) {
+        const uint64_t y = fma2(a, b, nc);
+        const uint64_t t = add2(s, y);
+        nc = sub2(y, sub2(t, s));
         s = t;
     }
-    MADI_DEV void scale(float f) { s *= f; c *= f; }
-    MADI_DEV double value() const { return (double)s - (double)c; }
+    MADI_DEV void scale(uint64_t f) { s = mul2(s, f); nc = mul2(nc, f); }
+    MADI_DEV double lo() const { return (double)split2(s).x + (double)split2(nc).x; }
+    MADI_DEV double hi() const { return (double)split2(s).y + (double)split2(nc).y; }
 };
 
 struct Plan {
@@ -73,7 +77,7 @@ struct Plan {
 };
 
 // One entry in shared memory: centred (fixed S0) or raw (free S0) row, raw row,
-// then |row|^2, log q, and kio, rho, V as pairs of floats.
+// then |row|^2, log q, and kio, rho, V as hi + lo: (kio, rho) hi, (kio, rho) lo, V.
 template <int N>
 struct Entry {
     static constexpr int RAW = N, AUX = 2 * N, FLOATS = 2 * N + 8;
@@ -85,12 +89,12 @@ MADI_DEV float2 pair_of(double x) {
     return make_float2(h, isfinite(h) ? (float)(x - (double)h) : 0.f);
 }
 
-// a - b of two pairs, rounded to fp32.
-MADI_DEV float pair_diff(float ah, float al, float2 b) {
-    const float s = ah - b.x;
-    const float t = s - ah;
-    const float e = (ah - (s - t)) - (b.x + t);              // exact error of s
-    return s + (e + (al - b.y));
+// Differences ah + al - (bh + bl) of two values at a time, rounded to fp32.
+MADI_DEV uint64_t pair_diff(uint64_t ah, uint64_t al, uint64_t bh, uint64_t bl) {
+    const uint64_t s = sub2(ah, bh);
+    const uint64_t t = sub2(s, ah);
+    const uint64_t e = sub2(sub2(ah, sub2(s, t)), add2(bh, t));      // exact error of s
+    return add2(s, add2(e, sub2(al, bl)));
 }
 
 // Screened log-weight of one entry from the fp32 score, and its error bound.
@@ -143,6 +147,25 @@ MADI_DEV bool exact(const float* mr, const float* L, int F, float& resid, float&
     return true;
 }
 
+// The same for a row of the staged form (zero padded; fixed S0 two differences at
+// a time, summed in the same order).
+template <int N, bool FREE>
+MADI_DEV bool exact_staged(const float* mr, const uint64_t* mr2, const float* L, int F, float& resid, float& rw, float& s0) {
+    if (FREE) return exact<N, true>(mr, L, F, resid, rw, s0);
+    s0 = 1.f;
+    float r = 0.f;
+    const ulonglong2* L2 = reinterpret_cast<const ulonglong2*>(L);
+#pragma unroll
+    for (int f = 0; f < N / 4; ++f) {
+        const ulonglong2 l = L2[f];
+        const float2 a = split2(sub2(mr2[2 * f], l.x)), b = split2(sub2(mr2[2 * f + 1], l.y));
+        r = fmaf(a.x, a.x, r); r = fmaf(a.y, a.y, r);
+        r = fmaf(b.x, b.x, r); r = fmaf(b.y, b.y, r);
+    }
+    resid = rw = r;
+    return true;
+}
+
 // Entry e of the library in the staged form.
 template <int N, bool FREE>
 MADI_DEV void make_entry(const Plan& P, int64_t e, const float* smu, float* o) {
@@ -158,7 +181,7 @@ MADI_DEV void make_entry(const Plan& P, int64_t e, const float* smu, float* o) {
     a[0] = FREE ? fmaxf(sn, 1e-30f) : sn;
     a[1] = (float)P.logq[e];
     const float2 k = pair_of(P.kio[e]), r = pair_of(P.rho[e]), v = pair_of(P.V[e]);
-    a[2] = k.x; a[3] = k.y; a[4] = r.x; a[5] = r.y; a[6] = v.x; a[7] = v.y;
+    a[2] = k.x; a[3] = r.x; a[4] = k.y; a[5] = r.y; a[6] = v.x; a[7] = v.y;
 }
 
 // The library in the staged form, and (|row|^2, log q) beside its embedding.
@@ -319,7 +342,7 @@ __global__ void __launch_bounds__(THREADS) bayes_kernel(const __grid_constant__ 
     // shift and centre from the exact residual of j*
     float S = 0.f;
     double x0[3] = {0.0, 0.0, 0.0};
-    float2 xp[3] = {};
+    uint64_t xh = 0, xl = 0, xv = 0, xvl = 0;                // (kio, rho) and V of j* as hi, lo
     bool any = bj >= 0;
     if (any) {
         float Lj[N];
@@ -331,11 +354,20 @@ __global__ void __launch_bounds__(THREADS) bayes_kernel(const __grid_constant__ 
         x0[0] = P.kio[bj];
         x0[1] = P.rho[bj];
         x0[2] = P.V[bj];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) xp[k] = pair_of(x0[k]);
+        const float2 k = pair_of(x0[0]), r = pair_of(x0[1]), v3 = pair_of(x0[2]);
+        xh = pair2(k.x, r.x);
+        xl = pair2(k.y, r.y);
+        xv = pair2(v3.x, 0.f);
+        xvl = pair2(v3.y, 0.f);
     }
     // ---- pass 2: exp-weighted sums over the entries above the cut ----
-    Kahan W, W2, R, S0, d1[3], d2[3];
+    // Sums in pairs: (w, w^2), (w resid, w s0), (w d_kio, w d_rho), (w d_V, w d_V^2),
+    // (w d_kio^2, w d_rho^2).  Entries the sweep visits go to the exact residual at
+    // once: most pass, and the cut on the exact log-weight is the one that counts.
+    Kahan2 WW, RS, D1, DV, D2;
+    uint64_t mr2[N / 2];
+#pragma unroll
+    for (int f = 0; f < N / 2; ++f) mr2[f] = pair2(mr[2 * f], mr[2 * f + 1]);
     sweep([&]() {
               // entries below S - CUT of every voxel; a voxel without any entry sums none
               const float s = warp_minf(any ? S : 3.0e38f);
@@ -343,52 +375,52 @@ __global__ void __launch_bounds__(THREADS) bayes_kernel(const __grid_constant__ 
           },
           [&](int, const float* o) {
               const float* a = o + Entry<N>::AUX;
-              float ee, err;
-              screen<N, FERR, FREE>(m, o, a[0], a[1], m2, P.inv2s2, ee, err);
-              if (!any || !(ee + err - S > -CUT)) return;
               float resid, rw, s0;
-              if (!exact<N, FREE>(mr, o + Entry<N>::RAW, F, resid, rw, s0)) return;
-              float x = a[1] - rw * P.inv2s2 - S;
+              const bool fits = any && exact_staged<N, FREE>(mr, mr2, o + Entry<N>::RAW, F, resid, rw, s0);
+              float x = fits ? a[1] - rw * P.inv2s2 - S : -3.0e38f;
               if (!(x > -CUT)) return;
               if (x > 0.f) {
                   // an entry above the screened maximum (within the screen's error):
                   // move the shift to it so that every weight stays <= 1
                   const float f = expf(-x);
-                  W.scale(f);
-                  W2.scale(f * f);
-                  R.scale(f);
-                  S0.scale(f);
-#pragma unroll
-                  for (int k = 0; k < 3; ++k) { d1[k].scale(f); d2[k].scale(f); }
+                  const uint64_t ff = pair2(f, f);
+                  WW.scale(pair2(f, f * f));
+                  RS.scale(ff);
+                  D1.scale(ff);
+                  DV.scale(ff);
+                  D2.scale(ff);
                   S += x;
                   x = 0.f;
               }
               const float w = expf(x);
-              W.add(w);
-              W2.add(w * w);
-              R.add(w * resid);
-              if (FREE) S0.add(w * s0);
-#pragma unroll
-              for (int k = 0; k < 3; ++k) {
-                  const float d = pair_diff(a[2 + 2 * k], a[3 + 2 * k], xp[k]);
-                  d1[k].add(w * d);
-                  d2[k].add(w * d * d);
-              }
+              const uint64_t ww = pair2(w, w);
+              const ulonglong2 kr = *reinterpret_cast<const ulonglong2*>(a + 4);     // (kio, rho) lo, V hi / lo
+              const uint64_t d = pair_diff(*reinterpret_cast<const uint64_t*>(a + 2), kr.x, xh, xl);
+              const float2 v3 = split2(kr.y);
+              const float dv = split2(pair_diff(pair2(v3.x, 0.f), pair2(v3.y, 0.f), xv, xvl)).x;
+              WW.add(ww, pair2(1.f, w));
+              RS.add(ww, pair2(resid, FREE ? s0 : 0.f));
+              const uint64_t wd = mul2(ww, d);             // rounded: it serves both sums
+              const float wdv = w * dv;
+              D1.add(wd, pair2(1.f, 1.f));
+              D2.add(wd, d);
+              DV.add(pair2(wdv, wdv), pair2(1.f, dv));
           });
     if (!live) return;
     const int64_t n = P.n_vox;
     double* o = P.out;
-    const double Wv = any ? W.value() : 0.0;
+    const double Wv = any ? WW.lo() : 0.0;
     const double Wd = fmax(Wv, 1e-300);
+    const double s1[3] = {D1.lo(), D1.hi(), DV.lo()}, s2[3] = {D2.lo(), D2.hi(), DV.hi()};
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        const double a = d1[k].value() / Wd, b = d2[k].value() / Wd;
+        const double a = s1[k] / Wd, b = s2[k] / Wd;
         o[(int64_t)k * n + v] = Wv > 0.0 ? x0[k] + a : 0.0;                      // kio, rho, V means
         o[(int64_t)(3 + k) * n + v] = Wv > 0.0 ? sqrt(fmax(b - a * a, 0.0)) : 0.0; // their std
     }
-    o[6 * n + v] = Wv > 0.0 ? R.value() / Wd : 0.0;
-    o[7 * n + v] = Wv > 0.0 ? Wv * Wv / fmax(W2.value(), 1e-300) : 0.0;
-    o[8 * n + v] = (FREE && Wv > 0.0) ? S0.value() / Wd : 0.0;
+    o[6 * n + v] = Wv > 0.0 ? RS.lo() / Wd : 0.0;
+    o[7 * n + v] = Wv > 0.0 ? Wv * Wv / fmax(WW.hi(), 1e-300) : 0.0;
+    o[8 * n + v] = (FREE && Wv > 0.0) ? RS.hi() / Wd : 0.0;
 }
 
 template <int N, bool FREE, int THREADS, bool INDEXED>

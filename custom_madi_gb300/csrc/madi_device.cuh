@@ -43,6 +43,37 @@ MADI_DEV void box_muller(uint32_t a, uint32_t b, float& g0, float& g1) {
     g1 = r * s;
 }
 
+// Pairs of fp32 values in one 64-bit register and the packed operations on them,
+// each half rounded as the scalar operation.
+MADI_DEV uint64_t pair2(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+MADI_DEV float2 split2(uint64_t v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+MADI_DEV uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+MADI_DEV uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+MADI_DEV uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+MADI_DEV uint64_t sub2(uint64_t a, uint64_t b) {          // a - b: the product with -1 is exact
+    return fma2(b, 0xBF800000BF800000ull, a);
+}
+
 // ---------------------------------------------------------------------------
 // Geometry view.  `base` is either shared memory (staged) or the global stage
 // buffer; both carry the layout of madi_geometry (include/madi_gb300.h).

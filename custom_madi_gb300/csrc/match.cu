@@ -223,23 +223,6 @@ MADI_DEV float box_distance2(const float4* __restrict__ b, const float (&lo)[6],
     return d2;
 }
 
-// Two fp32 fused multiply-adds in one instruction, each rounded as fmaf().
-MADI_DEV uint64_t pair2(float lo, float hi) {
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-MADI_DEV float2 split2(uint64_t v) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-MADI_DEV uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-
 // Scores a tile for the two voxels of every lane.  Rows come in pairs of entries,
 // feature by feature, so one packed instruction advances both entries' dot
 // products (m holds each feature twice).
