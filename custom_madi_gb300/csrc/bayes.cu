@@ -147,23 +147,35 @@ MADI_DEV bool exact(const float* mr, const float* L, int F, float& resid, float&
     return true;
 }
 
-// The same for a row of the staged form (zero padded; fixed S0 two differences at
-// a time, summed in the same order).
+// The same for an entry of the staged form (zero padded rows; |L|^2 as staged),
+// two differences at a time, summed in the same order.
 template <int N, bool FREE>
-MADI_DEV bool exact_staged(const float* mr, const uint64_t* mr2, const float* L, int F, float& resid, float& rw, float& s0) {
-    if (FREE) return exact<N, true>(mr, L, F, resid, rw, s0);
+MADI_DEV bool exact_staged(const float* mr, const uint64_t* mr2, const float* o, float& resid, float& rw, float& s0) {
+    const ulonglong2* L2 = reinterpret_cast<const ulonglong2*>(o + Entry<N>::RAW);
+    float dot = 0.f;
     s0 = 1.f;
+    if (FREE) {
+        const float4* L = reinterpret_cast<const float4*>(o + Entry<N>::RAW);
+#pragma unroll
+        for (int f = 0; f < N / 4; ++f) {
+            const float4 l = L[f];
+            dot = fmaf(mr[4 * f], l.x, dot); dot = fmaf(mr[4 * f + 1], l.y, dot);
+            dot = fmaf(mr[4 * f + 2], l.z, dot); dot = fmaf(mr[4 * f + 3], l.w, dot);
+        }
+        s0 = dot / o[Entry<N>::AUX];
+    }
+    const uint64_t ms0 = pair2(-s0, -s0);
     float r = 0.f;
-    const ulonglong2* L2 = reinterpret_cast<const ulonglong2*>(L);
 #pragma unroll
     for (int f = 0; f < N / 4; ++f) {
         const ulonglong2 l = L2[f];
-        const float2 a = split2(sub2(mr2[2 * f], l.x)), b = split2(sub2(mr2[2 * f + 1], l.y));
+        const float2 a = split2(fma2(l.x, ms0, mr2[2 * f])), b = split2(fma2(l.y, ms0, mr2[2 * f + 1]));
         r = fmaf(a.x, a.x, r); r = fmaf(a.y, a.y, r);
         r = fmaf(b.x, b.x, r); r = fmaf(b.y, b.y, r);
     }
-    resid = rw = r;
-    return true;
+    resid = r;
+    rw = FREE ? r / (s0 * s0) : r;
+    return !FREE || dot > 0.f;
 }
 
 // Entry e of the library in the staged form.
@@ -260,8 +272,8 @@ __global__ void __launch_bounds__(THREADS) bayes_kernel(const __grid_constant__ 
         // screen error (F + 8) 2^-21 (|m|^2 + |L|^2) twice, and the bound added to it
         e_max = warp_maxf_bits((float)(FERR + 8) * 2e-6f * (m2 + lmax));
     }
-    // Visits, in index order, the entries that may reach `floor` (a log-weight) for
-    // some voxel of the warp; visit(e, entry) runs warp-wide.
+    // Visits, in index order and by twos, the entries that may reach `floor` (a
+    // log-weight) for some voxel of the warp; visit runs warp-wide.
     auto sweep = [&](auto floor, auto visit) {
         for (int base = 0; base < P.n_lib; base += CHUNK) {
             const int cnt = min(CHUNK, P.n_lib - base);
@@ -299,9 +311,14 @@ __global__ void __launch_bounds__(THREADS) bayes_kernel(const __grid_constant__ 
             if (THREADS > 32) __syncthreads(); else __syncwarp();
 #pragma unroll
             for (int i = 0; i < CHUNK / 32; ++i)
-                for (unsigned w = mask[i]; w; w &= w - 1) {
-                    const int k = 32 * i + __ffs(w) - 1;
-                    visit(base + k, sent + k * EF);
+                for (unsigned w = mask[i]; w;) {
+                    // two entries at a time: their residuals are independent chains
+                    const int k0 = 32 * i + __ffs(w) - 1;
+                    w &= w - 1;
+                    const bool two = w != 0u;
+                    const int k1 = two ? 32 * i + __ffs(w) - 1 : k0;
+                    w &= w - 1;
+                    visit(base + k0, sent + k0 * EF, base + k1, sent + k1 * EF, two);
                 }
             if (THREADS > 32) __syncthreads(); else __syncwarp();
         }
@@ -334,10 +351,12 @@ __global__ void __launch_bounds__(THREADS) bayes_kernel(const __grid_constant__ 
         screen<N, FERR, FREE>(m, o, o[Entry<N>::AUX], o[Entry<N>::AUX + 1], m2, P.inv2s2, known, err);
     }
     sweep([&]() { return warp_minf(fmaxf(best, known)); },
-          [&](int e, const float* o) {
-              float ee, err;
-              screen<N, FERR, FREE>(m, o, o[Entry<N>::AUX], o[Entry<N>::AUX + 1], m2, P.inv2s2, ee, err);
-              if (ee > best) { best = ee; bj = e; }
+          [&](int e0, const float* o0, int e1, const float* o1, bool two) {
+              float ee0, ee1, err;
+              screen<N, FERR, FREE>(m, o0, o0[Entry<N>::AUX], o0[Entry<N>::AUX + 1], m2, P.inv2s2, ee0, err);
+              screen<N, FERR, FREE>(m, o1, o1[Entry<N>::AUX], o1[Entry<N>::AUX + 1], m2, P.inv2s2, ee1, err);
+              if (ee0 > best) { best = ee0; bj = e0; }
+              if (two && ee1 > best) { best = ee1; bj = e1; }
           });
     // shift and centre from the exact residual of j*
     float S = 0.f;
@@ -373,38 +392,42 @@ __global__ void __launch_bounds__(THREADS) bayes_kernel(const __grid_constant__ 
               const float s = warp_minf(any ? S : 3.0e38f);
               return s - CUT - 1e-5f * fabsf(s);
           },
-          [&](int, const float* o) {
-              const float* a = o + Entry<N>::AUX;
-              float resid, rw, s0;
-              const bool fits = any && exact_staged<N, FREE>(mr, mr2, o + Entry<N>::RAW, F, resid, rw, s0);
-              float x = fits ? a[1] - rw * P.inv2s2 - S : -3.0e38f;
-              if (!(x > -CUT)) return;
-              if (x > 0.f) {
-                  // an entry above the screened maximum (within the screen's error):
-                  // move the shift to it so that every weight stays <= 1
-                  const float f = expf(-x);
-                  const uint64_t ff = pair2(f, f);
-                  WW.scale(pair2(f, f * f));
-                  RS.scale(ff);
-                  D1.scale(ff);
-                  DV.scale(ff);
-                  D2.scale(ff);
-                  S += x;
-                  x = 0.f;
-              }
-              const float w = expf(x);
-              const uint64_t ww = pair2(w, w);
-              const ulonglong2 kr = *reinterpret_cast<const ulonglong2*>(a + 4);     // (kio, rho) lo, V hi / lo
-              const uint64_t d = pair_diff(*reinterpret_cast<const uint64_t*>(a + 2), kr.x, xh, xl);
-              const float2 v3 = split2(kr.y);
-              const float dv = split2(pair_diff(pair2(v3.x, 0.f), pair2(v3.y, 0.f), xv, xvl)).x;
-              WW.add(ww, pair2(1.f, w));
-              RS.add(ww, pair2(resid, FREE ? s0 : 0.f));
-              const uint64_t wd = mul2(ww, d);             // rounded: it serves both sums
-              const float wdv = w * dv;
-              D1.add(wd, pair2(1.f, 1.f));
-              D2.add(wd, d);
-              DV.add(pair2(wdv, wdv), pair2(1.f, dv));
+          [&](int, const float* o0, int, const float* o1, bool two) {
+              float resid0, rw0, s00, resid1, rw1, s01;
+              const bool fits0 = exact_staged<N, FREE>(mr, mr2, o0, resid0, rw0, s00) && any;
+              const bool fits1 = exact_staged<N, FREE>(mr, mr2, o1, resid1, rw1, s01) && any && two;
+              auto add = [&](const float* a, float resid, float rw, float s0) {
+                  float x = a[1] - rw * P.inv2s2 - S;
+                  if (!(x > -CUT)) return;
+                  if (x > 0.f) {
+                      // an entry above the screened maximum (within the screen's error):
+                      // move the shift to it so that every weight stays <= 1
+                      const float f = expf(-x);
+                      const uint64_t ff = pair2(f, f);
+                      WW.scale(pair2(f, f * f));
+                      RS.scale(ff);
+                      D1.scale(ff);
+                      DV.scale(ff);
+                      D2.scale(ff);
+                      S += x;
+                      x = 0.f;
+                  }
+                  const float w = expf(x);
+                  const uint64_t ww = pair2(w, w);
+                  const ulonglong2 kr = *reinterpret_cast<const ulonglong2*>(a + 4);     // (kio, rho) lo, V hi / lo
+                  const uint64_t d = pair_diff(*reinterpret_cast<const uint64_t*>(a + 2), kr.x, xh, xl);
+                  const float2 v3 = split2(kr.y);
+                  const float dv = split2(pair_diff(pair2(v3.x, 0.f), pair2(v3.y, 0.f), xv, xvl)).x;
+                  WW.add(ww, pair2(1.f, w));
+                  RS.add(ww, pair2(resid, FREE ? s0 : 0.f));
+                  const uint64_t wd = mul2(ww, d);             // rounded: it serves both sums
+                  const float wdv = w * dv;
+                  D1.add(wd, pair2(1.f, 1.f));
+                  D2.add(wd, d);
+                  DV.add(pair2(wdv, wdv), pair2(1.f, dv));
+              };
+              if (fits0) add(o0 + Entry<N>::AUX, resid0, rw0, s00);
+              if (fits1) add(o1 + Entry<N>::AUX, resid1, rw1, s01);
           });
     if (!live) return;
     const int64_t n = P.n_vox;
