@@ -321,14 +321,30 @@ MADI_DEV void clear_cache(const TileShared& ts) {
     FC(5) = make_float4(0.f, 0.f, __int_as_float(-1), __int_as_float(-1));
 }
 
-// Walk one tile (blockDim.x walkers of one job) on geometry view g.
-template <int OUT, bool PERIODIC, int NP>
+// The six normals of a step pair (the even step's first) and both acceptance words.
+MADI_DEV void draw_pair(uint32_t widx, uint32_t pair, const madi_walk_job& job, float (&gv)[6], uint32_t& even, uint32_t& odd) {
+    // the round keys are added up here: kept across steps they cost 20 registers
+    uint32_t k0 = job.key0, k1 = job.key1;
+    asm volatile("" : "+r"(k0), "+r"(k1));
+    const U4 ra = philox10(U4{widx, pair, 0u, 0u}, k0, k1);
+    const U4 rb = philox10(U4{widx, pair, 1u, 0u}, k0, k1);
+    box_muller(ra.x, ra.y, gv[0], gv[1]);
+    box_muller(ra.z, ra.w, gv[2], gv[3]);
+    box_muller(rb.x, rb.y, gv[4], gv[5]);
+    even = rb.z;
+    odd = rb.w;
+}
+
+// Walk blockDim.x >> spread walkers of one job on geometry view g: 32 >> spread of
+// them in the first lanes of each warp.  `local` is the lane's walker; lane groups
+// beyond the first (SPREAD) hold the same walkers' numbers and no walker.
+template <int OUT, bool PERIODIC, int NP, bool SPREAD>
 __device__ __forceinline__ void walk_tile(const madi_walk_desc& d, const madi_walk_job& job,
-                                          const madi_geometry& gd, const unsigned char* base, int local,
+                                          const madi_geometry& gd, const unsigned char* base, int local, int spread,
                                           const TileShared& ts) {
     const int lane = threadIdx.x & 31;
     const Geo g = make_geo(gd, base);
-    const bool active = local < job.n_walkers;
+    const bool active = local < job.n_walkers && (!SPREAD || lane < (32 >> spread));
     const uint32_t widx = job.walker_base + (uint32_t)local;
     const float L = (float)gd.L;
     const float sigma = (float)d.sigma;
@@ -397,8 +413,8 @@ __device__ __forceinline__ void walk_tile(const madi_walk_desc& d, const madi_wa
     // error bound of any facet margin in the box (|w|_1 <= 3 L)
     const float t_any = fmaf(6.0f * MADI_EPS21, L, (float)gd.facet_tol);
     const float a_min = gd.alpha_min;
-    float g3 = 0.f, g4 = 0.f, g5 = 0.f;
-    uint32_t acc_word_odd = 0;
+    float gv[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    uint32_t acc_word = 0, acc_word_odd = 0;
     int h_left = d.steps_per_h;
     int jgrid = 0;
 #pragma unroll 1
@@ -415,22 +431,21 @@ __device__ __forceinline__ void walk_tile(const madi_walk_desc& d, const madi_wa
                 nz = (float)d.incr[3 * o + 2];
                 ustream = d.unif[o];
             } else { nx = ny = nz = 0.f; }
+        } else if (SPREAD) {
+            // lane group i draws step pair i of 1 << spread pairs; each step reads its pair's
+            if ((step & ((2 << spread) - 1)) == 0)
+                draw_pair(widx, ((uint32_t)step >> 1) + ((uint32_t)lane >> (5 - spread)), job, gv, acc_word, acc_word_odd);
+            const int from = (lane & (31 >> spread)) | (((step >> 1) & ((1 << spread) - 1)) << (5 - spread));
+            const bool odd = step & 1;
+            nx = __shfl_sync(MADI_FULL, odd ? gv[3] : gv[0], from) * sigma;
+            ny = __shfl_sync(MADI_FULL, odd ? gv[4] : gv[1], from) * sigma;
+            nz = __shfl_sync(MADI_FULL, odd ? gv[5] : gv[2], from) * sigma;
+            word = __shfl_sync(MADI_FULL, odd ? acc_word_odd : acc_word, from);
         } else if ((step & 1) == 0) {
-            const uint32_t pair = (uint32_t)step >> 1;
-            // the round keys are added up here: kept across steps they cost 20 registers
-            uint32_t k0 = job.key0, k1 = job.key1;
-            asm volatile("" : "+r"(k0), "+r"(k1));
-            const U4 ra = philox10(U4{widx, pair, 0u, 0u}, k0, k1);
-            const U4 rb = philox10(U4{widx, pair, 1u, 0u}, k0, k1);
-            float g0, g1, g2;
-            box_muller(ra.x, ra.y, g0, g1);
-            box_muller(ra.z, ra.w, g2, g3);
-            box_muller(rb.x, rb.y, g4, g5);
-            nx = g0 * sigma; ny = g1 * sigma; nz = g2 * sigma;
-            word = rb.z;
-            acc_word_odd = rb.w;
+            draw_pair(widx, (uint32_t)step >> 1, job, gv, word, acc_word_odd);
+            nx = gv[0] * sigma; ny = gv[1] * sigma; nz = gv[2] * sigma;
         } else {
-            nx = g3 * sigma; ny = g4 * sigma; nz = g5 * sigma;
+            nx = gv[3] * sigma; ny = gv[4] * sigma; nz = gv[5] * sigma;
             word = acc_word_odd;
         }
         // ---- proposal and boundary ----
@@ -561,11 +576,23 @@ __device__ __forceinline__ void walk_tile(const madi_walk_desc& d, const madi_wa
     }
     // ---- phase epilogue: per (pair, dir, b) warp sums -> fixed point ----
     if (OUT == MADI_OUT_FUSED) {
-        const bool live = active && !escaped && !cerr;
+        bool live = active && !escaped && !cerr;
+        int from = threadIdx.x;
+        bool mine = true;
+        if (SPREAD) {
+            // the sums are those of the launch without lane groups: 32 walkers to a warp again
+            FC(0).x = live ? 1.f : 0.f;
+            __syncthreads();
+            const int per = 5 - spread;
+            mine = from < (int)(blockDim.x >> spread);
+            from = ((from >> per) << 5) | (from & ((1 << per) - 1));
+            if (mine) live = ts.fc[from].x != 0.f;
+        }
 #pragma unroll
         for (int p = 0; p < NP; ++p) {
-            if (p >= d.n_pairs) break;
-            const float mx = AUX_M(p, 0), my = AUX_M(p, 1), mz = AUX_M(p, 2);
+            if (p >= d.n_pairs || !mine) break;
+            const float* m = &ts.auxf[(3 + 3 * p) * blockDim.x + from];
+            const float mx = m[0], my = m[blockDim.x], mz = m[2 * blockDim.x];
             for (int u = 0; u < d.n_dirs; ++u) {
                 const float proj = fmaf(d.dirs[3 * u], mx, fmaf(d.dirs[3 * u + 1], my, d.dirs[3 * u + 2] * mz));
                 for (int bb = 0; bb < d.n_b; ++bb) {
@@ -610,13 +637,18 @@ __device__ __forceinline__ void walk_tile(const madi_walk_desc& d, const madi_wa
     }
 }
 
-template <int OUT, bool PERIODIC, int NP, int MINB>
-__global__ void __launch_bounds__(256, MINB) walk_f32_kernel(const __grid_constant__ madi_walk_desc d) {
+constexpr int SPREAD_THREADS = 128;
+
+template <int OUT, bool PERIODIC, int NP, int MINB, bool SPREAD>
+__global__ void __launch_bounds__(SPREAD ? SPREAD_THREADS : 256, MINB) walk_f32_kernel(const __grid_constant__ madi_walk_desc d, int spread) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int s_item;
     const int nthr = blockDim.x;
     const int tid = threadIdx.x;
     const int n_out = d.n_pairs * d.n_b * d.n_dirs;
+    if (!SPREAD) spread = 0;
+    const int parts = SPREAD ? (d.tile_walkers << spread) / SPREAD_THREADS : 1;      // CTAs' shares of a tile
+    const int n_items = d.n_tiles * parts;
     // Dynamic shared memory: [stage][acc int64 x 2 n_out][occ u32 x n_grid][snap x n_grid]
     unsigned char* stage = smem;
     TileShared ts;
@@ -629,7 +661,7 @@ __global__ void __launch_bounds__(256, MINB) walk_f32_kernel(const __grid_consta
     ts.fc = reinterpret_cast<float4*>(aux + 24 * nthr);
     ts.auxf = reinterpret_cast<float*>(aux + (24 + FC_BYTES_PER_WALKER) * nthr);
     ts.auxc = reinterpret_cast<uint32_t*>(ts.auxf + (3 + 3 * NP) * nthr);
-    ts.queue = reinterpret_cast<float4*>(ts.auxc + 2 * nthr);    // 2 of the 4 bytes a walker left of the 12
+    ts.queue = reinterpret_cast<float4*>(ts.auxc + 2 * nthr);    // the 4 bytes a walker left of the 12
 
     for (int j = tid; j < d.n_grid; j += nthr) {
         uint32_t code = 0, any = 0;
@@ -647,18 +679,20 @@ __global__ void __launch_bounds__(256, MINB) walk_f32_kernel(const __grid_consta
         __syncthreads();
         if (tid == 0) {
             if (d.grid_blocks > 0) s_item = (int)atomicAdd(d.work_counter, 1u);
-            else s_item = first ? (int)blockIdx.x : d.n_tiles;
+            else s_item = first ? (int)blockIdx.x : n_items;
         }
         first = 0;
         for (int i = tid; i < 2 * n_out; i += nthr) ts.acc[i] = 0;
         for (int j = tid; j < d.n_grid; j += nthr) ts.occ[j] = 0;
         __syncthreads();
         const int item = s_item;
-        if (item >= d.n_tiles) break;
-        const int jn = find_job(d.jobs, d.n_jobs, item);
+        if (item >= n_items) break;
+        const int tile = item / parts;
+        const int jn = find_job(d.jobs, d.n_jobs, tile);
         const madi_walk_job job = d.jobs[jn];
         const madi_geometry gd = d.geoms[job.geom];
-        const int local = (item - job.tile_begin) * nthr + tid;
+        const int local = SPREAD ? (((item - job.tile_begin * parts) * nthr + (tid & ~31)) >> spread) + (tid & (31 >> spread))
+                                 : (tile - job.tile_begin) * nthr + tid;
         const bool here = d.stage_smem > 0 && (int)gd.stage_bytes <= d.stage_smem;
         if (here && job.geom != cur_geom) {
             const uint4* src = reinterpret_cast<const uint4*>(gd.stage);
@@ -667,8 +701,8 @@ __global__ void __launch_bounds__(256, MINB) walk_f32_kernel(const __grid_consta
             cur_geom = job.geom;
         }
         __syncthreads();
-        walk_tile<OUT, PERIODIC, NP>(d, job, d.geoms[job.geom], here ? stage : reinterpret_cast<const unsigned char*>(gd.stage),
-                                     local, ts);
+        walk_tile<OUT, PERIODIC, NP, SPREAD>(d, job, d.geoms[job.geom],
+                                             here ? stage : reinterpret_cast<const unsigned char*>(gd.stage), local, spread, ts);
         __syncthreads();
         if (OUT == MADI_OUT_FUSED) {
             long long* out = reinterpret_cast<long long*>(d.accum) + (size_t)job.slot * 2 * n_out;
@@ -1115,40 +1149,68 @@ extern "C" int64_t madi_walk_smem_bytes(int32_t stage_bytes, int32_t tile_walker
            (24ll + FC_BYTES_PER_WALKER + 4 * (3 + 3 * MADI_MAX_PAIRS) + 12) * tile_walkers;
 }
 
-static int64_t fused_smem(const madi_walk_desc* d, int np) {
+static int64_t fused_smem(const madi_walk_desc* d, int np, int threads) {
     const int64_t n_out = (int64_t)d->n_pairs * d->n_b * d->n_dirs;
     return (int64_t)d->stage_smem + 16ll * n_out + 12ll * ((d->n_grid + 3) & ~3) +
-           (24 + FC_BYTES_PER_WALKER + 4 * (3 + 3 * np) + 12) * d->tile_walkers;
+           (24 + FC_BYTES_PER_WALKER + 4 * (3 + 3 * np) + 12) * threads;
 }
 
-template <int OUT, bool PER, int NP, int MINB>
-static madi_status launch_f32(const madi_walk_desc* d, cudaStream_t s) {
-    auto k = walk_f32_kernel<OUT, PER, NP, MINB>;
-    const int64_t sm = fused_smem(d, NP);
+// Walkers of a launch that leaves the chip idle go 16 or 8 to a warp.  A step is a
+// chain of ~2,200 cycles for a warp alone on its scheduler: 416 of them draw the
+// random numbers, which the free lanes then do for later steps (2 or 4 pairs at
+// once), and ~700 are facet passes, taken if any lane of the warp misses its cache:
+// fewer lanes, fewer passes.  10,000 walkers x 4,600 steps in a 64-cell box, 32 / 16
+// / 8 to a warp: 5.98 / 5.38 / 4.94 ms; 1,000: 5.76 / 5.03 / 4.46; 20,000: 6.33 /
+// 5.87 / -.  The line is one wave of the CTAs an SM holds: past it
+// the second wave costs more than it saves (40,000 walkers: 7.0 / 11.3 ms).
+constexpr int SPREAD_CTAS = 3;                   // resident on an SM: 168 registers a thread, no spills
+static int spread_of(const madi_walk_desc* d, int64_t smem) {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return 0;
+    const int64_t ctas = sms * std::min<int64_t>(SPREAD_CTAS, 227 * 1024 / (smem + 1024));
+    for (int spread = 2; spread > 0; --spread) {
+        const int64_t threads = (int64_t)d->n_tiles * d->tile_walkers << spread;
+        if (((d->tile_walkers << spread) % SPREAD_THREADS) == 0 && threads <= ctas * SPREAD_THREADS) return spread;
+    }
+    return 0;
+}
+
+template <int OUT, bool PER, int NP, int MINB, bool SPREAD>
+static madi_status launch_f32(const madi_walk_desc* d, int spread, cudaStream_t s) {
+    auto k = walk_f32_kernel<OUT, PER, NP, MINB, SPREAD>;
+    const int threads = SPREAD ? SPREAD_THREADS : d->tile_walkers;
+    const int64_t sm = fused_smem(d, NP, threads);
     if (sm > 227 * 1024) return host::fail(MADI_ERR_CAPACITY, "walker shared memory %lld B exceeds 227 KB", (long long)sm);
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return host::cuda_fail(e, "cudaFuncSetAttribute(walker)");
-    const int blocks = d->grid_blocks > 0 ? d->grid_blocks : d->n_tiles;
-    k<<<blocks, d->tile_walkers, (size_t)sm, s>>>(*d);
+    const int parts = SPREAD ? (d->tile_walkers << spread) / SPREAD_THREADS : 1;
+    const int blocks = (d->grid_blocks > 0 ? d->grid_blocks : d->n_tiles) * parts;
+    k<<<blocks, threads, (size_t)sm, s>>>(*d, spread);
     e = cudaGetLastError();
     if (e != cudaSuccess) return host::cuda_fail(e, "walker launch");
     return MADI_OK;
 }
 
+template <int OUT, bool PER, int NP>
+static madi_status launch_spread(const madi_walk_desc* d, cudaStream_t s) {
+    const int spread = spread_of(d, fused_smem(d, NP, SPREAD_THREADS));
+    if (spread) return launch_f32<OUT, PER, NP, SPREAD_CTAS, true>(d, spread, s);
+    return d->min_blocks >= 2 ? launch_f32<OUT, PER, NP, 2, false>(d, 0, s) : launch_f32<OUT, PER, NP, 1, false>(d, 0, s);
+}
+
 template <int OUT, bool PER>
 static madi_status launch_np(const madi_walk_desc* d, cudaStream_t s) {
-    const bool two = d->min_blocks >= 2;
-    if (OUT == MADI_OUT_FUSED && d->n_pairs > 4)
-        return two ? launch_f32<OUT, PER, 8, 2>(d, s) : launch_f32<OUT, PER, 8, 1>(d, s);
-    return two ? launch_f32<OUT, PER, 4, 2>(d, s) : launch_f32<OUT, PER, 4, 1>(d, s);
+    if (OUT == MADI_OUT_FUSED && d->n_pairs > 4) return launch_spread<OUT, PER, 8>(d, s);
+    return launch_spread<OUT, PER, 4>(d, s);
 }
 
 template <int OUT, bool PER>
 static const void* kernel_for(const madi_walk_desc* d) {
     const bool two = d->min_blocks >= 2;
     if (OUT == MADI_OUT_FUSED && d->n_pairs > 4)
-        return two ? (const void*)walk_f32_kernel<OUT, PER, 8, 2> : (const void*)walk_f32_kernel<OUT, PER, 8, 1>;
-    return two ? (const void*)walk_f32_kernel<OUT, PER, 4, 2> : (const void*)walk_f32_kernel<OUT, PER, 4, 1>;
+        return two ? (const void*)walk_f32_kernel<OUT, PER, 8, 2, false> : (const void*)walk_f32_kernel<OUT, PER, 8, 1, false>;
+    return two ? (const void*)walk_f32_kernel<OUT, PER, 4, 2, false> : (const void*)walk_f32_kernel<OUT, PER, 4, 1, false>;
 }
 
 extern "C" int32_t madi_walk_blocks_per_sm(const madi_walk_desc* d) {
@@ -1158,7 +1220,7 @@ extern "C" int32_t madi_walk_blocks_per_sm(const madi_walk_desc* d) {
         ? (per ? kernel_for<MADI_OUT_FUSED, true>(d) : kernel_for<MADI_OUT_FUSED, false>(d))
         : (per ? kernel_for<MADI_OUT_Y, true>(d) : kernel_for<MADI_OUT_Y, false>(d));
     const bool big = d->out_mode == MADI_OUT_FUSED && d->n_pairs > 4;
-    const int64_t sm = fused_smem(d, big ? 8 : 4);
+    const int64_t sm = fused_smem(d, big ? 8 : 4, d->tile_walkers);
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess) return 0;
     int n = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, d->tile_walkers, (size_t)sm) != cudaSuccess) return 0;

@@ -437,3 +437,39 @@ def test_f32_walker_equals_voxel_grid_rule(mode, n_cells, rho, V, pp):
     ens._device.clear()
     for x, y in zip(*out):
         assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("n, tile, out", [
+    (1, 32, "fused"), (33, 32, "fused"), (700, 64, "fused"), (225, 128, "fused"), (9_999, 128, "fused"),
+    (20_001, 128, "fused"), (300, 256, "fused"), (225, 128, "Y"), (5_003, 128, "Y"), (100, 64, "Y"),
+])
+@pytest.mark.parametrize("persistent", [True, False])
+def test_few_walkers_walk_as_in_a_full_launch(n, tile, out, persistent):
+    """A launch too small for the chip puts fewer walkers in a warp; sums, occupancy,
+    stored Y and crossing counts equal those of the same job in a launch that fills
+    it, bit for bit."""
+    import torch
+    from custom_madi_gb300 import _native as N
+    from custom_madi_gb300 import signal as S
+    from custom_madi_gb300.ensemble import create_ensemble
+    from custom_madi_gb300.walker_gpu import LaunchConfig, WalkBatch, WalkJob, pair_layout
+    fused = out == "fused"
+    over = dict(boundary_mode="periodic", n_cells=40) if fused else {}
+    cfg = SimConfig(n_walkers=n, n_ensembles=1, ts=0.01, T_max_ms=3.1, h_ms=0.31, small_deltas=[0.31], big_deltas=[1.55],
+                    b_values=[0.0, 1000.0, 3000.0], **over)
+    ens = create_ensemble(2.0e5, 3.0, cfg, seed=3, verify_vi=False, measure_vi=False)
+    c = S.build_columns(cfg)
+    lay = pair_layout(c.j_delta, c.j_Delta, c.j_sum, c.phase_coef) if fused else None
+    job = WalkJob(ens, 0.05, 11, n, walker_base=5)
+    res = []
+    for jobs in ([job], [job, WalkJob(ens, 0.05, 12, 120_000)]):
+        b = WalkBatch(jobs, cfg, layout=lay, out_mode=N.MADI_OUT_FUSED if fused else N.MADI_OUT_Y,
+                      launch=LaunchConfig(tile_walkers=tile, persistent=persistent))
+        b.launch()
+        torch.cuda.synchronize()
+        one = [b.occupancy[0], b.counters[0, [0, 1, 2, 6, 7]]]
+        one += [b.accum[0]] if fused else [b.Y[:n], b.inside_trace[:n]]
+        res.append([x.cpu().numpy() for x in one])
+    assert res[0][0][0] >= 0 and res[0][1][0] == n
+    for x, y in zip(*res):
+        assert np.array_equal(x, y)
