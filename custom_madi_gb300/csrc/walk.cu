@@ -78,8 +78,8 @@ struct TileShared {
 // walkers), so the rules above go for fewer of them.  Misses: 12.3 % of
 // walker-steps with the in / out rule of one sphere, 9.2 % with refused crossings
 // settled on one plane, 7.0 % with the rule across a plane, 5.9 % with M kept
-// instead of one radius (216 ms), 6.3 % with the first 16 slots deciding where
-// they can, in half the loads and sorting (203 ms).
+// instead of one radius (216 ms), 6.7 % with the first 16 slots deciding where
+// they can, in half the loads and sorting (204 ms).
 constexpr int FC_BYTES_PER_WALKER = 6 * 16;
 
 // Sort key of a facet margin: the margin with the low KEY_BITS mantissa bits
@@ -124,9 +124,10 @@ MADI_DEV void merge4(float& a0, float& a1, float& a2, float& a3, float b0, float
 // of each other, which the widened band covers); the fourth key bounds every other
 // facet from below.  Slots are in order of h and m_k >= h_k - |w|, so the first 16
 // slots decide whenever the last of them has h - |w| above the smallest margin
-// (`rest`, which then bounds the slots not read); else the next 16 follow.  The
-// group decides by the facet-plane rule and its first lane writes the walker's
-// label cache.  A walker whose point lies across a facet is queued again from the
+// (`rest`, which then bounds the slots not read); else the group reads the next
+// 16 (each by its own need: caches and counts do not depend on the other walkers
+// of the warp).  The group decides by the facet-plane rule and its first lane
+// writes the walker's label cache.  A walker whose point lies across a facet is queued again from the
 // cell beyond the most violated facet (at most three moves).  Called by all 32
 // lanes; `start` is each walker's first cell; `refuse` marks walkers inside
 // `start` whose acceptance number rejects any membrane crossing: a point outside
@@ -171,7 +172,7 @@ MADI_DEV int coop_facets(const Geo& g, const TileShared& ts, bool need, float qx
         float q0 = 0.f, q1 = 0.f, q2 = 0.f, q3 = 0.f;
         float4 p1, p2, p3;
         int nb1 = -1, nb2 = -1, k0 = 0;
-        bool more;
+        bool more = true;                             // this group reads these slots (others: no key below infinity)
         do {
             float4 f[FU];
 #pragma unroll
@@ -187,7 +188,8 @@ MADI_DEV int coop_facets(const Geo& g, const TileShared& ts, bool need, float qx
             }
             float k[FU];
 #pragma unroll
-            for (int i = 0; i < FU; ++i) k[i] = margin_key(facet_m(f[i], wx, wy, wz), (uint32_t)(k0 + sub + FG * i));
+            for (int i = 0; i < FU; ++i)
+                k[i] = more ? margin_key(facet_m(f[i], wx, wy, wz), (uint32_t)(k0 + sub + FG * i)) : __int_as_float(0x7f800000);
             sort4(k[0], k[1], k[2], k[3]);
 #pragma unroll
             for (int o = 1; o < FG; o <<= 1) {
@@ -213,11 +215,12 @@ MADI_DEV int coop_facets(const Geo& g, const TileShared& ts, bool need, float qx
             nb2 = n2;
             // |w| to 2^-22 relative, which T covers
             const float w2 = fmaf(wx, wx, fmaf(wy, wy, wz * wz));
-            rest = g.sorted ? h_last - w2 * rsqrtf(fmaxf(w2, 1e-30f)) - T : -3.0e38f;
             k0 += FG * FU;
-            more = act && k0 < S && !(rest > m1 + 2.0f * T);
+            if (more)
+                rest = k0 >= S ? 3.0e38f : (g.sorted ? h_last - w2 * rsqrtf(fmaxf(w2, 1e-30f)) - T : -3.0e38f);
+            more = more && act && !(rest > m1 + 2.0f * T);
         } while (__any_sync(MADI_FULL, more));
-        const float m4 = k0 < S ? fminf(key_floor(q3), rest) : key_floor(q3);
+        const float m4 = fminf(key_floor(q3), rest);
         const float dd = m1 - cc.w;
         int verdict = m1 > T ? (dd > T ? FACET_IN : (dd < -T ? FACET_OUT : FACET_BAND))
                              : (m1 < -T ? (nb1 >= 0 ? VERDICT_MOVE + nb1 : FACET_LEFT) : FACET_BAND);
