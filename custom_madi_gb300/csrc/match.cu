@@ -571,10 +571,12 @@ extern "C" madi_status madi_match(const madi_match_desc* d, void* stream) {
     }
     MatchPlan plan = match_plan(d->n_vox, d->n_lib, d->n_feat);
     unsigned char* scratch = nullptr;
-    if (d->scratch && (reinterpret_cast<uintptr_t>(d->scratch) & 255) == 0 && d->scratch_bytes >= FP32_SCRATCH + plan.bytes)
+    const bool ours = d->mode == MADI_MATCH_FIXED_S0 || (d->flags & MADI_MATCH_FLAG_SCRATCH);
+    if (ours && d->scratch && (reinterpret_cast<uintptr_t>(d->scratch) & 255) == 0 &&
+        d->scratch_bytes >= FP32_SCRATCH + plan.bytes)
         scratch = static_cast<unsigned char*>(d->scratch) + FP32_SCRATCH;
     else
-        plan = MatchPlan{false, 1, d->n_lib, 0};            // the caller's scratch holds the column means only
+        plan = MatchPlan{false, 1, d->n_lib, 0};            // no scratch, or it holds the column means only
     return d->mode == MADI_MATCH_FIXED_S0 ? launch_fp32_mode<MADI_MATCH_FIXED_S0>(d, plan, mu, scratch, s)
                                           : launch_fp32_mode<MADI_MATCH_FREE_S0>(d, plan, mu, scratch, s);
 }

@@ -76,6 +76,9 @@ def match_device(measured, lib_mat, *, free_s0: bool = False, precision: str = "
     res = torch.empty(n_vox, dtype=torch.float32, device=M.device)
     s0 = torch.empty(n_vox, dtype=torch.float32, device=M.device) if free_s0 else None
     need = int(N.lib().madi_match_scratch_bytes(n_vox, Lm.shape[0], F, prec, int(topk)))
+    if free_s0 and prec == N.MADI_MATCH_FP32:
+        scratch = None                  # never used the caller's, which overlapping calls may share
+        flags = int(flags) | N.MADI_MATCH_FLAG_SCRATCH
     if need > 0 and (scratch is None or scratch.numel() < need + 256):
         scratch = torch.empty(need + 256, dtype=torch.uint8, device=M.device)
     d = N.MadiMatchDesc()

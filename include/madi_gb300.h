@@ -173,7 +173,9 @@ enum {
  *
  * precision 64 is the reference's walker design (madi/walker_gpu.py:520-585):
  * one thread per walker of jobs[0], separately rounded fp64 arithmetic, the
- * exact KD rule at every step, Y output only; n_tiles = ceil(n_walkers / 128).
+ * label of the exact KD rule at every step (from the cell facet table where its
+ * margins prove it, else by the KD descent), Y output only; n_tiles =
+ * ceil(n_walkers / 128).
  * With MADI_RNG_PHILOX it evaluates the fp32 walker's Philox numbers in fp64.
  */
 typedef struct madi_walk_desc {
@@ -181,7 +183,8 @@ typedef struct madi_walk_desc {
     const madi_walk_job* jobs;     /* device array                                    */
     int32_t n_geoms, n_jobs;
     int32_t n_tiles;               /* total tiles over all jobs                       */
-    int32_t tile_walkers;          /* walkers per tile (= threads per block)          */
+    int32_t tile_walkers;          /* walkers per tile (threads per block, but in launches
+                                      too small for the GPU: 128 threads there)       */
     int32_t grid_blocks;           /* persistent CTAs; 0 = one per tile               */
     int32_t stage_smem;            /* max stage_bytes over geoms; 0 = read in place   */
     int32_t boundary;              /* MADI_BOUNDARY_* shared by every geometry        */
@@ -245,10 +248,11 @@ madi_status madi_walk_batched(const madi_walk_desc* desc, void* stream);
 /* Replaces _reduce_kernel (madi/walker_gpu.py:658-695) for grids too large for
  * the fused epilogue: Y [n_walkers][n_grid][3] fp64 -> cos_sum / sin_sum
  * [n_cols] fp64, the sums over walkers and the 3 axes of cos / sin(coef dM),
- * dM = Y[jd] + Y[jD] - Y[js] per column (jd, jD, js, coef).  Y is read once per
- * block of 1,024 columns; per-CTA fp64 partials are added as 2^-32 fixed-point
- * integers, so the result is independent of scheduling (each partial rounded
- * once: |error| <= 2^-33 per walker block and column).  scratch: device,
+ * dM = Y[jd] + Y[jD] - Y[js] per column (jd, jD, js, coef).  dM and the phase
+ * are fp64; the phase is reduced to turns, cos and sin are taken from it in
+ * fixed point and added as integers, so the result is independent of
+ * scheduling (no further from 64-bit arithmetic than fp64 sincos summed per
+ * CTA).  scratch: device,
  * 8-byte aligned, madi_reduce_Y_scratch_bytes(n_cols) bytes, no initialisation
  * needed. */
 int64_t madi_reduce_Y_scratch_bytes(int32_t n_cols);
@@ -271,9 +275,13 @@ enum { MADI_MATCH_FP32 = 0, MADI_MATCH_BF16 = 1 };
  *   fixed S0: best = argmin_j (|L_j|^2 - 2 m.L_j), resid = |m|^2 + that
  *   free  S0: best = argmin_j over m.L_j > 0 of |m|^2 - (m.L_j)^2/|L_j|^2
  * Ties pick the lowest library index.
- * FP32: exhaustive fp32 scan on the CUDA cores; fixed S0 scores the pair
- *       centred on the library column mean (same argmin, ~|L|^2/|L-mu|^2
- *       smaller rounding than the uncentred form).
+ * FP32: fp32 scores on the CUDA cores; fixed S0 scores the pair centred on the
+ *       library column mean (same argmin, ~|L|^2/|L-mu|^2 smaller rounding than
+ *       the uncentred form).  Large calls order voxels and entries by a search
+ *       index in the scratch and skip the tiles of entries whose lower bound
+ *       exceeds a voxel's best: the choice is the exhaustive scan's.  With only
+ *       256 bytes of scratch (fixed S0), or for free S0 without
+ *       MADI_MATCH_FLAG_SCRATCH, every call scans all entries.
  * BF16: tcgen05 BF16 x BF16 -> FP32 (TMEM) scores, a per-voxel top-k (k of 8,
  *       16, 32) candidate list, then an fp32 rescore of the k candidates.
  *       Fixed S0 (library <= 32768 entries): a first launch over each voxel
@@ -285,7 +293,7 @@ enum { MADI_MATCH_FP32 = 0, MADI_MATCH_BF16 = 1 };
  *       place.
  * measured: device fp32 [n_vox][n_feat]; lib: device fp32 [n_lib][n_feat].
  * scratch: 256-byte aligned device buffer of madi_match_scratch_bytes(...)
- * bytes (contents need no initialisation; FP32 free S0 ignores it).
+ * bytes (contents need no initialisation; FP32 runs with less, see above).
  */
 typedef struct madi_match_desc {
     const float* measured;
@@ -311,6 +319,9 @@ typedef struct madi_match_desc {
 /* BF16 fixed S0: scan every library tile for every voxel (no principal-axis
  * cut); the result is the same up to BF16 score ties at the k-th place. */
 #define MADI_MATCH_FLAG_FULL_SCAN 2
+/* FP32 free S0: the scratch belongs to this call and may be used (without the
+ * flag it is ignored, so calls that overlap may name the same buffer). */
+#define MADI_MATCH_FLAG_SCRATCH 4
 
 int64_t madi_match_scratch_bytes(int64_t n_vox, int32_t n_lib, int32_t n_feat, int32_t precision,
                                  int32_t topk);

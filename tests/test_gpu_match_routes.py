@@ -11,24 +11,26 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-def _match(vox, lib, free, scratch_bytes=None):
+def _match(vox, lib, free, scratch_bytes=None, flags=4):
     import torch
     from custom_madi_gb300 import _native as N
     M, L = torch.from_numpy(vox).cuda(), torch.from_numpy(lib).cuda()
     n, F = M.shape
     need = int(N.lib().madi_match_scratch_bytes(n, len(lib), F, N.MADI_MATCH_FP32, 32))
     nbytes = need if scratch_bytes is None else scratch_bytes
-    buf = torch.empty(nbytes + 256, dtype=torch.uint8, device="cuda")
+    buf = torch.full((nbytes + 256,), 0x5A, dtype=torch.uint8, device="cuda")
     out = [torch.full((n,), -7, dtype=torch.int32, device="cuda")] + [torch.zeros(n, device="cuda") for _ in range(2)]
     d = N.MadiMatchDesc()
     d.measured, d.lib, d.n_vox, d.n_lib, d.n_feat = N.ptr(M), N.ptr(L), n, len(lib), F
     d.mode = N.MADI_MATCH_FREE_S0 if free else N.MADI_MATCH_FIXED_S0
-    d.precision, d.topk = N.MADI_MATCH_FP32, 32
+    d.precision, d.topk, d.flags = N.MADI_MATCH_FP32, 32, flags
     d.best_idx, d.best_resid, d.best_s0 = (N.ptr(t) for t in out)
     base = N.ptr(buf)
     d.scratch, d.scratch_bytes = base + (-base) % 256, nbytes
     N.check(N.lib().madi_match(C.byref(d), torch.cuda.current_stream().cuda_stream), "madi_match")
     torch.cuda.synchronize()
+    if free and not flags:
+        assert bool((buf == 0x5A).all())         # the scratch is not this call's to write
     return need, [t.cpu().numpy() for t in out]
 
 
@@ -86,3 +88,12 @@ def test_split_scan_equals_scan(n_vox, n_lib, F, kind, free):
     _, b = _match(vox, lib, free, scratch_bytes=256)
     for x, y in zip(a, b):
         assert np.array_equal(x, y, equal_nan=True)
+
+
+@pytest.mark.parametrize("n_vox, n_lib, F", [(50_001, 4_099, 20), (3_001, 5_000, 12)])
+def test_free_s0_leaves_the_scratch_alone_without_the_flag(n_vox, n_lib, F):
+    vox, lib = _data("decays", n_vox, n_lib, F, np.random.default_rng(1))
+    _, a = _match(vox, lib, True)
+    _, b = _match(vox, lib, True, flags=0)
+    for x, y in zip(a, b):
+        assert np.array_equal(x, y)
