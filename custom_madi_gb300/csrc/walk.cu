@@ -349,8 +349,12 @@ __device__ __forceinline__ void walk_tile(const madi_walk_desc& d, const madi_wa
     const Geo g = make_geo(gd, base);
     const bool active = local < job.n_walkers && (!SPREAD || lane < (32 >> spread));
     const uint32_t widx = job.walker_base + (uint32_t)local;
-    const float L = (float)gd.L;
-    const float sigma = (float)d.sigma;
+    // fp64 is ~2 lanes a cycle: conversions and compares of the descriptor's doubles
+    // are done here once (the empty asm keeps them from being redone in each step,
+    // where they held 31 % of the fp64 pipe: 204 -> 199 ms, 64 entries x 25,000
+    // walkers; 4.98 -> 4.71 ms, one entry x 10,000)
+    float L = (float)gd.L, sigma = (float)d.sigma;
+    asm volatile("" : "+f"(L), "+f"(sigma));
     const bool cells = gd.has_cells != 0;
     const bool stream = d.rng == MADI_RNG_STREAM;
 
@@ -411,10 +415,12 @@ __device__ __forceinline__ void walk_tile(const madi_walk_desc& d, const madi_wa
         const unsigned b = __ballot_sync(0xffffffffu, active && inside);
         if (lane == 0 && b) atomicAdd(&ts.occ[0], (unsigned)__popc(b));
     }
-    const bool always = job.pp >= 1.0;
+    int always = job.pp >= 1.0;
+    asm volatile("" : "+r"(always));
     const uint32_t th1 = (uint32_t)(job.thr1 >> 32), th2 = (uint32_t)(job.thr2 >> 32);
     // error bound of any facet margin in the box (|w|_1 <= 3 L)
-    const float t_any = fmaf(6.0f * MADI_EPS21, L, (float)gd.facet_tol);
+    float t_any = fmaf(6.0f * MADI_EPS21, L, (float)gd.facet_tol);
+    asm volatile("" : "+f"(t_any));
     const float a_min = gd.alpha_min;
     float gv[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     uint32_t acc_word = 0, acc_word_odd = 0;
@@ -425,14 +431,15 @@ __device__ __forceinline__ void walk_tile(const madi_walk_desc& d, const madi_wa
         // ---- random numbers: one Philox call per step on average ----
         float nx, ny, nz;
         uint32_t word = 0;
-        double ustream = 0.0;
+        bool u_ge1 = false, u_lt1 = false, u_lt2 = false;
         if (stream) {
             if (!dead) {
                 const size_t o = ((size_t)step * job.n_walkers + local);
                 nx = (float)d.incr[3 * o + 0];
                 ny = (float)d.incr[3 * o + 1];
                 nz = (float)d.incr[3 * o + 2];
-                ustream = d.unif[o];
+                const double u = d.unif[o];
+                u_ge1 = u >= job.pp; u_lt1 = u < job.pp; u_lt2 = u < job.pp * job.pp;
             } else { nx = ny = nz = 0.f; }
         } else if (SPREAD) {
             // lane group i draws step pair i of 1 << spread pairs; each step reads its pair's
@@ -472,7 +479,7 @@ __device__ __forceinline__ void walk_tile(const madi_walk_desc& d, const madi_wa
         }
         const float ex = dx + nx, ey = dy + ny, ez = dz + nz;
         // ---- label from the cached facet planes ----
-        const bool refuse = inside && !always && (stream ? ustream >= job.pp : word > th1);
+        const bool refuse = inside && !always && (stream ? u_ge1 : word > th1);
         bool t1 = false;
         int t1_in = 0, t1_cell = cell;
         int start = cell;
@@ -506,7 +513,7 @@ __device__ __forceinline__ void walk_tile(const madi_walk_desc& d, const madi_wa
                 bool accept = true;
                 if (m > 0 && !always) {
                     if (stream) {
-                        accept = ustream < (m == 1 ? job.pp : job.pp * job.pp);
+                        accept = m == 1 ? u_lt1 : u_lt2;
                     } else {
                         const uint32_t th = m == 1 ? th1 : th2;
                         if (word != th) {
@@ -731,7 +738,7 @@ __global__ void __launch_bounds__(SPREAD ? SPREAD_THREADS : 256, MINB) walk_f32_
 // the fp64 point to fp32, sqrt(3) 2^-24 L), and from the KD rule in the rest
 // (~0.04 % of steps).  What remains is bound by the fp64 pipe: Box-Muller in
 // fp64, once per pair of steps.  16,000 walkers x 4,600 steps in a 64-cell box:
-// 888 ms before, 34 ms now.
+// ~900 ms before, 32 ms now.
 // ---------------------------------------------------------------------------
 constexpr int F64_THREADS = 128;
 
