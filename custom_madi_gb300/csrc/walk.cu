@@ -305,14 +305,14 @@ __device__ __noinline__ FullLabel full_labels(const madi_geometry* gd, const uns
         const float sz = __shfl_sync(MADI_FULL, qz, src);
         const int sg = __shfl_sync(MADI_FULL, guess, src);
         int s1 = 0, in = 0;
-        const int st = coop_classify(g, sx, sy, sz, sg, lane, s1, in);
+        int st = coop_classify(g, sx, sy, sz, sg, lane, s1, in);
+        if (__any_sync(MADI_FULL, st == CLS_FALLBACK)) {
+            st = coop_list_f64(g, sx, sy, sz, lane, s1, in);
+            if (lane == 0) atomicAdd(fallbacks, 1ull);
+        }
         if (lane == src) { status = st; seed = s1; inside = in; }
     }
     __syncwarp();
-    if (need && status == CLS_FALLBACK) {
-        status = classify_list_f64(g, qx, qy, qz, seed, inside);
-        atomicAdd(fallbacks, 1ull);
-    }
     return FullLabel{status, need && status == CLS_OK ? cell_of(g, seed) : 0, inside};
 }
 

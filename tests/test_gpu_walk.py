@@ -473,3 +473,38 @@ def test_few_walkers_walk_as_in_a_full_launch(n, tile, out, persistent):
     assert res[0][0][0] >= 0 and res[0][1][0] == n
     for x, y in zip(*res):
         assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("mode, n_cells, rho, V", [
+    ("periodic", 2, 2.0e5, 4.9), ("periodic", 27, 5.0e7, 0.0199), ("periodic", 300, 2.0e5, 3.0),
+    ("si_fatal_escape", 0, 2.0e5, 4.0),
+])
+def test_fp64_rule_of_undecided_points_equals_facet_planes(mode, n_cells, rho, V):
+    """Without the facet table every step takes the voxel-grid rule and the points it
+    leaves undecided its warp-wide fp64 form (candidate lists below and above 32,
+    images of one cell); with the table nearly all come from the facet planes.
+    Both walks are the same, bit for bit."""
+    import torch
+    from custom_madi_gb300 import _native as N
+    from custom_madi_gb300.ensemble import create_ensemble
+    from custom_madi_gb300.walker_gpu import WalkBatch, WalkJob
+    n = 4_000
+    over = dict(boundary_mode="periodic", n_cells=n_cells) if mode == "periodic" else {}
+    cfg = SimConfig(n_walkers=n, n_ensembles=1, ts=0.01, T_max_ms=6.0, h_ms=0.1, small_deltas=[1.0], big_deltas=[3.0],
+                    b_values=[0.0, 1000.0], **over)
+    ens = create_ensemble(rho, V, cfg, seed=4, verify_vi=False, measure_vi=False)
+    out = []
+    for table in (True, False):
+        ens._device.clear()
+        dev = ens.device()
+        if not table:
+            dev.struct.n_cells = 0
+        b = WalkBatch([WalkJob(ens, 0.05, 19, n)], cfg, out_mode=N.MADI_OUT_Y)
+        b.launch()
+        torch.cuda.synchronize()
+        cnt = b.counters_np()[0]
+        out.append((b.Y.cpu().numpy(), b.inside_trace.cpu().numpy(), b.occupancy.cpu().numpy(), cnt[[0, 1, 2, 6, 7]]))
+    assert cnt[5] > 20                       # points decided in fp64
+    ens._device.clear()
+    for x, y in zip(*out):
+        assert np.array_equal(x, y)
