@@ -43,8 +43,8 @@ METRIC = "walker-steps/s"
 CONFIG_NAME = "batched library build: 256 entries x 1e5 walkers x 4600 steps, 27-512 cells, 20 cols x 24 dirs"
 # walk_f32_kernel DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum)
 # per walker-step, from one ncu capture of 16 entries x 2e4 walkers x 4,600
-# steps: 6.39 MB + 0 MB over 1.472e9 walker-steps
-WALK_DRAM_BYTES_PER_WALKER_STEP = 6.39e6 / 1.472e9
+# steps: 5.50 MB + 0 MB over 1.472e9 walker-steps
+WALK_DRAM_BYTES_PER_WALKER_STEP = 5.50e6 / 1.472e9
 SIGNAL_ERR = 0.005          # absolute standard error on S (normalised to b = 0)
 
 
@@ -449,12 +449,13 @@ def plain_and_served(dev, cfg, jobs, lay, dirs, batched_rate, batch):
 
 
 def reference_design_leg(dev, cfg, jobs, cols, batched_rate, n_entries=4):
-    """The reference's GPU design for the same entries (madi/walker_gpu.py:
-    520-695 kernels, :989-1063 launch): per entry the geometry H2D, one fp64
-    walk launch (one thread per walker, exact KD rule every step, Y stored to
-    HBM), the column reduction over the 3 axes, synchronize, D2H of the sums.
-    Both kernels are this package's CUDA; the entries, walkers and Philox
-    numbers are the batched arm's, so the Monte Carlo error is matched."""
+    """The reference's launch structure and arithmetic for the same entries
+    (madi/walker_gpu.py:520-695 kernels, :989-1063 launch): per entry the geometry
+    H2D, one fp64 walk launch (one thread per walker, Y stored to HBM), the column
+    reduction over the 3 axes, synchronize, D2H of the sums.  Both kernels are
+    this package's CUDA, whose fp64 walker takes most labels from facet planes
+    instead of a KD descent per step; the entries, walkers and Philox numbers are
+    the batched arm's, so the Monte Carlo error is matched."""
     import torch
     from custom_madi_gb300 import _native as N
     from custom_madi_gb300.walker_gpu import WalkBatch
@@ -486,8 +487,9 @@ def reference_design_leg(dev, cfg, jobs, cols, batched_rate, n_entries=4):
     return {"entries": len(sub), "walkers_per_entry": int(sub[0].n_walkers), "s": t,
             "walker_steps_per_s": rate, "batched_over_reference_design": batched_rate / rate,
             "clean": bool(ok),
-            "note": "the reference's GPU design (fp64, one thread per walker, exact KD rule every step, "
-                    "Y stored, separate reduction), one entry per launch, as CUDA kernels of this package"}
+            "note": "the reference's launch structure and arithmetic (fp64, one thread per walker, the KD rule's "
+                    "labels, Y stored, separate reduction), one entry per launch, as this package's CUDA kernels "
+                    "(labels from facet planes, the KD descent in their error band only)"}
 
 
 def match_leg(dev, threads):
@@ -724,7 +726,7 @@ def reduce_leg(dev):
     return {"columns": int(len(pc)), "walkers": n, "n_grid": ng, "ms": t * 1e3,
             "walker_column_axis_terms_per_s": terms / t, "Y_bytes": int(Y.numel() * 8),
             "cpu_oracle_terms_per_s_1_thread": 64.0 * len(pc) * 3 / t_cpu,
-            "note": "Y read once per block of 1,024 columns (31 blocks), fp64 sincos per term"}
+            "note": "Y read once per block of 1,024 columns (31 blocks), fp64 phase, fixed-point cos and sin"}
 
 
 if __name__ == "__main__":

@@ -32,7 +32,7 @@
 //     voxels in the index's embedding and only visits those that can matter;
 //   - d is formed in pairs of floats (48 bits), then rounded to fp32 as before.
 // The entries a voxel sums, and their order, are unchanged.  100,000 voxels x
-// 20,000 entries x 20 features, sigma_m 0.02: 33.2 ms before, 6.4 ms now (5.2 ms of it this
+// 20,000 entries x 20 features, sigma_m 0.02: 33.2 ms before, 6.5 ms now (5.4 ms of it this
 // kernel, bound by issue; the rest is the index and host copies).
 #include <cstdint>
 #include "madi_device.cuh"

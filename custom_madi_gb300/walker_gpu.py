@@ -456,7 +456,7 @@ def run_walk_Y(ens: Ensemble, kio: float, cfg: Optional[SimConfig] = None, seed:
                precision: Optional[int] = None, launch: Optional[LaunchConfig] = None):
     """Walk one ensemble and return Y [N, n_grid, 3] (madi/walker_gpu.py:1093-1133).
 
-    A replay stream runs the fp64 walker (reference arithmetic, exact KD rule)
+    A replay stream runs the fp64 walker (reference arithmetic, the KD rule's labels)
     unless precision=32 asks for the production fp32 walker; without a stream
     the walker draws Philox4x32-10 numbers keyed by ``seed`` (fp32 walker by
     default; precision=64 walks the same numbers with the fp64 walker).
@@ -533,9 +533,9 @@ def simulate_jobs(jobs: Sequence[WalkJob], cfg: SimConfig, columns: Tuple, *, di
                   launch: Optional[LaunchConfig] = None, check: bool = True, precision: int = 32) -> list:
     """Walk every job in one persistent launch; per job cos / sin sums [n_cols, n_dirs].
 
-    precision=64 runs the reference's GPU design instead (madi/walker_gpu.py:
-    520-695, :989-1063): per job one fp64 walk launch that stores Y, then a
-    column reduction over the 3 Cartesian axes (sums [n_cols, 1]).
+    precision=64 runs the reference's arithmetic and launch structure instead
+    (madi/walker_gpu.py:520-695, :989-1063): per job one fp64 walk launch that
+    stores Y, then a column reduction over the 3 Cartesian axes (sums [n_cols, 1]).
     """
     _require_gpu(None)
     if precision not in (32, 64):
