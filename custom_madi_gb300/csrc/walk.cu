@@ -202,7 +202,9 @@ MADI_DEV int coop_facets(const Geo& g, const TileShared& ts, bool need, float qx
             if (k0 == 0) { q0 = k[0]; q1 = k[1]; q2 = k[2]; q3 = k[3]; }
             else merge4(q0, q1, q2, q3, k[0], k[1], k[2], k[3]);
             const float h_last = __shfl_sync(MADI_FULL, f[FU - 1].w, lane | (FG - 1));
-            const uint32_t k1 = base + key_slot(q0), k2 = base + key_slot(q1), k3 = base + key_slot(q2);
+            // (a NaN margin's key names no slot of the cell)
+            const uint32_t last = (uint32_t)S - 1u;
+            const uint32_t k1 = base + min(key_slot(q0), last), k2 = base + min(key_slot(q1), last), k3 = base + min(key_slot(q2), last);
             // the three candidates' records and neighbours, loaded together (L1)
             p1 = g.fpl[k1]; p2 = g.fpl[k2]; p3 = g.fpl[k3];
             const int n1 = g.fnbr[k1], n2 = g.fnbr[k2], n3 = g.fnbr[k3];
@@ -218,7 +220,8 @@ MADI_DEV int coop_facets(const Geo& g, const TileShared& ts, bool need, float qx
             k0 += FG * FU;
             if (more)
                 rest = k0 >= S ? 3.0e38f : (g.sorted ? h_last - w2 * rsqrtf(fmaxf(w2, 1e-30f)) - T : -3.0e38f);
-            more = more && act && !(rest > m1 + 2.0f * T);
+            // the stride ends the loop: for a point that is not finite m1 + 2 T is NaN
+            more = more && act && k0 < S && !(rest > m1 + 2.0f * T);
         } while (__any_sync(MADI_FULL, more));
         const float m4 = fminf(key_floor(q3), rest);
         const float dd = m1 - cc.w;
@@ -254,7 +257,8 @@ MADI_DEV int coop_facets(const Geo& g, const TileShared& ts, bool need, float qx
 // `refuse`: the walker is inside `cell` and its acceptance number rejects any
 // crossing, so a point outside that shrunk cell is as good as decided (reported
 // as outside, whatever its own label): one plane with m < alpha_c - T(q) does,
-// anywhere (t_any >= T(q)).  Otherwise `start` becomes the cell beyond the cached
+// anywhere in the box (t_any >= T(q) while |w|_1 <= 3 L, which an infinite step
+// does not pass).  Otherwise `start` becomes the cell beyond the cached
 // facet k1 or k2 that the point lies farther across (exact planes of the cell).
 template <bool PERIODIC>
 MADI_DEV bool cached_label(const TileShared& ts, float L, float qx, float qy, float qz, bool refuse, int cell, float t_any,
@@ -281,7 +285,7 @@ MADI_DEV bool cached_label(const TileShared& ts, float L, float qx, float qy, fl
     cell_q = cc;
     in = in_c ? 1 : 0;
     if (near && (in_c || out)) return true;
-    if (refuse && cc == cell && mm < th.x - t_any) { in = 0; return true; }
+    if (refuse && cc == cell && mm < th.x - t_any && fabsf(wx) + fabsf(wy) + fabsf(wz) <= 3.0f * L) { in = 0; return true; }
     const int nb = __float_as_int(m1 <= m2 ? th.w : ce.w);
     if (!refuse && fminf(m1, m2) < -th.y && nb >= 0) start = nb;
     return false;
@@ -861,7 +865,7 @@ __global__ void __launch_bounds__(F64_THREADS) walk_f64_kernel(const madi_walk_d
         if (facets) {
             const float fx = (float)qx, fy = (float)qy, fz = (float)qz;
             // a step longer than the box leaves a periodic point outside after one wrap
-            const bool boxed = ok && fminf(fx, fminf(fy, fz)) >= 0.f && fmaxf(fx, fmaxf(fy, fz)) <= Lf;
+            const bool boxed = ok && fx >= 0.f && fx <= Lf && fy >= 0.f && fy <= Lf && fz >= 0.f && fz <= Lf;     // no NaN
             int start = cell;
             // (no early refusal here: `refuse` is false)
             if (boxed) known = periodic ? cached_label<true>(ts, Lf, fx, fy, fz, false, cell, 0.f, a_min, nin, ncell, start)
@@ -1250,6 +1254,9 @@ extern "C" madi_status madi_walk(const madi_walk_desc* d, void* stream) {
     if (!d->counters || !d->occupancy) return host::fail(MADI_ERR_INVALID, "counters and occupancy are required");
     if (d->rng == MADI_RNG_STREAM && (!d->init || !d->incr || !d->unif))
         return host::fail(MADI_ERR_INVALID, "stream replay needs init / incr / unif");
+    // a replay stream brings its own steps
+    if (d->rng == MADI_RNG_PHILOX && !std::isfinite(d->precision == 32 ? (double)(float)d->sigma : d->sigma))
+        return host::fail(MADI_ERR_INVALID, "walk: sigma %g is not a finite step", d->sigma);
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     if (d->precision == 64) {
         if (d->n_jobs != 1) return host::fail(MADI_ERR_UNSUPPORTED, "fp64 walker walks one job");

@@ -192,7 +192,8 @@ typedef struct madi_walk_desc {
     int32_t rng;                   /* MADI_RNG_*                                      */
     int32_t out_mode;              /* MADI_OUT_*                                      */
     int32_t n_steps, steps_per_h, n_grid;
-    double  sigma, ts;
+    double  sigma, ts;             /* sigma: finite (precision 32: in fp32), or the walk is
+                                      refused (MADI_ERR_INVALID); a replay stream ignores it */
     /* fused epilogue */
     int32_t n_pairs, n_b, n_dirs;
     int32_t min_blocks;            /* register budget: 1 = 255 regs, 2 = 128 regs/thread */
