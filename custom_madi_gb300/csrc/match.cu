@@ -265,17 +265,17 @@ MADI_DEV void tile_fetch(float4* dst, const float4* src, uint32_t bytes, uint64_
                  :: "r"(d), "l"(src), "r"(bytes), "r"(b) : "memory");
 }
 
-// Waits for phase `parity` of a tile copy, ~1 s at most (20 us suspends); false
-// if it ran out.
-MADI_DEV bool tile_wait(uint64_t* bar, uint32_t parity) {
+// Waits for phase `parity` of a tile copy, ~1 s at most (20 us suspends); false in
+// every lane if it ran out for one.
+constexpr int WAIT_POLLS = 50000;
+constexpr int STALL_POLLS = 64;                 // the test-only stalled wait (MADI_MATCH_FLAG_TEST_STALL)
+MADI_DEV bool tile_wait(uint64_t* bar, uint32_t parity, int polls = WAIT_POLLS) {
     const uint32_t b = (uint32_t)__cvta_generic_to_shared(bar);
-    for (int i = 0; i < 50000; ++i) {
-        uint32_t done;
+    uint32_t done = 0;
+    for (int i = 0; i < polls && !done; ++i)
         asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n selp.u32 %0, 1, 0, p;\n}"
                      : "=r"(done) : "r"(b), "r"(parity), "r"(20000u) : "memory");
-        if (done) return true;
-    }
-    return false;
+    return __all_sync(MADI_FULL, done);
 }
 
 template <int N, int MODE, int WARPS>
@@ -287,7 +287,7 @@ __global__ void __launch_bounds__(MATCH_THREADS, N <= 12 ? 4 : N <= 24 ? 3 : 2) 
     constexpr int TILE4 = prune::TILE * (N / 4 + 1);                           // float4 of a tile's rows
     extern __shared__ __align__(128) float4 stage[];                           // [warp][2][TILE4]
     __shared__ float sv[prune::B_FLOATS], smu[N];
-    __shared__ uint64_t bars[NW][2];
+    __shared__ uint64_t bars[NW][2], never;                                    // never: no thread arrives (tests)
     __shared__ unsigned long long merged[WARPS > 1 ? GROUPS : 1][64];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int i = threadIdx.x; i < prune::B_FLOATS; i += MATCH_THREADS) sv[i] = ix.basis[i];
@@ -296,6 +296,7 @@ __global__ void __launch_bounds__(MATCH_THREADS, N <= 12 ? 4 : N <= 24 ? 3 : 2) 
     if (WARPS > 1)
         for (int i = threadIdx.x; i < GROUPS * 64; i += MATCH_THREADS) merged[i >> 6][i & 63] = ~0ull;
     if (lane < 2) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"((uint32_t)__cvta_generic_to_shared(&bars[warp][lane])) : "memory");
+    if (threadIdx.x == 0) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"((uint32_t)__cvta_generic_to_shared(&never)) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     __syncthreads();
     const int64_t p0 = ((int64_t)blockIdx.x * GROUPS + warp / WARPS) * 64;
@@ -354,8 +355,9 @@ __global__ void __launch_bounds__(MATCH_THREADS, N <= 12 ? 4 : N <= 24 ? 3 : 2) 
         };
         auto scan = [&]() {
             const uint32_t i = scanned & 1;
-            if (!tile_wait(&bars[warp][i], (scanned >> 1) & 1)) stuck = true;
-            else scan_tile<N, MODE>(reinterpret_cast<const ulonglong2*>(buf + i * TILE4), mm[0], mm[1], pv[0], pv[1]);
+            stuck = !tile_wait(&bars[warp][i], (scanned >> 1) & 1);
+            if (stuck) return;
+            scan_tile<N, MODE>(reinterpret_cast<const ulonglong2*>(buf + i * TILE4), mm[0], mm[1], pv[0], pv[1]);
             ++scanned;
             __syncwarp();                                                      // read before it is fetched over
         };
@@ -380,16 +382,17 @@ __global__ void __launch_bounds__(MATCH_THREADS, N <= 12 ? 4 : N <= 24 ? 3 : 2) 
         }
         fetch(t0);
         scan();
+        if (ix.test_stall && !tile_wait(&never, 0, STALL_POLLS)) stuck = true;
         // ---- every other tile some voxel still needs (this warp's share), one
         // in flight while the one before is scanned ----
         unsigned share = 0xffffffffu;
         if (WARPS > 1) share = (0x11111111u * ((1u << (4 / WARPS)) - 1u)) << (part * (4 / WARPS));
-        for (int base = 0; base < ix.n_tiles; base += 32) {
+        for (int base = 0; base < ix.n_tiles && !stuck; base += 32) {
             const float top = warp_maxf32(fmaxf(pv[0].limit, pv[1].limit));
             const int mine = base + lane;
             bool want = false;
             if (mine < ix.n_tiles && mine != t0) want = !(0.998f * box_distance2(boxes + 4ll * mine, glo, ghi) > top);
-            for (unsigned mask = __ballot_sync(MADI_FULL, want) & share; mask; mask &= mask - 1) {
+            for (unsigned mask = __ballot_sync(MADI_FULL, want) & share; mask && !stuck; mask &= mask - 1) {
                 const int t = base + __ffs(mask) - 1;
                 const float4* b = boxes + 4ll * t;
                 const bool need = !(0.998f * box_distance2(b, phi[0], phi[0]) > pv[0].limit) ||
@@ -399,10 +402,17 @@ __global__ void __launch_bounds__(MATCH_THREADS, N <= 12 ? 4 : N <= 24 ? 3 : 2) 
                 if (fetched - scanned == 2) scan();
             }
         }
-        while (fetched != scanned) scan();
-        // a copy that never completed (not seen; the wait is bounded): no result
-        // is better than a wrong one
-        if (stuck) pv[0].bj = pv[1].bj = -1;
+        while (fetched != scanned && !stuck) scan();
+        // a copy that did not complete in time (not seen; the waits are bounded): no
+        // result is better than a wrong one.  The copies in flight are waited for
+        // again, so that none lands in the next CTA's memory, and the call's status
+        // says so (2: this wait ran out too).
+        if (stuck) {
+            pv[0].bj = pv[1].bj = -1;
+            bool drained = true;
+            for (; fetched != scanned; ++scanned) drained = tile_wait(&bars[warp][scanned & 1], (scanned >> 1) & 1) && drained;
+            if (lane == 0) atomicMax(ix.status, drained ? 1 : 2);
+        }
     }
     if (WARPS > 1) {
         const int g = warp / WARPS;
@@ -421,7 +431,11 @@ __global__ void __launch_bounds__(MATCH_THREADS, N <= 12 ? 4 : N <= 24 ? 3 : 2) 
 #pragma unroll
     for (int i = 0; i < 2; ++i)
         if (p0 + 32 * i + lane < ix.n_vox) {
-            if (pv[i].bj < 0) best_idx[vox[i]] = -1;
+            if (pv[i].bj < 0) {
+                best_idx[vox[i]] = -1;
+                best_resid[vox[i]] = __int_as_float(0x7fc00000);
+                if (MODE == MADI_MATCH_FREE_S0 && best_s0) best_s0[vox[i]] = __int_as_float(0x7fc00000);
+            }
             else match_write<N, MODE>(meas, lib, vox[i], pv[i].bj, ix.F, best_idx, best_resid, best_s0);
         }
 }
@@ -478,6 +492,7 @@ static madi_status launch_fp32(const madi_match_desc* d, const MatchPlan& p, flo
         prune::layout(ix, scratch, d->n_vox, d->n_lib, d->n_feat);
         ix.mu = MODE == MADI_MATCH_FIXED_S0 ? mu : nullptr;
         ix.free_s0 = MODE == MADI_MATCH_FREE_S0;
+        ix.test_stall = (d->flags & MADI_MATCH_FLAG_TEST_STALL) != 0;
         const madi_status st = prune::build(ix, d->measured, d->lib, true, s);
         if (st != MADI_OK) return st;
         // Warps a group: more shorten the longest group's chain of tiles while the
@@ -547,6 +562,18 @@ extern "C" int64_t madi_match_scratch_bytes(int64_t n_vox, int32_t n_lib, int32_
     return FP32_SCRATCH + match_plan(n_vox, n_lib, n_feat).bytes;
 }
 
+// The route of an fp32 call and the scratch behind the column means it uses.
+static MatchPlan fp32_route(const madi_match_desc* d, unsigned char*& scratch) {
+    const MatchPlan plan = match_plan(d->n_vox, d->n_lib, d->n_feat);
+    const bool ours = d->mode == MADI_MATCH_FIXED_S0 || (d->flags & MADI_MATCH_FLAG_SCRATCH);
+    if (ours && d->scratch && (reinterpret_cast<uintptr_t>(d->scratch) & 255) == 0 &&
+        d->scratch_bytes >= FP32_SCRATCH + plan.bytes) {
+        scratch = static_cast<unsigned char*>(d->scratch) + FP32_SCRATCH;
+        return plan;
+    }
+    return MatchPlan{false, 1, d->n_lib, 0};                // no scratch, or it holds the column means only
+}
+
 extern "C" madi_status madi_match(const madi_match_desc* d, void* stream) {
     host::clear_error();
     if (!d || !d->measured || !d->lib || !d->best_idx || !d->best_resid || d->n_vox < 0 || d->n_lib < 1 ||
@@ -569,14 +596,8 @@ extern "C" madi_status madi_match(const madi_match_desc* d, void* stream) {
         mu = static_cast<float*>(d->scratch);
         madi_match_column_mean(d->lib, d->n_lib, d->n_feat, mu, s);
     }
-    MatchPlan plan = match_plan(d->n_vox, d->n_lib, d->n_feat);
     unsigned char* scratch = nullptr;
-    const bool ours = d->mode == MADI_MATCH_FIXED_S0 || (d->flags & MADI_MATCH_FLAG_SCRATCH);
-    if (ours && d->scratch && (reinterpret_cast<uintptr_t>(d->scratch) & 255) == 0 &&
-        d->scratch_bytes >= FP32_SCRATCH + plan.bytes)
-        scratch = static_cast<unsigned char*>(d->scratch) + FP32_SCRATCH;
-    else
-        plan = MatchPlan{false, 1, d->n_lib, 0};            // no scratch, or it holds the column means only
+    const MatchPlan plan = fp32_route(d, scratch);
     return d->mode == MADI_MATCH_FIXED_S0 ? launch_fp32_mode<MADI_MATCH_FIXED_S0>(d, plan, mu, scratch, s)
                                           : launch_fp32_mode<MADI_MATCH_FREE_S0>(d, plan, mu, scratch, s);
 }
@@ -585,6 +606,22 @@ extern "C" madi_status madi_match_wait(const madi_match_desc* d, void* stream) {
     host::clear_error();
     if (!d) return host::fail(MADI_ERR_INVALID, "match_wait: null descriptor");
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+    if (d->precision == MADI_MATCH_FP32 && d->n_vox > 0 && d->n_lib > 0 && d->n_feat > 0 && d->n_feat <= 32) {
+        unsigned char* scratch = nullptr;
+        if (fp32_route(d, scratch).pruned) {
+            prune::Index ix;
+            prune::layout(ix, scratch, d->n_vox, d->n_lib, d->n_feat);
+            int word = 0;
+            cudaError_t e = cudaMemcpyAsync(&word, ix.status, sizeof(int), cudaMemcpyDeviceToHost, s);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+            if (e != cudaSuccess) return host::cuda_fail(e, "match_wait: stream");
+            if (word != 0)
+                return host::fail(MADI_ERR_TIMEOUT, "match fp32: a bounded wait ran out; the voxels of the warps that gave up "
+                                                    "have index -1 (%s)",
+                                  word == 1 ? "issued copies were drained" : "and the drain of the issued copies ran out");
+            return MADI_OK;
+        }
+    }
     cudaError_t e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return host::cuda_fail(e, "match_wait: stream");
     if (d->precision != MADI_MATCH_BF16 || d->n_vox == 0) return MADI_OK;

@@ -36,6 +36,7 @@ struct Index {
     const float* mu;            // [32] subtracted from the row (fixed S0), or null
     float* basis;               // [KDIR][32] directions, [32] centre of unit rows (free S0), ranges
     float* lmax;                // largest |row|^2; free S0: then the largest 1 / max(|row|^2, 1e-30)
+    int* status;                // 0, or a bounded wait of the search ran out (match.cu)
     uint32_t* bins;             // [LIB_BINS + VOX_BINS]
     uint32_t* lbin;             // [n_lib]
     uint32_t* vbin;             // [n_vox]
@@ -47,6 +48,7 @@ struct Index {
     int64_t n_vox;
     int n_lib, F, n_tiles, slabs, stride;
     int free_s0;
+    int test_stall;             // tests only: one wait that nothing completes
 };
 
 constexpr int B_CENTRE = KDIR * FMAX, B_RANGE = B_CENTRE + FMAX, B_FLOATS = B_RANGE + 16;
@@ -69,10 +71,12 @@ inline int64_t layout(Index& ix, unsigned char* base, int64_t n_vox, int32_t n_l
     ix.slabs = (int)std::min<double>(MAX_SLABS, std::max(4.0, 2.5 * std::sqrt((double)ix.n_tiles)));
     ix.mu = nullptr;
     ix.free_s0 = 0;
+    ix.test_stall = 0;
     ix.stride = row_stride(F);
     ix.basis = reinterpret_cast<float*>(take(B_FLOATS * 4));
     ix.bins = reinterpret_cast<uint32_t*>(take((LIB_BINS + VOX_BINS) * 4 + 256));
     ix.lmax = reinterpret_cast<float*>(ix.bins + LIB_BINS + VOX_BINS);      // zeroed with the bins
+    ix.status = reinterpret_cast<int*>(ix.lmax + 2);                        // so is the status
     ix.lbin = reinterpret_cast<uint32_t*>(take(4ll * n_lib));
     ix.vbin = reinterpret_cast<uint32_t*>(take(4ll * n_vox));
     ix.lperm = reinterpret_cast<int32_t*>(take(4ll * ix.n_tiles * TILE));

@@ -35,8 +35,8 @@ class MatchOutput(tuple):
     """(best_idx, best_resid, best_s0) device tensors of one madi_match call.
 
     ``check()`` waits for the call and raises ``MadiError`` (a RuntimeError,
-    status MADI_ERR_TIMEOUT) if a bounded wait of the tensor-core scan ran out;
-    the rows it could not finish keep -1 in best_idx.  The inputs and scratch
+    status MADI_ERR_TIMEOUT) if a bounded wait of the tensor-core scan or of the
+    indexed FP32 search ran out; the rows it could not finish have -1 in best_idx.  The inputs and scratch
     stay referenced until then.
     """
 
@@ -102,7 +102,7 @@ def match_device(measured, lib_mat, *, free_s0: bool = False, precision: str = "
 def _indices(idx) -> np.ndarray:
     b = idx.cpu().numpy().astype(np.int64)
     if np.any(b < 0):
-        raise RuntimeError("tensor-core library match gave up on a bounded wait; no result for some voxels")
+        raise RuntimeError("library match gave up on a bounded wait; no result for some voxels")
     return b
 
 

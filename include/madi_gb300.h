@@ -316,7 +316,8 @@ typedef struct madi_match_desc {
 /* Tests only: every CTA of the BF16 scan makes one bounded wait on a barrier
  * that nothing completes, so the timeout path runs (the CTA drains its issued
  * copies and MMAs, frees TMEM, leaves its rows at the caller's fill value) and
- * madi_match_wait reports MADI_ERR_TIMEOUT.  Nothing faults or hangs. */
+ * madi_match_wait reports MADI_ERR_TIMEOUT.  The indexed FP32 search does the
+ * same (index -1, NaN residual).  Nothing faults or hangs. */
 #define MADI_MATCH_FLAG_TEST_STALL 1
 /* BF16 fixed S0: scan every library tile for every voxel (no principal-axis
  * cut); the result is the same up to BF16 score ties at the k-th place. */
@@ -335,8 +336,10 @@ madi_status madi_match(const madi_match_desc* desc, void* stream);
  * returns MADI_OK; MADI_ERR_TIMEOUT if a bounded wait of the BF16 scan ran out
  * (the rows of the CTAs that gave up keep the value the caller left in
  * best_idx, e.g. -1; every issued copy and MMA was drained before TMEM was
- * freed, unless the message says the drain ran out too); MADI_ERR_CUDA if the
- * stream reports an error.  The FP32 scan has no bounded waits. */
+ * freed, unless the message says the drain ran out too) or one of the indexed
+ * FP32 search (best_idx -1, NaN residual and S0 for the voxels of the warps that
+ * gave up); MADI_ERR_CUDA if the stream reports an error.  The FP32 scans of
+ * every entry have no bounded waits. */
 madi_status madi_match_wait(const madi_match_desc* desc, void* stream);
 
 /* ------------------------------------------------------------------------ */
