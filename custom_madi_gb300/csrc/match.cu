@@ -59,10 +59,11 @@ MADI_DEV void match_write(const float* __restrict__ meas, const float* __restric
 // free S0 score_j = -(m.r)^2 / |r|^2 when m.r > 0.  The free score's division is
 // only made for pairs that may reach the best so far: dot^2 >= bar |r|^2, bar
 // 4e-7 below the best (the rounding on both sides is below 2e-7), 0 where the
-// best is subnormal or there is none.
+// best is subnormal or there is none.  An entry whose |r|^2 overflows (bar |r|^2
+// infinite, or NaN with the bar 0) is left to the score itself.
 MADI_DEV float free_bar(float best) { return best < -1e-36f ? -best * (1.f - 4e-7f) : 0.f; }
 MADI_DEV bool free_may_win(float dot, float sn, float bar) {
-    return dot > 0.f && fmaxf(dot * dot, 1e-36f) >= bar * sn;
+    return dot > 0.f && !(fmaxf(dot * dot, 1e-36f) < bar * sn);
 }
 
 template <int MODE>
