@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(THREADS) bayes_kernel(const __grid_constant__ 
         }
         const float lmax = P.ix.lmax[0];
         const bool ok = FREE ? m2 < 1e30f && m2 * lmax < 1e30f && m2 > 1e-25f * P.ix.lmax[1] && P.ix.lmax[1] < 1e20f
-                             : m2 + lmax < 1e30f;
+                             : m2 + lmax < 1e30f && m2 + lmax > 1e-30f;
         bounded = __all_sync(MADI_FULL, ok);
 #pragma unroll
         for (int k = 0; k < 6; ++k) {

@@ -187,9 +187,10 @@ __global__ void __launch_bounds__(256) match_finish_kernel(const float* __restri
 // the directions are orthonormal to 1e-5: 0.998 d^2 and the margin E = (F + 8)
 // 2^-21 (|m|^2 + max |L|^2) cover them together ((a + b)^2 <= 1.001 a^2 + 1001
 // b^2).  A tile is skipped only if the bound lies strictly above the best score,
-// so ties keep the lowest index.  Where fp32 scores can overflow, or the free
-// score's dot^2 become subnormal, the bound says nothing: those voxels (and ones
-// that are not finite) skip nothing.
+// so ties keep the lowest index.  Where fp32 scores can overflow or the terms of
+// the bounds become subnormal (rounded by an absolute amount, which no relative
+// margin covers), the bound says nothing: those voxels (and ones that are not
+// finite) skip nothing.
 // ---------------------------------------------------------------------------
 struct PrunedVoxel {
     float m2, e, limit, best;
@@ -326,7 +327,7 @@ __global__ void __launch_bounds__(MATCH_THREADS, N <= 12 ? 4 : N <= 24 ? 3 : 2) 
             if (MODE == MADI_MATCH_FIXED_S0) {
                 e = prune::embed(m, sv);
                 v.e = slack * (v.m2 + lmax);
-                v.bounded = v.m2 + lmax < 1e36f;
+                v.bounded = v.m2 + lmax < 1e36f && v.m2 + lmax > 1e-30f;
             } else {
                 float u[N];
                 const float sc = v.m2 > 0.f ? rsqrtf(v.m2) : 0.f;
@@ -334,7 +335,7 @@ __global__ void __launch_bounds__(MATCH_THREADS, N <= 12 ? 4 : N <= 24 ? 3 : 2) 
                 for (int f = 0; f < N; ++f) u[f] = f < ix.F ? fmaf(m[f], sc, -sv[prune::B_CENTRE + f]) : 0.f;
                 e = prune::embed(u, sv);
                 v.e = slack;
-                v.bounded = v.m2 < 1e36f && v.m2 * lmax < 1e36f && v.m2 > 1e-32f * inv_lmin;
+                v.bounded = v.m2 < 1e36f && v.m2 * lmax < 1e36f && v.m2 > 1e-32f * inv_lmin && inv_lmin < 1e25f;
             }
 #pragma unroll
             for (int k = 0; k < prune::KDIR; ++k) phi[i][k] = e.p[k];
