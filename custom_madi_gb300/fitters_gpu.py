@@ -31,6 +31,20 @@ def _as_dev(x):
     return torch.from_numpy(np.ascontiguousarray(x, dtype=np.float32)).cuda()
 
 
+def _side_stream(stream, device):
+    """``stream`` as a torch stream if it is not the current one, ordered after the
+    work enqueued there (the call's buffers are made on it); else None."""
+    cur = torch.cuda.current_stream(device)
+    if stream is None or stream.cuda_stream == cur.cuda_stream:
+        return None
+    s = stream if isinstance(stream, torch.cuda.Stream) else torch.cuda.ExternalStream(stream.cuda_stream, device=device)
+    with torch.cuda.stream(s):
+        capturing = torch.cuda.is_current_stream_capturing()
+    if not capturing:               # a capture cannot wait for work outside it
+        s.wait_stream(cur)
+    return s
+
+
 class MatchOutput(tuple):
     """(best_idx, best_resid, best_s0) device tensors of one madi_match call.
 
@@ -58,6 +72,7 @@ def match_device(measured, lib_mat, *, free_s0: bool = False, precision: str = "
     ``check=True`` waits for the result and raises if the scan could not
     finish (see ``MatchOutput.check``); ``check=False`` returns as soon as the
     work is enqueued on ``stream`` and the caller calls ``.check()`` later.
+    The work on ``stream`` is ordered after what the current stream holds.
     ``flags``: MADI_MATCH_FLAG_FULL_SCAN (BF16 fixed S0 without the
     principal-axis scan cut; same result up to BF16 score ties at the k-th
     place) or, for tests, MADI_MATCH_FLAG_TEST_STALL.
@@ -93,7 +108,12 @@ def match_device(measured, lib_mat, *, free_s0: bool = False, precision: str = "
     else:
         d.scratch, d.scratch_bytes = 0, 0
     s = stream if stream is not None else torch.cuda.current_stream(M.device)
+    side = _side_stream(stream, M.device)
     st = N.lib().madi_match(C.byref(d), s.cuda_stream)
+    if side is not None:            # freed, the memory is not used again before `stream` is done with it
+        for t in (M, Lm, idx, res, s0, scratch):
+            if t is not None:
+                t.record_stream(side)
     N.check(st, "madi_match")
     out = MatchOutput(idx, res, s0, d, s, (M, Lm, scratch))
     return out.check() if check else out
@@ -164,9 +184,10 @@ def bayes_fit_gpu(measured_batch, lib_mat, kios_arr, rhos_arr, Vs_arr, sigma_m, 
     base = N.ptr(scratch)
     pad = (-base) % 256
     d.scratch, d.scratch_bytes = base + pad, int(scratch.numel()) - pad
-    s = stream if stream is not None else torch.cuda.current_stream(dev)
-    N.check(N.lib().madi_bayes(C.byref(d), s.cuda_stream), "madi_bayes")
-    o = out.cpu().numpy()
+    s = _side_stream(stream, dev) or torch.cuda.current_stream(dev)
+    with torch.cuda.stream(s):
+        N.check(N.lib().madi_bayes(C.byref(d), s.cuda_stream), "madi_bayes")
+        o = out.cpu().numpy()       # on the fit's stream: it is done before the buffers are freed
     res = dict(kio_mean=o[0], rho_mean=o[1], V_mean=o[2], kio_std=o[3], rho_std=o[4], V_std=o[5],
                residual=o[6], n_eff=o[7])
     if fit_s0:
