@@ -120,14 +120,17 @@ MADI_DEV Geo make_geo(const madi_geometry& g, const unsigned char* base) {
     v.cerr = (float)g.coord_err;
     v.n_seeds = g.n_seeds;
     v.ccen = reinterpret_cast<const float4*>(base + g.off_cell_center);
-    v.fstride = (int)g.facet_stride;
+    v.fstride = (int)(g.facet_stride & ~MADI_FACETS_ORDERED);
     v.fpl = reinterpret_cast<const float4*>(base + g.off_facet_plane);
     v.fnbr = reinterpret_cast<const int32_t*>(base + g.off_facet_nbr);
     v.n_cells = g.n_cells;
     v.ftol = (float)g.facet_tol;
-    v.sorted = g.alpha_min > 0.f;
+    v.sorted = (g.facet_stride & MADI_FACETS_ORDERED) != 0;
     return v;
 }
+
+// A lower bound of every cell's alpha, 0 where the caller gives none.
+MADI_DEV float alpha_bound(const madi_geometry& g) { return (g.facet_stride & MADI_FACETS_ORDERED) ? g.alpha_min : 0.f; }
 
 MADI_DEV int cand_id(const Geo& g, uint32_t k) {
     return g.ids_u32 ? (int)reinterpret_cast<const uint32_t*>(g.ids)[k]

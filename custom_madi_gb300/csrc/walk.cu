@@ -425,7 +425,7 @@ __device__ __forceinline__ void walk_tile(const madi_walk_desc& d, const madi_wa
     // error bound of any facet margin in the box (|w|_1 <= 3 L)
     float t_any = fmaf(6.0f * MADI_EPS21, L, (float)gd.facet_tol);
     asm volatile("" : "+f"(t_any));
-    const float a_min = gd.alpha_min;
+    const float a_min = alpha_bound(gd);
     float gv[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     uint32_t acc_word = 0, acc_word_odd = 0;
     int h_left = d.steps_per_h;
@@ -803,7 +803,7 @@ __global__ void __launch_bounds__(F64_THREADS) walk_f64_kernel(const madi_walk_d
         }
     }
     const bool facets = cells && gd.n_cells > 0;
-    const float Lf = (float)L, a_min = gd.alpha_min;
+    const float Lf = (float)L, a_min = alpha_bound(gd);
     clear_cache(ts);
     int cell = 0, inside = 0, escaped = 0, cerr = 0;
     uint32_t n_acc = 0, n_rej = 0, n_full = 0;

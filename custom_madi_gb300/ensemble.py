@@ -476,7 +476,7 @@ class DeviceGeometry:
         s.source_hi = float(ens.source_hi)
         s.coord_err = self.coord_err
         s.off_cell_center, s.off_facet_plane, s.off_facet_nbr = (int(o) for o in offs[4:7])
-        s.facet_stride = self.facet_stride
+        s.facet_stride = self.facet_stride | (N.MADI_FACETS_ORDERED if n_cells > 0 else 0)
         s.n_cells = n_cells
         s.facet_tol = self.facet_tol
         # rounded down: a lower bound of every fp64 annulus

@@ -64,6 +64,12 @@ enum { MADI_BOUNDARY_FATAL = 0, MADI_BOUNDARY_PERIODIC = 1 };
  * contracted cell boundary: a proven superset, so the fp32 and fp64 rules run
  * on these lists return the labels of the all-seed rule.
  */
+
+/* Set in madi_geometry.facet_stride: each cell's slots are in ascending order of h
+ * (as madi_facets_build writes them) and alpha_min holds its bound.  Without it
+ * alpha_min is not read and the walker reads every slot of a cell. */
+#define MADI_FACETS_ORDERED 0x80000000u
+
 typedef struct madi_geometry {
     const void*    stage;          /* device, 16-byte aligned                     */
     const double*  seed_f64;       /* device, [n_seeds][4]                        */
@@ -93,13 +99,12 @@ typedef struct madi_geometry {
      * (0, 0, 0, 3e38) and neighbour -1.  With n_cells = 0 the walker labels
      * every step with the voxel-grid classifier. */
     uint32_t off_cell_center;      /* float4 [n_cells]: base seed x, y, z, alpha  */
-    uint32_t facet_stride;         /* facet slots per cell, a multiple of 32      */
+    uint32_t facet_stride;         /* facet slots per cell, a multiple of 32, and
+                                    * MADI_FACETS_ORDERED                         */
     uint32_t off_facet_plane;      /* float4 [n_cells][facet_stride]: n, offset h */
     uint32_t off_facet_nbr;        /* int32 [n_cells][facet_stride]: cell across  */
     int32_t  n_cells;              /* cells in the table (0 = no table)           */
-    float    alpha_min;            /* > 0: <= every cell's alpha, and each cell's slots
-                                    * are in ascending order of h (as madi_facets_build
-                                    * writes them); 0: neither is promised           */
+    float    alpha_min;            /* <= every cell's alpha (with MADI_FACETS_ORDERED) */
     double   facet_tol;            /* fp32 error of h - n.w, without the |w| term */
 } madi_geometry;
 
