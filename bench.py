@@ -417,7 +417,7 @@ def plain_and_served(dev, cfg, jobs, lay, dirs, batched_rate, batch):
     from custom_madi_gb300.walker_gpu import LaunchConfig, WalkBatch
     out = {"entries": len(jobs), "walkers_per_entry": int(jobs[0].n_walkers), "batched_walker_steps_per_s": batched_rate}
     host = [_host_geometry(j.ensemble, dev) for j in jobs]
-    plain_lc = LaunchConfig(tile_walkers=128, persistent=False)
+    plain_lc = LaunchConfig(tile_walkers=128, persistent=False, alone=True)
     # warm-up on one entry
     WalkBatch([jobs[0]], cfg, layout=lay, dirs=dirs, launch=plain_lc, device=dev).launch()
     torch.cuda.synchronize(dev)
@@ -660,7 +660,7 @@ def mixed_leg(dev, lib, threads, chunk_walkers=262_144, launch_walkers=622_592, 
     sim_span = max(r.finish for r in sims)
     rate = out["walker_steps"] / sim_span
     # plain path on the same entries (same walkers: matched Monte Carlo error)
-    plain_lc = LaunchConfig(tile_walkers=128, persistent=False)
+    plain_lc = LaunchConfig(tile_walkers=128, persistent=False, alone=True)
     sub = [WalkJob(r.ensemble, r.pp, r.seed, r.n_walkers) for r in reqs if isinstance(r, SimRequest)]
     WalkBatch([sub[0]], cfg, layout=lay, dirs=dirs, launch=plain_lc, device=dev).launch()
     torch.cuda.synchronize(dev)

@@ -40,6 +40,7 @@ MADI_MATCH_FLAG_TEST_STALL = 1
 MADI_MATCH_FLAG_FULL_SCAN = 2
 MADI_MATCH_FLAG_SCRATCH = 4
 MADI_FACETS_ORDERED = 0x80000000
+MADI_WALK_ALONE = 256
 
 CNT_NAMES = ("walkers", "escaped", "classifier_error", "full", "tier1", "fallback64",
              "cross_accept", "cross_reject", "facet_pass")

@@ -1169,23 +1169,33 @@ static int64_t fused_smem(const madi_walk_desc* d, int np, int threads) {
            (24 + FC_BYTES_PER_WALKER + 4 * (3 + 3 * np) + 12) * threads;
 }
 
-// Walkers of a launch that leaves the chip idle go 16 or 8 to a warp.  A step is a
+// Walkers of a launch that leaves the chip idle go 16 or 8 to a warp where the
+// caller says that the launch has it to itself (MADI_WALK_ALONE).  A step is a
 // chain of ~2,200 cycles for a warp alone on its scheduler: 416 of them draw the
 // random numbers, which the free lanes then do for later steps (2 or 4 pairs at
 // once), and ~700 are facet passes, taken if any lane of the warp misses its cache:
 // fewer lanes, fewer passes.  10,000 walkers x 4,600 steps in a 64-cell box, 32 / 16
-// / 8 to a warp: 5.98 / 5.38 / 4.94 ms; 1,000: 5.76 / 5.03 / 4.46; 20,000: 6.33 /
-// 5.87 / -.  The line is one wave of the CTAs an SM holds: past it
-// the second wave costs more than it saves (40,000 walkers: 7.0 / 11.3 ms).
+// / 8 to a warp: 5.85 / 5.24 / 4.84 ms; 1,000: 5.80 / 5.03 / 4.42.
+//
+// The line is half a wave of the CTAs an SM holds.  Past one wave the second costs
+// more than this saves (40,000 walkers: 7.0 / 11.3 ms), and a walk that comes along
+// after all needs room: two launches of 20,000, the first in a full wave of its own,
+// take 12.6 ms, both 32 to a warp 7.1 ms.  Two launches that both took lane groups
+// unasked made 9.3 ms of what 32 to a warp do in 6.3 (10,000 walkers each), eight
+// 27.7 ms of 12.8.
 constexpr int SPREAD_CTAS = 3;                   // resident on an SM: 168 registers a thread, no spills
+static bool walk_alone(const madi_walk_desc* d) { return d->min_blocks > 0 && (d->min_blocks & MADI_WALK_ALONE); }
+static bool two_blocks(const madi_walk_desc* d) { return d->min_blocks - (walk_alone(d) ? MADI_WALK_ALONE : 0) >= 2; }
+
 static int spread_of(const madi_walk_desc* d, int64_t smem) {
+    if (!walk_alone(d)) return 0;
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return 0;
     const int64_t ctas = sms * std::min<int64_t>(SPREAD_CTAS, 227 * 1024 / (smem + 1024));
     for (int spread = 2; spread > 0; --spread) {
         const int64_t threads = (int64_t)d->n_tiles * d->tile_walkers << spread;
-        if (((d->tile_walkers << spread) % SPREAD_THREADS) == 0 && threads <= ctas * SPREAD_THREADS) return spread;
+        if (((d->tile_walkers << spread) % SPREAD_THREADS) == 0 && 2 * threads <= ctas * SPREAD_THREADS) return spread;
     }
     return 0;
 }
@@ -1197,6 +1207,13 @@ static madi_status launch_f32(const madi_walk_desc* d, int spread, cudaStream_t 
     const int64_t sm = fused_smem(d, NP, threads);
     if (sm > 227 * 1024) return host::fail(MADI_ERR_CAPACITY, "walker shared memory %lld B exceeds 227 KB", (long long)sm);
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (SPREAD && e == cudaSuccess) {
+        // as much shared memory an SM as four CTAs of a launch without lane groups
+        // need: with less, such a launch waits for this one's SMs to drain before it
+        // gets any (10,000 walkers beside 10,000 of these: 12.3 ms, 6.9 ms so)
+        const int64_t percent = (4 * (sm + 1024) * 100 + 228 * 1024 - 1) / (228 * 1024);
+        e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, (int)std::min<int64_t>(percent, 100));
+    }
     if (e != cudaSuccess) return host::cuda_fail(e, "cudaFuncSetAttribute(walker)");
     const int parts = SPREAD ? (d->tile_walkers << spread) / SPREAD_THREADS : 1;
     const int blocks = (d->grid_blocks > 0 ? d->grid_blocks : d->n_tiles) * parts;
@@ -1210,7 +1227,7 @@ template <int OUT, bool PER, int NP>
 static madi_status launch_spread(const madi_walk_desc* d, cudaStream_t s) {
     const int spread = spread_of(d, fused_smem(d, NP, SPREAD_THREADS));
     if (spread) return launch_f32<OUT, PER, NP, SPREAD_CTAS, true>(d, spread, s);
-    return d->min_blocks >= 2 ? launch_f32<OUT, PER, NP, 2, false>(d, 0, s) : launch_f32<OUT, PER, NP, 1, false>(d, 0, s);
+    return two_blocks(d) ? launch_f32<OUT, PER, NP, 2, false>(d, 0, s) : launch_f32<OUT, PER, NP, 1, false>(d, 0, s);
 }
 
 template <int OUT, bool PER>
@@ -1221,7 +1238,7 @@ static madi_status launch_np(const madi_walk_desc* d, cudaStream_t s) {
 
 template <int OUT, bool PER>
 static const void* kernel_for(const madi_walk_desc* d) {
-    const bool two = d->min_blocks >= 2;
+    const bool two = two_blocks(d);
     if (OUT == MADI_OUT_FUSED && d->n_pairs > 4)
         return two ? (const void*)walk_f32_kernel<OUT, PER, 8, 2, false> : (const void*)walk_f32_kernel<OUT, PER, 8, 1, false>;
     return two ? (const void*)walk_f32_kernel<OUT, PER, 4, 2, false> : (const void*)walk_f32_kernel<OUT, PER, 4, 1, false>;

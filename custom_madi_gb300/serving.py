@@ -33,7 +33,7 @@ import numpy as np
 
 from . import _native as N
 from .config import SimConfig
-from .walker_gpu import FIXED_POINT_SCALE, LaunchConfig, PairLayout, WalkBatch, WalkJob
+from .walker_gpu import FIXED_POINT_SCALE, LaunchConfig, PairLayout, WalkBatch, WalkJob, walk_in_flight
 
 try:
     import torch
@@ -230,6 +230,10 @@ class Server:
     def run(self, requests: Sequence, *, realtime: bool = True, poll_s: float = 2e-4) -> Dict[str, Any]:
         """Serve ``requests`` (arrival times relative to the start); returns per-request records
         and the run's latency and throughput statistics."""
+        with walk_in_flight():
+            return self._run(requests, realtime, poll_s)
+
+    def _run(self, requests: Sequence, realtime: bool, poll_s: float) -> Dict[str, Any]:
         order = sorted(range(len(requests)), key=lambda i: requests[i].arrival)
         recs = {i: Record(i, "sim" if isinstance(requests[i], SimRequest) else "fit", float(requests[i].arrival),
                           self._nbytes(requests[i])) for i in order}
@@ -421,6 +425,10 @@ class NativeSimServer:
                 "counters": dict(zip(N.CNT_NAMES, self.counters[slot].cpu().numpy().tolist()))}
 
     def run(self, requests: Sequence[SimRequest], *, realtime: bool = True, poll_s: float = 2e-4) -> Dict[str, Any]:
+        with walk_in_flight():
+            return self._run(requests, realtime, poll_s)
+
+    def _run(self, requests: Sequence[SimRequest], realtime: bool, poll_s: float) -> Dict[str, Any]:
         C = self._C
         torch.cuda.synchronize(self.dev)       # pools and geometry ready before the native streams start
         order = sorted(range(len(requests)), key=lambda i: requests[i].arrival)

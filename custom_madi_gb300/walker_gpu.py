@@ -15,6 +15,8 @@ from __future__ import annotations
 import ctypes as C
 import math
 import sys
+import threading
+from contextlib import contextmanager
 from dataclasses import dataclass, field, replace
 from typing import Optional, Sequence, Tuple
 
@@ -243,6 +245,28 @@ class LaunchConfig:
     staged: Optional[bool] = None   # False = always read geometry in place
     stage_budget: int = 48 * 1024   # largest geometry staged into shared memory
     min_blocks: int = 2             # register budget: 2 -> 128 registers/thread, 1 -> 255
+    alone: bool = False             # no other walk shares the GPU meanwhile: small launches may take more of it
+
+
+_walks = 0                          # walks of this process that are being waited for, and running servers
+_walks_lock = threading.Lock()
+
+
+@contextmanager
+def walk_in_flight():
+    """Counts a walk while its caller waits for it; yields True if it is the only one.
+
+    The synchronous entry points launch with ``alone`` then.  A later walk finds this
+    one counted and launches without; the results are the same either way."""
+    global _walks
+    with _walks_lock:
+        _walks += 1
+        only = _walks == 1
+    try:
+        yield only
+    finally:
+        with _walks_lock:
+            _walks -= 1
 
 
 class WalkBatch:
@@ -311,7 +335,7 @@ class WalkBatch:
         d.out_mode = out_mode
         d.n_steps, d.steps_per_h, d.n_grid = cfg.n_steps, cfg.steps_per_h, cfg.n_grid
         d.sigma, d.ts = cfg.sigma, cfg.ts
-        d.min_blocks = int(lc.min_blocks)
+        d.min_blocks = int(lc.min_blocks) + (N.MADI_WALK_ALONE if lc.alone else 0)
         u = np.eye(3) if dirs is None else np.asarray(dirs, np.float64)
         self.n_dirs = len(u)
         self.layout = layout
@@ -442,6 +466,11 @@ class WalkBatch:
         return out
 
 
+def _launch_alone(launch: Optional[LaunchConfig], only: bool) -> LaunchConfig:
+    lc = launch or LaunchConfig()
+    return replace(lc, alone=True) if only else lc
+
+
 def _raise_on_status(counters: dict, n: int) -> None:
     if counters.get("classifier_error", 0):
         raise RuntimeError("CUDA full-facet KD-tree classification failed")
@@ -470,10 +499,11 @@ def run_walk_Y(ens: Ensemble, kio: float, cfg: Optional[SimConfig] = None, seed:
     if random_stream is not None:
         random_stream.validate(cfg, ens)
     prec = precision or (64 if random_stream is not None else 32)
-    batch = WalkBatch([WalkJob(ens, actual_pp, int(seed), int(cfg.n_walkers))], cfg, out_mode=N.MADI_OUT_Y,
-                      stream=random_stream, precision=prec, launch=launch)
-    batch.launch()
-    torch.cuda.current_stream(batch.dev).synchronize()
+    with walk_in_flight() as only:
+        batch = WalkBatch([WalkJob(ens, actual_pp, int(seed), int(cfg.n_walkers))], cfg, out_mode=N.MADI_OUT_Y,
+                          stream=random_stream, precision=prec, launch=_launch_alone(launch, only))
+        batch.launch()
+        torch.cuda.current_stream(batch.dev).synchronize()
     res = batch.results()[0]
     cnt = res["counters"]
     Y = batch.Y.cpu().numpy()
@@ -537,6 +567,11 @@ def simulate_jobs(jobs: Sequence[WalkJob], cfg: SimConfig, columns: Tuple, *, di
     (madi/walker_gpu.py:520-695, :989-1063): per job one fp64 walk launch that
     stores Y, then a column reduction over the 3 Cartesian axes (sums [n_cols, 1]).
     """
+    with walk_in_flight() as only:
+        return _simulate_jobs(jobs, cfg, columns, dirs, _launch_alone(launch, only), check, precision)
+
+
+def _simulate_jobs(jobs, cfg, columns, dirs, launch, check, precision) -> list:
     _require_gpu(None)
     if precision not in (32, 64):
         raise ValueError("precision must be 32 or 64")

@@ -183,13 +183,19 @@ enum {
  * ceil(n_walkers / 128).
  * With MADI_RNG_PHILOX it evaluates the fp32 walker's Philox numbers in fp64.
  */
+
+/* Added to madi_walk_desc.min_blocks: no other walk shares the GPU while this one
+ * runs.  An fp32 launch too small for the GPU then puts fewer walkers in a warp and
+ * takes more CTAs: the same results sooner, but later for walks beside it. */
+#define MADI_WALK_ALONE 256
+
 typedef struct madi_walk_desc {
     const madi_geometry* geoms;    /* device array                                    */
     const madi_walk_job* jobs;     /* device array                                    */
     int32_t n_geoms, n_jobs;
     int32_t n_tiles;               /* total tiles over all jobs                       */
     int32_t tile_walkers;          /* walkers per tile (threads per block, but in launches
-                                      too small for the GPU: 128 threads there)       */
+                                      too small for the GPU with MADI_WALK_ALONE: 128) */
     int32_t grid_blocks;           /* persistent CTAs; 0 = one per tile               */
     int32_t stage_smem;            /* max stage_bytes over geoms; 0 = read in place   */
     int32_t boundary;              /* MADI_BOUNDARY_* shared by every geometry        */
@@ -201,7 +207,8 @@ typedef struct madi_walk_desc {
                                       refused (MADI_ERR_INVALID); a replay stream ignores it */
     /* fused epilogue */
     int32_t n_pairs, n_b, n_dirs;
-    int32_t min_blocks;            /* register budget: 1 = 255 regs, 2 = 128 regs/thread */
+    int32_t min_blocks;            /* register budget: 1 = 255 regs, 2 = 128 regs/thread,
+                                      plus MADI_WALK_ALONE                              */
     int32_t pair_jd[MADI_MAX_PAIRS], pair_jD[MADI_MAX_PAIRS], pair_js[MADI_MAX_PAIRS];
     float   coef[MADI_MAX_PAIRS * MADI_MAX_B];   /* phase coefficient per (pair, b)  */
     float   dirs[MADI_MAX_DIRS * 3];
