@@ -30,9 +30,10 @@
 //     32 voxels of a warp need the same entries;
 //   - a warp tests 32 entries at a time, one per lane, against the box of its
 //     voxels in the index's embedding and only visits those that can matter;
-//   - d is formed in pairs of floats (48 bits), then rounded to fp32 as before.
+//   - d is formed from three floats a parameter, which hold its 53 bits, and
+//     rounded to fp32 once as before.
 // The entries a voxel sums, and their order, are unchanged.  100,000 voxels x
-// 20,000 entries x 20 features, sigma_m 0.02: 33.2 ms before, 6.5 ms now (5.4 ms of it this
+// 20,000 entries x 20 features, sigma_m 0.02: 33.2 ms before, 7.0 ms now (5.9 ms of it this
 // kernel, bound by issue; the rest is the index and host copies).
 #include <cstdint>
 #include "madi_device.cuh"
@@ -77,25 +78,46 @@ struct Plan {
 };
 
 // One entry in shared memory: centred (fixed S0) or raw (free S0) row, raw row,
-// then |row|^2, log q, and kio, rho, V as hi + lo: (kio, rho) hi, (kio, rho) lo, V.
+// then |row|^2, log q, and kio, rho, V in three parts each: (kio, rho) high, middle,
+// low, V high, middle, low, 1 if one of them is not in parts (else 0).
 template <int N>
 struct Entry {
-    static constexpr int RAW = N, AUX = 2 * N, FLOATS = 2 * N + 8;
+    static constexpr int RAW = N, AUX = 2 * N, FLOATS = 2 * N + 12;
 };
 
-// x as hi + lo (48 bits).
-MADI_DEV float2 pair_of(double x) {
+// x = h + m + l exactly: h to 24 bits, m a multiple of 2^-46 of h's binade (so that
+// differences of two middles are exact wherever the highs are near each other), l the
+// rest, <= 7 bits.  `out`: x is outside the range where all three are exact.
+struct Parts { float h, m, l; };
+MADI_DEV Parts parts_of(double x, bool& out) {
     const float h = (float)x;
-    return make_float2(h, isfinite(h) ? (float)(x - (double)h) : 0.f);
+    if (!(fabsf(h) >= 1e-28f && fabsf(h) <= 3.4e38f)) {
+        out |= x != 0.0;
+        return Parts{0.f, 0.f, 0.f};
+    }
+    const double r = x - (double)h;
+    const float grid = __int_as_float(((__float_as_int(h) & 0x7f800000) - (23 << 23)) | 0x400000);       // 1.5 2^(E - 23)
+    const float m = __fadd_rn(__fadd_rn((float)r, grid), -grid);
+    return Parts{h, m, (float)(r - (double)m)};
 }
 
-// Differences ah + al - (bh + bl) of two values at a time, rounded to fp32.
-MADI_DEV uint64_t pair_diff(uint64_t ah, uint64_t al, uint64_t bh, uint64_t bl) {
+// Differences a - b of two values at a time, rounded to fp32 once: where the highs
+// are near, s, m, l and s + m are exact; elsewhere e and g are the errors of s and p.
+// (Two floats a value hold 48 bits: for parameters that agree to 2^-25 the
+// difference was short of bits.  100,000 voxels x 20,000 entries x 20: 6.4 ms a fit
+// with two, 7.0 ms with three.)
+MADI_DEV uint64_t parts_diff(uint64_t ah, uint64_t am, uint64_t al, uint64_t bh, uint64_t bm, uint64_t bl) {
     const uint64_t s = sub2(ah, bh);
     const uint64_t t = sub2(s, ah);
-    const uint64_t e = sub2(sub2(ah, sub2(s, t)), add2(bh, t));      // exact error of s
-    return add2(s, add2(e, sub2(al, bl)));
+    const uint64_t e = sub2(sub2(ah, sub2(s, t)), add2(bh, t));
+    const uint64_t m = sub2(am, bm);
+    const uint64_t p = add2(s, m);
+    const uint64_t g = sub2(m, sub2(p, s));
+    return add2(p, add2(add2(e, g), sub2(al, bl)));
 }
+
+// The same in fp64, from memory; a call of its own so that nothing of it is done ahead.
+__device__ __noinline__ float diff_f64(const double* a, double b) { return (float)(*a - b); }
 
 // Screened log-weight of one entry from the fp32 score, and its error bound.
 // The error bound counts FERR features (the row rounded up to a multiple of 8).
@@ -192,8 +214,10 @@ MADI_DEV void make_entry(const Plan& P, int64_t e, const float* smu, float* o) {
     float* a = o + Entry<N>::AUX;
     a[0] = FREE ? fmaxf(sn, 1e-30f) : sn;
     a[1] = (float)P.logq[e];
-    const float2 k = pair_of(P.kio[e]), r = pair_of(P.rho[e]), v = pair_of(P.V[e]);
-    a[2] = k.x; a[3] = r.x; a[4] = k.y; a[5] = r.y; a[6] = v.x; a[7] = v.y;
+    bool out = false;
+    const Parts k = parts_of(P.kio[e], out), r = parts_of(P.rho[e], out), v = parts_of(P.V[e], out);
+    a[2] = k.h; a[3] = r.h; a[4] = k.m; a[5] = r.m; a[6] = k.l; a[7] = r.l;
+    a[8] = v.h; a[9] = v.m; a[10] = v.l; a[11] = out ? 1.f : 0.f;
 }
 
 // The library in the staged form, and (|row|^2, log q) beside its embedding.
@@ -361,7 +385,9 @@ __global__ void __launch_bounds__(THREADS) bayes_kernel(const __grid_constant__ 
     // shift and centre from the exact residual of j*
     float S = 0.f;
     double x0[3] = {0.0, 0.0, 0.0};
-    uint64_t xh = 0, xl = 0, xv = 0, xvl = 0;                // (kio, rho) and V of j* as hi, lo
+    uint64_t xh = 0, xm = 0, xl = 0;                         // parts of (kio, rho) of j*
+    Parts xv{0.f, 0.f, 0.f};                                 // and of its V
+    bool x_out = false;
     bool any = bj >= 0;
     if (any) {
         float Lj[N];
@@ -373,11 +399,11 @@ __global__ void __launch_bounds__(THREADS) bayes_kernel(const __grid_constant__ 
         x0[0] = P.kio[bj];
         x0[1] = P.rho[bj];
         x0[2] = P.V[bj];
-        const float2 k = pair_of(x0[0]), r = pair_of(x0[1]), v3 = pair_of(x0[2]);
-        xh = pair2(k.x, r.x);
-        xl = pair2(k.y, r.y);
-        xv = pair2(v3.x, 0.f);
-        xvl = pair2(v3.y, 0.f);
+        const Parts k = parts_of(x0[0], x_out), r = parts_of(x0[1], x_out);
+        xh = pair2(k.h, r.h);
+        xm = pair2(k.m, r.m);
+        xl = pair2(k.l, r.l);
+        xv = parts_of(x0[2], x_out);
     }
     // ---- pass 2: exp-weighted sums over the entries above the cut ----
     // Sums in pairs: (w, w^2), (w resid, w s0), (w d_kio, w d_rho), (w d_V, w d_V^2),
@@ -392,11 +418,11 @@ __global__ void __launch_bounds__(THREADS) bayes_kernel(const __grid_constant__ 
               const float s = warp_minf(any ? S : 3.0e38f);
               return s - CUT - 1e-5f * fabsf(s);
           },
-          [&](int, const float* o0, int, const float* o1, bool two) {
+          [&](int e0, const float* o0, int e1, const float* o1, bool two) {
               float resid0, rw0, s00, resid1, rw1, s01;
               const bool fits0 = exact_staged<N, FREE>(mr, mr2, o0, resid0, rw0, s00) && any;
               const bool fits1 = exact_staged<N, FREE>(mr, mr2, o1, resid1, rw1, s01) && any && two;
-              auto add = [&](const float* a, float resid, float rw, float s0) {
+              auto add = [&](int entry, const float* a, float resid, float rw, float s0) {
                   float x = a[1] - rw * P.inv2s2 - S;
                   if (!(x > -CUT)) return;
                   if (x > 0.f) {
@@ -414,10 +440,15 @@ __global__ void __launch_bounds__(THREADS) bayes_kernel(const __grid_constant__ 
                   }
                   const float w = expf(x);
                   const uint64_t ww = pair2(w, w);
-                  const ulonglong2 kr = *reinterpret_cast<const ulonglong2*>(a + 4);     // (kio, rho) lo, V hi / lo
-                  const uint64_t d = pair_diff(*reinterpret_cast<const uint64_t*>(a + 2), kr.x, xh, xl);
-                  const float2 v3 = split2(kr.y);
-                  const float dv = split2(pair_diff(pair2(v3.x, 0.f), pair2(v3.y, 0.f), xv, xvl)).x;
+                  const ulonglong2 kr = *reinterpret_cast<const ulonglong2*>(a + 4);     // (kio, rho) middle, low
+                  const float4 v3 = *reinterpret_cast<const float4*>(a + 8);
+                  uint64_t d = parts_diff(*reinterpret_cast<const uint64_t*>(a + 2), kr.x, kr.y, xh, xm, xl);
+                  float dv = split2(parts_diff(pair2(v3.x, 0.f), pair2(v3.y, 0.f), pair2(v3.z, 0.f), pair2(xv.h, 0.f),
+                                               pair2(xv.m, 0.f), pair2(xv.l, 0.f))).x;
+                  if (v3.w != 0.f || x_out) {                  // a parameter that three floats do not hold
+                      d = pair2(diff_f64(P.kio + entry, x0[0]), diff_f64(P.rho + entry, x0[1]));
+                      dv = diff_f64(P.V + entry, x0[2]);
+                  }
                   WW.add(ww, pair2(1.f, w));
                   RS.add(ww, pair2(resid, FREE ? s0 : 0.f));
                   const uint64_t wd = mul2(ww, d);             // rounded: it serves both sums
@@ -426,8 +457,8 @@ __global__ void __launch_bounds__(THREADS) bayes_kernel(const __grid_constant__ 
                   D2.add(wd, d);
                   DV.add(pair2(wdv, wdv), pair2(1.f, dv));
               };
-              if (fits0) add(o0 + Entry<N>::AUX, resid0, rw0, s00);
-              if (fits1) add(o1 + Entry<N>::AUX, resid1, rw1, s01);
+              if (fits0) add(e0, o0 + Entry<N>::AUX, resid0, rw0, s00);
+              if (fits1) add(e1, o1 + Entry<N>::AUX, resid1, rw1, s01);
           });
     if (!live) return;
     const int64_t n = P.n_vox;
@@ -479,7 +510,7 @@ static madi_status launch_mode(const madi_bayes_desc* d, const Plan& P, bool ind
     }
 }
 
-static int entry_floats(int F) { return 2 * (F <= 8 ? 8 : F <= 16 ? 16 : F <= 20 ? 20 : F <= 24 ? 24 : 32) + 8; }
+static int entry_floats(int F) { return 2 * (F <= 8 ? 8 : F <= 16 ? 16 : F <= 20 ? 20 : F <= 24 ? 24 : 32) + 12; }
 
 }  // namespace bayes
 }  // namespace madi
