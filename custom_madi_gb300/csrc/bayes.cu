@@ -119,27 +119,22 @@ MADI_DEV uint64_t parts_diff(uint64_t ah, uint64_t am, uint64_t al, uint64_t bh,
 // The same in fp64, from memory; a call of its own so that nothing of it is done ahead.
 __device__ __noinline__ float diff_f64(const double* a, double b) { return (float)(*a - b); }
 
-// Screened log-weight of one entry from the fp32 score, and its error bound.
-// The error bound counts FERR features (the row rounded up to a multiple of 8).
-template <int FMAX, int FERR, bool FREE>
-MADI_DEV void screen(const float* m, const float* l, float sn, float lq, float m2, float inv2s2, float& e,
-                     float& err) {
+// Screened log-weight of one entry from the fp32 score.
+template <int FMAX, bool FREE>
+MADI_DEV float screen(const float* m, const float* l, float sn, float lq, float m2, float inv2s2) {
     float dot = 0.f;
 #pragma unroll
     for (int f = 0; f < FMAX; ++f) dot = fmaf(m[f], l[f], dot);
     if (!FREE) {
         // centred: r = |m~|^2 + |L~|^2 - 2 m~.L~ ; fp32 error <= (F + 4) 2^-23 (|m~|^2 + |L~|^2)
         const float r = fmaxf(fmaf(-2.f, dot, sn) + m2, 0.f);
-        e = lq - r * inv2s2;
-        err = ((float)(FERR + 4) * 1.2e-7f * (m2 + sn)) * inv2s2 + 1e-3f;
-    } else {
-        // rw = |L|^2 (|m|^2 |L|^2 / (m.L)^2 - 1) when m.L > 0
-        if (!(dot > 0.f)) { e = -3.0e38f; err = 0.f; return; }
-        const float ratio = m2 * sn / (dot * dot);
-        const float rw = fmaxf(sn * (ratio - 1.f), 0.f);
-        e = lq - rw * inv2s2;
-        err = (sn * ratio * (float)(FERR + 8) * 2.4e-7f) * inv2s2 + 1e-3f;
+        return lq - r * inv2s2;
     }
+    // rw = |L|^2 (|m|^2 |L|^2 / (m.L)^2 - 1) when m.L > 0
+    if (!(dot > 0.f)) return -3.0e38f;
+    const float ratio = m2 * sn / (dot * dot);
+    const float rw = fmaxf(sn * (ratio - 1.f), 0.f);
+    return lq - rw * inv2s2;
 }
 
 // Residuals of one entry from the direct difference (raw data): resid (the
@@ -250,7 +245,7 @@ MADI_DEV float least_rw(float d2, float sn, float e) {
 
 template <int N, bool FREE, int THREADS, bool INDEXED>
 __global__ void __launch_bounds__(THREADS) bayes_kernel(const __grid_constant__ Plan P) {
-    constexpr int FERR = (N + 7) / 8 * 8, EF = Entry<N>::FLOATS;
+    constexpr int EF = Entry<N>::FLOATS;
     extern __shared__ __align__(16) float sent[];            // [CHUNK][EF]
     __shared__ float smu[N], sv[INDEXED ? prune::B_FLOATS : 1];
     const int F = P.F, lane = threadIdx.x & 31;
@@ -294,7 +289,7 @@ __global__ void __launch_bounds__(THREADS) bayes_kernel(const __grid_constant__ 
             ghi[k] = o2f(__reduce_max_sync(MADI_FULL, f2o(x)));
         }
         // screen error (F + 8) 2^-21 (|m|^2 + |L|^2) twice, and the bound added to it
-        e_max = warp_maxf_bits((float)(FERR + 8) * 2e-6f * (m2 + lmax));
+        e_max = warp_maxf_bits((float)((N + 7) / 8 * 8 + 8) * 2e-6f * (m2 + lmax));
     }
     // Visits, in index order and by twos, the entries that may reach `floor` (a
     // log-weight) for some voxel of the warp; visit runs warp-wide.
@@ -371,14 +366,12 @@ __global__ void __launch_bounds__(THREADS) bayes_kernel(const __grid_constant__ 
         const unsigned who = __ballot_sync(MADI_FULL, top == w);
         tj = __shfl_sync(MADI_FULL, tj, who ? __ffs(who) - 1 : 0);
         const float* o = P.blocks + (int64_t)tj * EF;
-        float err;
-        screen<N, FERR, FREE>(m, o, o[Entry<N>::AUX], o[Entry<N>::AUX + 1], m2, P.inv2s2, known, err);
+        known = screen<N, FREE>(m, o, o[Entry<N>::AUX], o[Entry<N>::AUX + 1], m2, P.inv2s2);
     }
     sweep([&]() { return warp_minf(fmaxf(best, known)); },
           [&](int e0, const float* o0, int e1, const float* o1, bool two) {
-              float ee0, ee1, err;
-              screen<N, FERR, FREE>(m, o0, o0[Entry<N>::AUX], o0[Entry<N>::AUX + 1], m2, P.inv2s2, ee0, err);
-              screen<N, FERR, FREE>(m, o1, o1[Entry<N>::AUX], o1[Entry<N>::AUX + 1], m2, P.inv2s2, ee1, err);
+              const float ee0 = screen<N, FREE>(m, o0, o0[Entry<N>::AUX], o0[Entry<N>::AUX + 1], m2, P.inv2s2);
+              const float ee1 = screen<N, FREE>(m, o1, o1[Entry<N>::AUX], o1[Entry<N>::AUX + 1], m2, P.inv2s2);
               if (ee0 > best) { best = ee0; bj = e0; }
               if (two && ee1 > best) { best = ee1; bj = e1; }
           });
@@ -519,8 +512,16 @@ using namespace madi;
 
 void madi_match_column_mean(const float* lib, int32_t n_lib, int32_t n_feat, float* mu, cudaStream_t s);
 
-// The index pays for its ~0.1 ms from about here on.
+// Fits that get room for the index.
 static bool bayes_indexed(int64_t n_vox, int32_t n_lib) { return n_vox >= 64 && n_lib >= 256 && n_vox < 0x7fffffff; }
+
+// Where it pays for its ~0.06 ms: while the fit is one wave it saves a share of each
+// voxel's entries (20 features, us without / with it: 500 voxels x 256 entries 100 /
+// 145, x 600 206 / 220, x 1,000 331 / 305, x 5,000 1,575 / 1,134; 64 x 1,000 331 /
+// 348, x 1,500 480 / 466), in larger ones also of the chip's work (50,000 x 256 145 /
+// 149, x 400 216 / 181).  Five features and free S0 cross over at the same sizes, ten
+// at 1,500 entries, with 15 % lost at 1,000.
+static bool bayes_index_pays(int64_t n_vox, int32_t n_lib) { return n_lib >= (n_vox < 152 * 128 ? 1000 : 400); }
 
 extern "C" int64_t madi_bayes_work_bytes(int64_t n_vox, int32_t n_lib, int32_t n_feat) {
     if (n_vox <= 0 || n_lib < 1 || n_feat < 1 || n_feat > 32 || !bayes_indexed(n_vox, n_lib)) return 256;
@@ -570,7 +571,7 @@ extern "C" madi_status madi_bayes(const madi_bayes_desc* d, void* stream) {
     P.F = d->n_feat;
     P.inv2s2 = (float)inv;
     P.out = d->out;
-    const bool indexed = bayes_indexed(d->n_vox, d->n_lib) &&
+    const bool indexed = bayes_indexed(d->n_vox, d->n_lib) && bayes_index_pays(d->n_vox, d->n_lib) &&
                          d->scratch_bytes >= madi_bayes_work_bytes(d->n_vox, d->n_lib, d->n_feat);
     if (indexed) {
         unsigned char* base = static_cast<unsigned char*>(d->scratch) + 256;

@@ -367,11 +367,12 @@ madi_status madi_match_wait(const madi_match_desc* desc, void* stream);
  * n_eff = (sum w)^2 / sum w^2 and (free S0) the weighted S0.  A free-S0 voxel
  * that no entry fits with s0 > 0 gets zeros.  Entries whose weight is below
  * e^-60 of the voxel's largest weight are dropped.  Arithmetic: fp32 scores
- * screen the entries; the kept ones get a direct-difference fp32 residual
- * (error ~F ulp of the residual) and Kahan-compensated fp32 sums of
- * parameter differences from the best entry, combined in fp64.
+ * find the best entry; every entry that can weigh in gets a direct-difference
+ * fp32 residual (error ~F ulp of the residual) and adds to Kahan-compensated
+ * fp32 sums of parameter differences from the best entry (all 53 bits of the
+ * parameters, rounded to fp32 once), combined in fp64.
  * scratch: 256-byte aligned, at least madi_bayes_scratch_bytes() bytes; with
- * madi_bayes_work_bytes() the fit orders the voxels and skips entries that
+ * madi_bayes_work_bytes() large fits order the voxels and skip entries that
  * cannot weigh in (the same sums, several times faster). */
 #define MADI_BAYES_N_OUT 9
 typedef struct madi_bayes_desc {
