@@ -1,8 +1,9 @@
 """Library match on the GPU (madi/fitters_gpu.py:414-463 entry points).
 
 ``map_match_gpu`` / ``map_match_fits0_gpu`` keep the reference signatures and
-return shapes; ``precision`` selects the exhaustive FP32 scan or the BF16
-tensor-core scan with top-k FP32 rescoring.  Inputs are numpy (host) or torch
+return shapes; ``precision`` selects the FP32 match (the choice of an exhaustive
+scan; large fits skip entries by a search index) or the BF16 tensor-core scan
+with top-k FP32 rescoring.  Inputs are numpy (host) or torch
 CUDA tensors; outputs are numpy.
 """
 
@@ -45,6 +46,19 @@ def _side_stream(stream, device):
     return s
 
 
+FP32_LEAST_SCRATCH = 256            # the column means: the match then scans every entry, the fit sums the same
+
+
+def _scratch(nbytes: int, least: int, device):
+    """nbytes of scratch and its alignment, or ``least`` where the device has no room for more."""
+    try:
+        return torch.empty(nbytes + 256, dtype=torch.uint8, device=device)
+    except torch.cuda.OutOfMemoryError:
+        if least >= nbytes:
+            raise
+        return torch.empty(least + 256, dtype=torch.uint8, device=device)
+
+
 class MatchOutput(tuple):
     """(best_idx, best_resid, best_s0) device tensors of one madi_match call.
 
@@ -66,7 +80,7 @@ class MatchOutput(tuple):
 
 
 def match_device(measured, lib_mat, *, free_s0: bool = False, precision: str = "fp32", topk: int = DEFAULT_TOPK,
-                 scratch=None, stream=None, check: bool = True, flags: int = 0) -> MatchOutput:
+                 scratch=None, stream=None, check: bool = True, flags: int = 0, lean: bool = False) -> MatchOutput:
     """Run madi_match on device tensors; returns (best_idx, best_resid, best_s0) device tensors.
 
     ``check=True`` waits for the result and raises if the scan could not
@@ -76,6 +90,8 @@ def match_device(measured, lib_mat, *, free_s0: bool = False, precision: str = "
     ``flags``: MADI_MATCH_FLAG_FULL_SCAN (BF16 fixed S0 without the
     principal-axis scan cut; same result up to BF16 score ties at the k-th
     place) or, for tests, MADI_MATCH_FLAG_TEST_STALL.
+    ``lean``: FP32 without the memory of the search index (8 bytes a voxel and
+    ~150 an entry): every entry is scanned, for the same choice.
     """
     if not HAS_CUDA:
         raise RuntimeError("CUDA is unavailable: the library match runs on a CUDA device only")
@@ -91,11 +107,14 @@ def match_device(measured, lib_mat, *, free_s0: bool = False, precision: str = "
     res = torch.empty(n_vox, dtype=torch.float32, device=M.device)
     s0 = torch.empty(n_vox, dtype=torch.float32, device=M.device) if free_s0 else None
     need = int(N.lib().madi_match_scratch_bytes(n_vox, Lm.shape[0], F, prec, int(topk)))
+    least = FP32_LEAST_SCRATCH if prec == N.MADI_MATCH_FP32 else need
+    if lean:
+        need = least
     if free_s0 and prec == N.MADI_MATCH_FP32:
         scratch = None                  # never used the caller's, which overlapping calls may share
         flags = int(flags) | N.MADI_MATCH_FLAG_SCRATCH
     if need > 0 and (scratch is None or scratch.numel() < need + 256):
-        scratch = torch.empty(need + 256, dtype=torch.uint8, device=M.device)
+        scratch = _scratch(need, least, M.device)
     d = N.MadiMatchDesc()
     d.measured, d.lib, d.n_vox, d.n_lib, d.n_feat = N.ptr(M), N.ptr(Lm), n_vox, Lm.shape[0], F
     d.mode = N.MADI_MATCH_FREE_S0 if free_s0 else N.MADI_MATCH_FIXED_S0
@@ -173,7 +192,7 @@ def bayes_fit_gpu(measured_batch, lib_mat, kios_arr, rhos_arr, Vs_arr, sigma_m, 
     par = [torch.from_numpy(np.ascontiguousarray(a, np.float64)).to(dev)
            for a in (np.log(q), kios_arr, np.asarray(rhos_arr, np.float64), np.asarray(Vs_arr, np.float64))]
     out = torch.empty((N.MADI_BAYES_N_OUT, n_vox), dtype=torch.float64, device=dev)
-    scratch = torch.empty(int(N.lib().madi_bayes_work_bytes(n_vox, n_lib, F)) + 256, dtype=torch.uint8, device=dev)
+    scratch = _scratch(int(N.lib().madi_bayes_work_bytes(n_vox, n_lib, F)), FP32_LEAST_SCRATCH, dev)
     d = N.MadiBayesDesc()
     d.measured, d.lib = N.ptr(M), N.ptr(Lm)
     d.log_weight, d.kio, d.rho, d.V = (N.ptr(t) for t in par)

@@ -206,10 +206,17 @@ class Server:
     def _nbytes(self, req) -> int:
         if isinstance(req, SimRequest):
             return req.ensemble.device(str(self.dev)).nbytes
+        return self._fit_bytes(req)[0]
+
+    def _fit_bytes(self, req) -> tuple:
+        """Device memory of a fit and whether it has to do without the search index to fit the budget."""
+        from .fitters_gpu import FP32_LEAST_SCRATCH
         n, f = int(req.voxels.shape[0]), int(req.voxels.shape[1])
         prec = N.MADI_MATCH_BF16 if req.precision == "bf16" else N.MADI_MATCH_FP32
         scratch = int(N.lib().madi_match_scratch_bytes(n, int(self.library.shape[0]), f, prec, int(req.topk)))
-        return n * f * 4 + n * 12 + scratch + 512
+        base = n * f * 4 + n * 12 + 512
+        lean = prec == N.MADI_MATCH_FP32 and base + scratch > self.sched.budget
+        return base + (FP32_LEAST_SCRATCH if lean else scratch), lean
 
     def _slot_result(self, slot: int) -> dict:
         lay = self.layout
@@ -274,7 +281,8 @@ class Server:
                     from .fitters_gpu import match_device
                     with torch.cuda.stream(self.fit_stream):
                         out = match_device(req.voxels, self.library, free_s0=req.free_s0, precision=req.precision,
-                                           topk=req.topk, stream=self.fit_stream, check=False)
+                                           topk=req.topk, stream=self.fit_stream, check=False,
+                                           lean=self._fit_bytes(req)[1])
                         ev = torch.cuda.Event()
                         ev.record(self.fit_stream)
                     fits.append((ev, rid, out))
