@@ -513,7 +513,7 @@ using namespace madi;
 void madi_match_column_mean(const float* lib, int32_t n_lib, int32_t n_feat, float* mu, cudaStream_t s);
 
 // Fits that get room for the index.
-static bool bayes_indexed(int64_t n_vox, int32_t n_lib) { return n_vox >= 64 && n_lib >= 256 && n_vox < 0x7fffffff; }
+static bool bayes_indexed(int64_t n_vox, int32_t n_lib) { return n_vox >= 64 && n_lib >= 256 && n_lib <= prune::MAX_LIB && n_vox < 0x7fffffff; }
 
 // Where it pays for its ~0.06 ms: while the fit is one wave it saves a share of each
 // voxel's entries (20 features, us without / with it: 500 voxels x 256 entries 100 /

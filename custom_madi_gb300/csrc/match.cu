@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(MATCH_THREADS) match_scan_kernel(const float* 
         bar[i] = 0.f;
         bj[i] = 0;
     }
-    const int j0 = blockIdx.y * part, j1 = min(n_lib, j0 + part);
+    const int j0 = blockIdx.y * part, j1 = n_lib - j0 > part ? j0 + part : n_lib;
     float* flat = reinterpret_cast<float*>(sl);
     for (int t = threadIdx.x; t < MATCH_CHUNK * (N - n_feat); t += MATCH_THREADS) {      // never written again
         const int e = t / (N - n_feat), f = n_feat + t - e * (N - n_feat);
@@ -117,8 +117,8 @@ __global__ void __launch_bounds__(MATCH_THREADS) match_scan_kernel(const float* 
     // a thread's place in the rows moves by (de, df) from one of its loads to the next
     const int e0 = threadIdx.x / n_feat, f0 = threadIdx.x - e0 * n_feat;
     const int de = MATCH_THREADS / n_feat, df = MATCH_THREADS - de * n_feat;
-    for (int base = j0; base < j1; base += MATCH_CHUNK) {
-        const int cnt = min(MATCH_CHUNK, j1 - base);
+    for (int base = j0, left = j1 - j0; left > 0; base += MATCH_CHUNK, left -= MATCH_CHUNK) {
+        const int cnt = min(MATCH_CHUNK, left);
         __syncthreads();
         const float* src = lib + (int64_t)base * n_feat;
         int e = e0, f = f0;
@@ -485,7 +485,7 @@ static MatchPlan match_plan(int64_t n_vox, int32_t n_lib, int32_t n_feat) {
     MatchPlan p{false, 1, n_lib, 0};
     // The index costs ~0.1 ms: 20,000 voxels x 20,000 entries x 20 take 1.73 ms
     // scanned by one part, 0.20 ms pruned; 4,096 voxels 0.15 ms split over parts.
-    if (n_vox >= 4096 && n_lib >= 1024 && (double)n_vox * n_lib * n_feat >= 4e9 && n_vox < 0x7fffffff) {
+    if (n_vox >= 4096 && n_lib >= 1024 && n_lib <= prune::MAX_LIB && (double)n_vox * n_lib * n_feat >= 4e9 && n_vox < 0x7fffffff) {
         p.pruned = true;
         prune::Index ix;
         p.bytes = prune::layout(ix, nullptr, n_vox, n_lib, n_feat);
@@ -497,11 +497,11 @@ static MatchPlan match_plan(int64_t n_vox, int32_t n_lib, int32_t n_feat) {
     // (50 voxels x 200 entries x 5: 17.4 us in one part, 20.5 in two; 384 entries x
     // 20: 35 in one, 24 in three).
     const int64_t blocks = (n_vox + MATCH_THREADS - 1) / MATCH_THREADS;
-    const int64_t chunks = (n_lib + MATCH_CHUNK - 1) / MATCH_CHUNK;
+    const int64_t chunks = ((int64_t)n_lib + MATCH_CHUNK - 1) / MATCH_CHUNK;
     const int64_t want = std::min<int64_t>(std::min<int64_t>(chunks, 65535), blocks > 0 ? 1216 / blocks : 1);
     if (want > 1 && chunks > 2) {
         p.part = (int)((chunks + want - 1) / want * MATCH_CHUNK);
-        p.parts = (n_lib + p.part - 1) / p.part;
+        p.parts = (int)(((int64_t)n_lib + p.part - 1) / p.part);
         p.bytes = 8 * n_vox;
     }
     return p;

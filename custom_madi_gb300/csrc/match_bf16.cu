@@ -203,10 +203,10 @@ __global__ void column_mean_kernel(const float* __restrict__ lib, int n_lib, int
     const int f = blockIdx.x;
     double acc = 0.0;
     constexpr int AHEAD = 16;
-    for (int i = threadIdx.x; i < n_lib; i += 256 * AHEAD) {
+    for (int64_t i = threadIdx.x; i < n_lib; i += 256 * AHEAD) {
         float x[AHEAD];
 #pragma unroll
-        for (int k = 0; k < AHEAD; ++k) x[k] = i + 256 * k < n_lib ? lib[(size_t)(i + 256 * k) * F + f] : 0.f;
+        for (int k = 0; k < AHEAD; ++k) x[k] = i + 256 * k < n_lib ? lib[(i + 256 * k) * F + f] : 0.f;
 #pragma unroll
         for (int k = 0; k < AHEAD; ++k)
             if (i + 256 * k < n_lib) acc += x[k];

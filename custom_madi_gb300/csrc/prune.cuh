@@ -26,6 +26,7 @@ constexpr int FMAX = 32;
 constexpr int SAMPLE = 512;                     // rows sampled for the directions and ranges
 constexpr int LIB_FINE = 512;                   // v_2 buckets of a slab
 constexpr int MAX_SLABS = 64;
+constexpr int MAX_LIB = 1 << 30;                // entries: rounded up to tiles and blocks they stay in 32 bits
 constexpr int LIB_BINS = MAX_SLABS * LIB_FINE;
 constexpr int VOX_BINS = 64 * 32 * 16;          // (v_1, v_2, v_3) buckets
 
