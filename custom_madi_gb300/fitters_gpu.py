@@ -35,13 +35,16 @@ def _as_dev(x):
 def _side_stream(stream, device):
     """``stream`` as a torch stream if it is not the current one, ordered after the
     work enqueued there (the call's buffers are made on it); else None."""
+    if stream is None:
+        return None
     cur = torch.cuda.current_stream(device)
-    if stream is None or stream.cuda_stream == cur.cuda_stream:
+    if stream.cuda_stream == cur.cuda_stream:
         return None
     s = stream if isinstance(stream, torch.cuda.Stream) else torch.cuda.ExternalStream(stream.cuda_stream, device=device)
+    capturing = torch.cuda.is_current_stream_capturing()
     with torch.cuda.stream(s):
-        capturing = torch.cuda.is_current_stream_capturing()
-    if not capturing:               # a capture cannot wait for work outside it
+        capturing = capturing or torch.cuda.is_current_stream_capturing()
+    if not capturing:               # a wait would tie the capture to work outside it
         s.wait_stream(cur)
     return s
 
