@@ -519,9 +519,12 @@ static madi_status launch_fp32(const madi_match_desc* d, const MatchPlan& p, flo
         if (st != MADI_OK) return st;
         // Warps a group: more shorten the longest group's chain of tiles while the
         // groups alone do not fill the chip, but each repeats the group's set-up and
-        // holds a staler bound (20,000 entries, ms at 1 / 2 / 4 warps, before the
-        // packed multiply-adds: 100,000 voxels 0.83 / 0.53 / 0.47, 150,000 0.76 /
-        // 0.65 / 0.67, 300,000 1.06 / 1.07 / 1.14, 1e6 2.97 / 3.15 / 3.48).
+        // holds a staler bound.  Fixed S0, 20,000 entries x 20, ms at 1 / 2 / 4 warps:
+        // 50,000 voxels 0.40 / 0.29 / 0.24, 100,000 0.47 / 0.35 / 0.35, 125,000 0.49 /
+        // 0.40 / 0.42, 200,000 0.59 / 0.54 / 0.60, 300,000 0.74 / 0.75 / 0.85, 1e6 2.02 /
+        // 2.22 / 2.57.  40,000 entries, 10 or 28 features and free S0 cross over
+        // within 75,000 to 150,000 and 200,000 to 400,000 voxels; the lines cost them
+        // 10 % at most, and 8 % at 1,024 entries, where one warp is best from 200,000.
         const cudaError_t e = d->n_vox < 125000 ? launch_pruned<N, MODE, 4>(d, ix, s)
                               : d->n_vox < 300000 ? launch_pruned<N, MODE, 2>(d, ix, s)
                                                   : launch_pruned<N, MODE, 1>(d, ix, s);
