@@ -203,13 +203,15 @@ __global__ void column_mean_kernel(const float* __restrict__ lib, int n_lib, int
     const int f = blockIdx.x;
     double acc = 0.0;
     constexpr int AHEAD = 16;
-    for (int64_t i = threadIdx.x; i < n_lib; i += 256 * AHEAD) {
+    const float* p = lib + (int64_t)threadIdx.x * F + f;
+    const int step = 256 * F;
+    for (int left = n_lib - (int)threadIdx.x; left > 0; left -= 256 * AHEAD, p += (int64_t)AHEAD * step) {
         float x[AHEAD];
 #pragma unroll
-        for (int k = 0; k < AHEAD; ++k) x[k] = i + 256 * k < n_lib ? lib[(i + 256 * k) * F + f] : 0.f;
+        for (int k = 0; k < AHEAD; ++k) x[k] = 256 * k < left ? p[k * step] : 0.f;
 #pragma unroll
         for (int k = 0; k < AHEAD; ++k)
-            if (i + 256 * k < n_lib) acc += x[k];
+            if (256 * k < left) acc += x[k];
     }
     s[threadIdx.x] = acc;
     __syncthreads();
