@@ -43,8 +43,8 @@ METRIC = "walker-steps/s"
 CONFIG_NAME = "batched library build: 256 entries x 1e5 walkers x 4600 steps, 27-512 cells, 20 cols x 24 dirs"
 # walk_f32_kernel DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum)
 # per walker-step, from one ncu capture of 16 entries x 2e4 walkers x 4,600
-# steps: 5.50 MB + 0 MB over 1.472e9 walker-steps
-WALK_DRAM_BYTES_PER_WALKER_STEP = 5.50e6 / 1.472e9
+# steps: 5.52 MB + 0 MB over 1.472e9 walker-steps
+WALK_DRAM_BYTES_PER_WALKER_STEP = 5.52e6 / 1.472e9
 SIGNAL_ERR = 0.005          # absolute standard error on S (normalised to b = 0)
 
 

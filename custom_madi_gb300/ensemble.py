@@ -344,8 +344,9 @@ class Ensemble:
         """SI Eq. S2 labels (cell id, inside) of (N, 3) positions, on the GPU.
 
         ``method="kd"`` runs the reference's fp64 KD rule, ``"grid"`` the
-        walker's voxel-grid rule (fp64 inputs are decided in fp64 on the same
-        proven candidate lists).  Periodic positions are wrapped into [0, L).
+        walker's voxel-grid rule (in fp32, its error band widened by the rounding of
+        the fp64 points; points within the band in fp64 on the same proven candidate
+        lists).  Periodic positions are wrapped into [0, L).
         """
         import torch
         pts = np.asarray(positions, dtype=np.float64)
