@@ -742,7 +742,7 @@ __global__ void __launch_bounds__(SPREAD ? SPREAD_THREADS : 256, MINB) walk_f32_
 // the fp64 point to fp32, sqrt(3) 2^-24 L), and from the KD rule in the rest
 // (~0.04 % of steps).  What remains is bound by the fp64 pipe: Box-Muller in
 // fp64, once per pair of steps.  16,000 walkers x 4,600 steps in a 64-cell box:
-// ~900 ms before, 32 ms now.
+// ~900 ms before, 33 ms now.
 // ---------------------------------------------------------------------------
 constexpr int F64_THREADS = 128;
 
